@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include "mpgb_fastmath.cuh"
+#include "mpgb_fixed.cuh"
 
 namespace mpgb {
 
@@ -85,6 +86,7 @@ struct QuadParams {
     int maxSub, minSub;
     double absTol, relTol;
     long long maxIntervals;  // per-point interval budget (status kStatusBudget)
+    fx::Rule fx;             // the same rule in fixed point (ok 0: not provided)
 };
 
 // Constants of the last-coordinate basis.

@@ -1,0 +1,448 @@
+// 64-bit fixed-point arithmetic for the quadrature of the rectified integrand.
+//
+// Why.  A GB300 SM issues FP64 at 2 lanes a clock (measured: 1.6, DFMA or
+// DADD) but 32 x 32 + 64-bit integer multiply-adds (IMAD.WIDE) at 55 and
+// integer additions at 115.  A quadrature node of the adaptive rule is an
+// exponential, a logarithm, a reciprocal and a short polynomial on arguments
+// of known range, so it can be carried in 64-bit fixed point: a product's high
+// word is three IMAD.WIDE, a twentieth of a DFMA's time.  The fraction has 57
+// to 63 bits, so every step rounds at 2^-57 or below where a double near 1
+// rounds at 2^-53: the integrand, its weighted sums and the error estimate
+// that drives the subdivision are closer to the exact ones than in FP64.
+// Arguments outside the range (|d_D f| possibly above 31, non-finite values,
+// other rules) keep the FP64 path.
+//
+// The functions are plain C++ on uint64_t, the same on the host (tests) and
+// the device.
+#pragma once
+#include <cstdint>
+
+#if defined(__CUDA_ARCH__)
+#define MPGB_FX_TABLE __device__ const
+#elif defined(__CUDACC__)
+#define MPGB_FX_TABLE __device__ const
+#else
+#define MPGB_FX_TABLE static const
+#endif
+
+#include "mpgb_fixed_tables.h"
+
+#ifdef __CUDACC__
+#define MPGB_HD __host__ __device__ __forceinline__
+#else
+#define MPGB_HD inline
+#endif
+
+namespace mpgb {
+namespace fx {
+
+MPGB_HD uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
+MPGB_HD uint32_t lo32(uint64_t x) { return (uint32_t)x; }
+MPGB_HD uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+
+// floor(a b / 2^64) less at most 1 (the product of the low words is left
+// out), for a + b <= 2^64.
+MPGB_HD uint64_t mulhi(uint64_t a, uint64_t b) {
+    const uint64_t mid = wide(hi32(a), lo32(b)) + wide(lo32(a), hi32(b));
+    return wide(hi32(a), hi32(b)) + hi32(mid);
+}
+
+// The same for any a, b (less at most 2).
+MPGB_HD uint64_t mulhiAny(uint64_t a, uint64_t b) {
+    const uint64_t m1 = wide(lo32(a), hi32(b)), m2 = wide(hi32(a), lo32(b));
+    return wide(hi32(a), hi32(b)) + hi32(m1) + hi32(m2);
+}
+
+// floor(a b / 2^32).
+MPGB_HD uint64_t mul32(uint64_t a, uint32_t b) { return wide(hi32(a), b) + hi32(wide(lo32(a), b)); }
+
+// a b / 2^32, rounded.
+MPGB_HD uint64_t mul32Round(uint64_t a, uint32_t b) {
+    return wide(hi32(a), b) + hi32(wide(lo32(a), b) + 0x80000000ull);
+}
+
+// a b / 2^32 of two 32-bit numbers, rounded.
+MPGB_HD uint32_t hi(uint32_t a, uint32_t b) { return hi32(wide(a, b) + 0x80000000ull); }
+
+MPGB_HD uint64_t shr(uint64_t x, int n) { return n < 64 ? x >> n : 0; }
+// x / 2^n rounded to nearest, n >= 0.
+MPGB_HD uint64_t shrRound(uint64_t x, int n) { return n < 64 ? (x + ((1ull << n) >> 1)) >> n : 0; }
+
+#ifdef __CUDA_ARCH__
+MPGB_HD uint64_t expTab(uint32_t j) { return __ldg((const unsigned long long*)kExpTab + j); }
+MPGB_HD void logTab(uint32_t j, uint64_t& lg, uint32_t& inv) {
+    const uint4 v = __ldg(reinterpret_cast<const uint4*>(kLogTab) + j);
+    lg = ((uint64_t)v.y << 32) | v.x;
+    inv = v.z;
+}
+#else
+MPGB_HD uint64_t expTab(uint32_t j) { return kExpTab[j]; }
+MPGB_HD void logTab(uint32_t j, uint64_t& lg, uint32_t& inv) {
+    lg = kLogTab[j].lg;
+    inv = kLogTab[j].inv;
+}
+#endif
+
+// 2^-W for W with 57 fraction bits: the mantissa 2^-frac(W) in (1/2, 1), 63
+// fraction bits, and the integer part n (2^-W = mantissa 2^-n).
+MPGB_HD uint64_t exp2neg(uint64_t W, int& n) {
+    n = (int)(hi32(W) >> 25);
+    const uint64_t T = expTab((hi32(W) >> 20) & 31);
+    const uint64_t s = (W << 12) >> 1;  // 16 r, r = the fraction below the table's step
+    const uint32_t R = hi32(s);
+    uint32_t q = kE6 - hi(R, kE7);
+    q = kE5 - hi(R, q);
+    q = kE4 - hi(R, q);
+    const uint64_t q3 = kE3 - ((uint64_t)hi(R, q) << 11);
+    const uint64_t q2 = kE2 - mulhi(s, q3);
+    const uint64_t q1 = kE1 - mulhi(s, q2);
+    return T - mulhi(T, mulhi(s, q1));
+}
+
+// exp(-u), u with 58 fraction bits, u < 32: 63 fraction bits, below 1.
+MPGB_HD uint64_t expNeg(uint64_t u) {
+    int n;
+    const uint64_t m = exp2neg(mulhiAny(u, kLog2e63) + 1, n);  // (+ 1: the mean of what mulhiAny drops)
+    return m >> n;
+}
+
+// log(1 + e) (63 fraction bits) for e in [0, 1) with 63, and with RECIP
+// 1 / (1 + e) (63 fraction bits).  1 + e times a tabulated reciprocal is
+// 1 + r, r < 1/32: log1p(r) by its series; the reciprocal from its series to
+// 30 bits and one Newton step.
+template <bool RECIP>
+MPGB_HD uint64_t log1p(uint64_t e, uint64_t& recip) {
+    uint64_t lg;
+    uint32_t inv;
+    logTab(hi32(e) >> 26, lg, inv);
+    const uint64_t v = e | 0x8000000000000000ull;  // 1 + e
+    const uint64_t s = (mul32(v, inv) << 7) >> 1;  // 16 r (62 fraction bits of 1 + r)
+    const uint32_t R = hi32(s);
+    uint32_t q = kL9 - hi(R, kL10);
+    q = kL8 - hi(R, q);
+    q = kL7 - hi(R, q);
+    q = kL6 - hi(R, q);
+    q = kL5 - hi(R, q);
+    const uint64_t q4 = kL4 - ((uint64_t)hi(R, q) << 11);
+    const uint64_t q3 = kL3 - mulhi(s, q4);
+    const uint64_t q2 = kL2 - mulhi(s, q3);
+    const uint64_t q1 = kL1 - mulhi(s, q2);
+    if constexpr (RECIP) {
+        uint32_t z = (1u << 12) - hi(R, 1u << 8);
+        z = (1u << 16) - hi(R, z);
+        z = (1u << 20) - hi(R, z);
+        z = (1u << 24) - hi(R, z);
+        z = hi(R, (1u << 28) - hi(R, z));     // 1 - 1 / (1 + r), 32 fraction bits
+        const uint32_t y = inv - hi(inv, z);  // 31 fraction bits
+        const int64_t eps = (int64_t)(0x4000000000000000ull - mul32(v, y));  // 1 - v y, 62 fraction bits
+        const int64_t c = (int64_t)(int32_t)(y >> 1) * (int32_t)(eps >> 3);  // y eps, 89 fraction bits
+        recip = ((uint64_t)y << 32) + (uint64_t)(c >> 26);
+    }
+    return lg + (mulhi(s, q1) >> 1);
+}
+
+// SoftPlus at d = D / 2^58 - 32, |d| < 32: g = log(1 + e^-|d|) + max(d, 0)
+// with 57 fraction bits and, with DERIV, g' = 1 / (1 + e^-d) with 63.
+template <bool DERIV>
+MPGB_HD uint64_t softPlus(uint64_t D, uint64_t& gp) {
+    const bool pos = (D >> 63) != 0;
+    const uint64_t x = D ^ 0x8000000000000000ull;
+    const uint64_t u = pos ? x : 0 - x;
+    uint64_t r = 0;
+    const uint64_t l = log1p<DERIV>(expNeg(u), r);
+    if constexpr (DERIV) gp = pos ? r : 0x8000000000000000ull - r;
+    return ((l + 32) >> 6) + (pos ? u >> 1 : 0);
+}
+
+// e^d at d = D / 2^58 - 32, |d| < 32: m 2^E with m in [1/2, 1), 62 fraction bits.
+MPGB_HD uint64_t expMant(uint64_t D, int& E) {
+    // 64 - d log2(e) = (64 + 32 log2(e)) - (d + 32) log2(e), 57 fraction bits
+    constexpr uint64_t kBias = (64ull << 57) + (kLog2e63 >> 1);
+    int n;
+    const uint64_t m = exp2neg(kBias - mulhiAny(D, kLog2e63) - 1, n);
+    E = 64 - n;
+    return m >> 1;
+}
+
+// x with 58 fraction bits; bad is set for |x| >= 32 and non-finite x.
+MPGB_HD int64_t toFixed58(double x, bool& bad) {
+#ifdef __CUDA_ARCH__
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t b;
+    __builtin_memcpy(&b, &x, 8);
+#endif
+    const int e = (int)((b >> 52) & 0x7ff);
+    if (e > 1027) bad = true;
+    const uint64_t m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
+    const int sh = 1027 - e;  // (subnormal x: shifted out)
+    const int64_t v = (sh >= 0 && sh < 64) ? (int64_t)(m >> sh) : 0;
+    return (b >> 63) ? -v : v;
+}
+
+// The adaptive rule in fixed point: three coarse and five fine nodes (-1, 0, 1
+// and -rho, rho) with weights scaled to sum to 1, 64 fraction bits; mLo, mHi:
+// the weights of -rho and rho times their position in [0, 1] to the power j.
+constexpr int kMoments = 12;
+struct Rule {
+    int ok;
+    uint64_t rho, c0, cM, w0, wM, w1, rel;
+    uint64_t mLo[kMoments], mHi[kMoments];
+};
+
+
+// d_D f along one quadrature, t in [0, 1]: sum_j c_j t^j (ENV false) or
+// a + exp2(-Z t^2) sum_j c_j t^j (the envelope of the Hermite functions).
+// c_0 and a carry the bias 32 (2^63) that keeps every partial sum positive.
+template <int NB, bool ENV>
+struct Poly {
+    uint64_t c[NB];  // 58 fraction bits; every entry biased
+    uint64_t a;      // 58 fraction bits, biased
+    uint64_t Z;      // 57 fraction bits
+};
+
+// sum_j c_j t^j, biased; t with 64 fraction bits.  acc' = acc + 2^63 steps as
+// c_j' + t acc' - t 2^63 (c_j' rounds the truncated product back up).
+template <int NB, bool ENV>
+MPGB_HD uint64_t horner(const Poly<NB, ENV>& p, uint64_t t) {
+    uint64_t acc = p.c[NB - 1];
+    const uint64_t th = t >> 1;
+#pragma unroll
+    for (int j = NB - 2; j >= 0; --j) acc = (p.c[j] - th) + mulhiAny(acc, t) + 1;
+    return acc;
+}
+
+// A node: g (SoftPlus: 57 fraction bits; Exp: mantissa with 62 and exponent
+// E), f = g' (62 fraction bits; Exp: g itself), fe = g' times the envelope.
+struct Node {
+    uint64_t g, f, fe;
+    int E;
+};
+
+template <bool EXPR, bool DERIV>
+MPGB_HD void rect(uint64_t D, Node& o, uint64_t& gp63) {
+    o.E = 0;
+    o.f = o.fe = 0;
+    gp63 = 0;
+    if constexpr (EXPR) {
+        o.g = expMant(D, o.E);
+        if constexpr (DERIV) {
+            o.f = o.g;
+            gp63 = o.g << 1;
+        }
+    } else {
+        o.g = softPlus<DERIV>(D, gp63);
+        if constexpr (DERIV) o.f = gp63 >> 1;
+    }
+}
+
+template <bool EXPR, bool DERIV, int NB, bool ENV>
+MPGB_HD Node nodeAt(const Poly<NB, ENV>& p, uint64_t t) {
+    Node o;
+    uint64_t gp;
+    if constexpr (ENV) {
+        int n;
+        const uint64_t m = exp2neg(mulhiAny(mulhiAny(t, t), p.Z), n);
+        const uint64_t e = shr(m, n);  // the envelope, 63 fraction bits
+        rect<EXPR, DERIV>(p.a + mulhiAny(horner(p, t), e << 1) - e, o, gp);
+        if constexpr (DERIV) o.fe = mulhi(gp, e);
+    } else {
+        rect<EXPR, DERIV>(horner(p, t), o, gp);
+    }
+    return o;
+}
+
+// t = 0 and t = 1.
+template <bool EXPR, bool DERIV, int NB, bool ENV>
+MPGB_HD Node nodeEnd(const Poly<NB, ENV>& p, bool one) {
+    uint64_t q = p.c[0];
+    if (one) {
+#pragma unroll
+        for (int j = 1; j < NB; ++j) q += p.c[j] - 0x8000000000000000ull;
+    }
+    Node o;
+    uint64_t gp;
+    if constexpr (ENV) {
+        int n = 0;
+        uint64_t e = 0x7fffffffffffffffull;
+        if (one) {
+            const uint64_t m = exp2neg(p.Z, n);
+            e = shr(m, n);
+        }
+        rect<EXPR, DERIV>(p.a + mulhiAny(q, e << 1) - e, o, gp);
+        if constexpr (DERIV) o.fe = mulhi(gp, e);
+    } else {
+        rect<EXPR, DERIV>(q, o, gp);
+    }
+    return o;
+}
+
+// Integrals over [0, 1]: g (SoftPlus: 57 fraction bits; Exp: 62, times 2^E),
+// with NM > 0 m0 = int g' (ENV; 62 fraction bits) and m[j] = int g' t^j (times
+// the envelope with ENV); Exp: all times 2^E.
+template <int NM>
+struct Sums {
+    uint64_t g, m0, m[NM > 0 ? NM : 1];
+    int E, nInt;
+    bool over;
+};
+
+// absTol / |x_D| against sums of g scaled by 2^-level: SoftPlus as an integer
+// with 57 fraction bits, Exp as m 2^(E - 62).
+struct Threshold {
+    uint64_t m;
+    int E;
+};
+
+// The adaptive traversal of `integrate` (depth first, left first; the same
+// rule, accept test and order of accepted sums) on [0, 1].  An interval is
+// (lo, level), lo with 32 fraction bits and width 2^-level; the pending right
+// halves have distinct levels (a bit mask), and a stack indexed by level holds
+// the node at their right end.  An accepted interval's moments are formed
+// about its left end and shifted to t = 0 by repeated multiply-adds with lo.
+template <bool EXPR, int NB, bool ENV, int NM>
+MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int minSub, int maxIntervals,
+                       Threshold thr, Sums<NM>& R) {
+    constexpr bool D = NM > 0;
+    uint64_t stG[32], stF[D && !EXPR ? 32 : 1], stFe[D && ENV ? 32 : 1];
+    int stE[EXPR ? 32 : 1];
+    R.g = R.m0 = 0;
+    R.E = -200;
+    R.over = false;
+#pragma unroll
+    for (int j = 0; j < (NM > 0 ? NM : 1); ++j) R.m[j] = 0;
+    Node A = nodeEnd<EXPR, D>(p, false), B = nodeEnd<EXPR, D>(p, true);
+    uint32_t lo = 0, pend = 0;
+    int level = 0;
+    int count = 0;
+    while (true) {
+        const uint64_t mid = ((uint64_t)lo << 32) + (0x8000000000000000ull >> level);
+        const uint64_t dr = Q.rho >> (level + 1);
+        const Node V = nodeAt<EXPR, D>(p, mid - dr), M = nodeAt<EXPR, D>(p, mid), W = nodeAt<EXPR, D>(p, mid + dr);
+        uint64_t a = A.g, b = B.g, m = M.g, v = V.g, w = W.g;
+        int E = 0;
+        if constexpr (EXPR) {
+            // One exponent for the interval's nodes.
+            E = A.E > B.E ? A.E : B.E;
+            E = M.E > E ? M.E : E;
+            E = V.E > E ? V.E : E;
+            E = W.E > E ? W.E : E;
+            a = shr(a, E - A.E);
+            b = shr(b, E - B.E);
+            m = shr(m, E - M.E);
+            v = shr(v, E - V.E);
+            w = shr(w, E - W.E);
+        }
+        const uint64_t ab = a + b, vw = v + w;
+        const uint64_t ic = mulhi(ab, Q.c0) + mulhi(m, Q.cM) + 1;
+        const uint64_t ih = mulhi(ab, Q.w0) + mulhi(m, Q.wM) + mulhi(vw, Q.w1) + 2;
+        const uint64_t err = ih > ic ? ih - ic : ic - ih;
+        // err < max(relTol ic, (absTol / |x_D|) 2^level)
+        uint64_t tol = mulhi(ic, Q.rel);
+        {
+            uint64_t ta;
+            if constexpr (EXPR) {
+                const int sh = E - thr.E - level;
+                ta = sh < 0 ? ~0ull : shr(thr.m, sh);
+            } else {
+                ta = (thr.m >> (63 - level)) ? ~0ull : thr.m << level;
+            }
+            tol = ta > tol ? ta : tol;
+        }
+        const bool accept = (err < tol || level == maxSub - 1) && level >= minSub;
+        ++count;
+        if (accept) {
+            // Exp: the sums' exponent follows the largest contribution (the
+            // interval's exponent less its level), so a narrow peak keeps its
+            // bits.
+            int dn = level;
+            if constexpr (EXPR) {
+                const int e = E - level;
+                if (e > R.E) {
+                    const int up = e - R.E;
+                    R.g = shr(R.g, up);
+                    R.m0 = shr(R.m0, up);
+#pragma unroll
+                    for (int j = 0; j < (NM > 0 ? NM : 1); ++j) R.m[j] = shr(R.m[j], up);
+                    R.E = e;
+                }
+                dn = R.E - e;
+            }
+            R.g += shrRound(ih, dn);
+            if constexpr (D) {
+                uint64_t fa, fb, fm, fv, fw;
+                if constexpr (ENV) {
+                    fa = A.fe; fb = B.fe; fm = M.fe; fv = V.fe; fw = W.fe;
+                    if constexpr (EXPR) {
+                        fa = shr(fa, E - A.E); fb = shr(fb, E - B.E); fm = shr(fm, E - M.E);
+                        fv = shr(fv, E - V.E); fw = shr(fw, E - W.E);
+                        R.m0 = R.g;
+                    } else {
+                        R.m0 += shrRound(mulhi(A.f + B.f, Q.w0) + mulhi(M.f, Q.wM) + mulhi(V.f + W.f, Q.w1) + 2, level);
+                    }
+                } else if constexpr (EXPR) {
+                    fa = a; fb = b; fm = m; fv = v; fw = w;
+                } else {
+                    fa = A.f; fb = B.f; fm = M.f; fv = V.f; fw = W.f;
+                }
+                uint64_t mu[NM];
+                fb = mulhi(fb, Q.w0);
+                fm = mulhi(fm, Q.wM);
+                mu[0] = mulhi(fa, Q.w0) + fb + fm + mulhi(fv + fw, Q.w1) + 3;
+#pragma unroll
+                for (int j = 1; j < NM; ++j) mu[j] = fb + (fm >> j) + mulhi(fv, Q.mLo[j]) + mulhi(fw, Q.mHi[j]) + 2;
+#pragma unroll
+                for (int j = 0; j < NM; ++j) mu[j] = shrRound(mu[j], level * j + dn);
+#pragma unroll
+                for (int i = 0; i + 1 < NM; ++i) {
+#pragma unroll
+                    for (int j = NM - 1; j > i; --j) mu[j] += mul32Round(mu[j - 1], lo);
+                }
+#pragma unroll
+                for (int j = 0; j < NM; ++j) R.m[j] += mu[j];
+            }
+            if constexpr (EXPR) {
+                if (R.g >> 62) {
+                    R.g >>= 1;
+                    R.m0 >>= 1;
+#pragma unroll
+                    for (int j = 0; j < (NM > 0 ? NM : 1); ++j) R.m[j] >>= 1;
+                    ++R.E;
+                }
+            }
+            if (pend == 0) break;
+#ifdef __CUDA_ARCH__
+            const int L = 31 - __clz((int)pend);
+#else
+            const int L = 31 - __builtin_clz(pend);
+#endif
+            pend ^= 1u << L;
+            lo += 1u << (32 - level);
+            level = L;
+            A = B;
+            B.g = stG[L];
+            if constexpr (EXPR) B.E = stE[L];
+            if constexpr (D) {
+                if constexpr (EXPR) B.f = B.g;
+                else B.f = stF[L];
+                if constexpr (ENV) B.fe = stFe[L];
+            }
+        } else {
+            ++level;
+            pend |= 1u << level;
+            stG[level] = B.g;
+            if constexpr (EXPR) stE[level] = B.E;
+            if constexpr (D && !EXPR) stF[level] = B.f;
+            if constexpr (D && ENV) stFe[level] = B.fe;
+            B = M;
+        }
+        if (count >= maxIntervals) {
+            R.over = true;
+            return;
+        }
+    }
+    R.nInt = count;
+}
+
+}  // namespace fx
+}  // namespace mpgb

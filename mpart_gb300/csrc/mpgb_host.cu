@@ -533,6 +533,34 @@ void buildLaunchConstants(const MapOptions& o, QuadParams& q, BasisConsts& b) {
     q.absTol = o.quadAbsTol;
     q.relTol = o.quadRelTol;
     q.maxIntervals = 1LL << 24;
+    // The fixed-point form of the three / five point rules (mpgb_fixed.cuh),
+    // weights scaled to sum to 1.  Midpoints at level 30 still fit its 32-bit
+    // positions, and a zero absolute tolerance (subdivision driven by rounding
+    // where the integrand vanishes) stays with FP64.
+    q.fx = fx::Rule{};
+    if (q.kind != kQuadFixedCC && q.nCoarse == 3 && q.nFine == 5 && q.maxSub <= 31 && q.relTol < 0.5 &&
+        q.absTol > 0 && std::isfinite(q.absTol)) {
+        auto frac = [](double w) { return (uint64_t)std::ldexp(w, 64); };
+        q.fx.ok = 1;
+        q.fx.rho = frac(q.fPts[3]);
+        q.fx.c0 = frac(0.5 * q.cWts[0]);
+        q.fx.cM = frac(0.5 * q.cWts[1]);
+        q.fx.w0 = frac(0.5 * q.fWts[0]);
+        q.fx.wM = frac(0.5 * q.fWts[2]);
+        q.fx.w1 = frac(0.5 * q.fWts[3]);
+        q.fx.rel = frac(q.relTol);
+        // Powers of the positions in 64-bit integers: in double their rounding
+        // would grow with j and bias the moments.
+        auto mulRound = [](uint64_t x, uint64_t y) {
+            return (uint64_t)(((unsigned __int128)x * y + ((unsigned __int128)1 << 63)) >> 64);
+        };
+        const uint64_t half = 1ull << 63, tauLo = half - (q.fx.rho >> 1), tauHi = half + (q.fx.rho >> 1);
+        q.fx.mLo[0] = q.fx.mHi[0] = q.fx.w1;
+        for (int j = 1; j < fx::kMoments; ++j) {
+            q.fx.mLo[j] = mulRound(q.fx.mLo[j - 1], tauLo);
+            q.fx.mHi[j] = mulRound(q.fx.mHi[j - 1], tauHi);
+        }
+    }
 
     const bool norm = o.basisNorm;
     for (int k = 0; k <= kMaxLastOrder; ++k) {

@@ -342,6 +342,183 @@ __device__ __forceinline__ void integrate(const double* a, int P, double xd, con
     }
 }
 
+// Power-basis coefficients of the per-order functions u_k of a node (see
+// scaleCoeffs): ProbabilistHermite u_(k+1) = He_k; HermiteFunctions
+// u_(k+2) = 2 k H_(k-1) - y H_k (row k, column j: the coefficient of y^j).
+template <int BASIS, int N>
+struct NodePoly {
+    double c[N][N + 1];
+    constexpr NodePoly() : c{} {
+        if (BASIS == kBasisProbHermite) {
+            for (int k = 0; k < N; ++k)
+                for (int j = 0; j <= k; ++j) {
+                    double v = (k == 0) ? 1.0 : (j > 0 ? c[k - 1][j - 1] : 0.0);
+                    if (k >= 2) v -= (k - 1.0) * c[k - 2][j];
+                    c[k][j] = v;
+                }
+        } else {
+            double H[N + 1][N + 2] = {};
+            H[0][0] = 1.0;
+            for (int k = 0; k < N; ++k) {
+                if (k >= 1)
+                    for (int j = 0; j <= k; ++j)
+                        H[k][j] = (j > 0 ? 2.0 * H[k - 1][j - 1] : 0.0) - (k >= 2 ? 2.0 * (k - 1.0) * H[k - 2][j] : 0.0);
+                for (int j = 0; j <= k + 1 && j <= N; ++j)
+                    c[k][j] = (k >= 1 && j < k ? 2.0 * k * H[k - 1][j] : 0.0) - (j >= 1 ? H[k][j - 1] : 0.0);
+            }
+        }
+    }
+};
+
+// Largest last-input order the fixed-point quadrature is built for.
+constexpr int kFxMaxOrder = 6;
+
+// The quadrature of `integrate` in 64-bit fixed point (fx::integrate): the
+// coefficients a_k become those of d_D f(t x_D) as a polynomial in t, the
+// traversal integrates g and, for adjoints, the moments of g' t^j, and J and
+// E follow from the moments.  False (nothing done) where its range does not
+// hold: a rule it is not built for, a nugget, coefficients with
+// sum |b_j| > 31 or not finite, an envelope exponent above 126, or SoftPlus
+// with d_D f(0) < -4 (g' would lose relative accuracy).  The bounds hold for
+// all but the far tails of ordinary maps (dim 8, order 4, N(0, 1) points:
+// every point up to |x_D| = 5).
+template <int BASIS, int POS, int PMAX, bool NEEDJ, int NEEDE>
+__device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd, const QuadParams& Q,
+                                               const BasisConsts& bc, double nugget, QuadOut<PMAX, NEEDJ, NEEDE>& R,
+                                               int& st) {
+    constexpr bool EXPR = POS == kPosExp;
+    constexpr bool ENV = BASIS == kBasisHermiteFunctions;
+    constexpr int NM = !NEEDJ ? 0 : (ENV && NEEDE) ? PMAX + 2 : PMAX;
+    static_assert(PMAX <= kFxMaxOrder && NM <= fx::kMoments, "order");
+    if (!Q.fx.ok || nugget != 0.0) return false;
+    constexpr NodePoly<BASIS, PMAX> U;
+    double as[PMAX + 1];
+    scaleCoeffs<BASIS, PMAX>(a, P, bc, as);
+    double b[PMAX];
+    {
+        double xp = 1.0;
+#pragma unroll
+        for (int j = 0; j < PMAX; ++j) {
+            double s = 0.0;
+#pragma unroll
+            for (int k = 0; k < PMAX; ++k) {
+                const double u = ENV ? (k >= 1 ? U.c[k - 1][j] : 0.0) : U.c[k][j];
+                if (u != 0.0) s = fma(u, as[k + 1], s);
+            }
+            b[j] = j == 0 ? s : s * xp;
+            xp = j == 0 ? xd : xp * xd;
+        }
+    }
+    bool bad = !(fabs(xd) < 1e100);
+    fx::Poly<PMAX, ENV> p;
+    uint32_t sum = 0;
+    int64_t d0 = 0;
+#pragma unroll
+    for (int j = 0; j < PMAX; ++j) {
+        const int64_t v = fx::toFixed58(b[j], bad);
+        if (j == 0) d0 = v;
+        sum += (uint32_t)((v < 0 ? -v : v) >> 35) + 1;
+        p.c[j] = (uint64_t)v + 0x8000000000000000ull;
+    }
+    p.a = p.Z = 0;
+    if constexpr (ENV) {
+        const int64_t v = fx::toFixed58(as[1], bad);
+        d0 += v;
+        sum += (uint32_t)((v < 0 ? -v : v) >> 35) + 1;
+        p.a = (uint64_t)v + 0x8000000000000000ull;
+        const double z = (xd * xd) * 0.72134752044448170368;  // x_D^2 / (2 ln 2)
+        bad |= !(z < 126.0);
+        p.Z = bad ? 0 : (uint64_t)(z * 0x1p57);
+    }
+    bad |= sum > (31u << 23);
+    if constexpr (!EXPR) bad |= d0 < -(4ll << 58);
+    if (bad) return false;
+    const double ta = Q.absTol / fabs(xd);
+    fx::Threshold thr;
+    if constexpr (EXPR) {
+        const uint64_t t = (uint64_t)__double_as_longlong(ta);
+        thr.m = ((t & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
+        thr.E = (int)(t >> 52) - 1023;
+    } else {
+        thr.m = ta < 32.0 ? (uint64_t)(ta * 0x1p57) : 1ull << 62;
+        thr.E = 0;
+    }
+    fx::Sums<NM> S;
+    fx::integrate<EXPR, PMAX, ENV, NM>(p, Q.fx, Q.maxSub, Q.minSub, (int)Q.maxIntervals, thr, S);
+    R.nInt = S.nInt;
+    if (S.over) {
+        st |= kStatusBudget;
+        R.Ih = __longlong_as_double(0x7ff8000000000000ULL);
+        return true;
+    }
+    // 2^E of the Exp sums (|E| <= 64)
+    const double sc = EXPR ? __longlong_as_double((long long)(S.E - 62 + 1023) << 52) : 0x1p-62;
+    const double G = (double)S.g * (EXPR ? sc : 0x1p-57);
+    R.Ih = xd * G;
+    if constexpr (NEEDJ) {
+        double m[NM];
+#pragma unroll
+        for (int j = 0; j < NM; ++j) m[j] = (double)S.m[j] * sc;
+        if constexpr (NEEDE) {
+            // d/dx_D of the integrand is g + t d/dt g(d_D f(t x_D))
+            double e = G;
+#pragma unroll
+            for (int j = 0; j < PMAX; ++j) {
+                double q = double(j) * m[j];
+                if constexpr (ENV) q = fma(-(xd * xd), m[j + 2], q);
+                e = fma(b[j], q, e);
+            }
+            R.IE = e;
+        }
+        double xp = xd;  // x_D^(j + 1)
+#pragma unroll
+        for (int j = 0; j < PMAX; ++j) {
+            m[j] *= xp;
+            if (j + 1 < PMAX) xp *= xd;
+        }
+        if constexpr (ENV) R.J[0] = xd * ((double)S.m0 * sc);
+#pragma unroll
+        for (int k = ENV ? 1 : 0; k < PMAX; ++k) {
+            double s = 0.0;
+#pragma unroll
+            for (int j = 0; j < PMAX; ++j) {
+                const double u = ENV ? (k >= 1 ? U.c[k >= 1 ? k - 1 : 0][j] : 0.0) : U.c[k][j];
+                if (u != 0.0) s = fma(u, m[j], s);
+            }
+            R.J[k] = s * basisScale<BASIS>(k + 1, bc);
+        }
+    }
+    return true;
+}
+
+// The FP64 quadrature out of line, for the points the fixed-point one leaves.
+template <int BASIS, int POS, int PMAX, bool NEEDJ, int NEEDE>
+__device__ __noinline__ void integrateOut(const double* a, int P, double xd, const QuadParams* Q,
+                                          const BasisConsts* bc, double nugget, QuadOut<PMAX, NEEDJ, NEEDE>* R,
+                                          int* st) {
+    integrate<BASIS, POS, PMAX, NEEDJ, NEEDE>(a, P, xd, *Q, *bc, nugget, *R, *st);
+}
+
+// The quadrature of one point: fixed point where its range holds, else FP64.
+template <int BASIS, int POS, int PMAX, bool NEEDJ, int NEEDE>
+__device__ __forceinline__ void integratePoint(const double* a, int P, double xd, const QuadParams& Q,
+                                               const BasisConsts& bc, double nugget, QuadOut<PMAX, NEEDJ, NEEDE>& R,
+                                               int& st) {
+    if constexpr (PMAX <= kFxMaxOrder && NEEDE < 2) {
+        if (integrateFixed<BASIS, POS, PMAX, NEEDJ, NEEDE>(a, P, xd, Q, bc, nugget, R, st)) return;
+        QuadOut<PMAX, NEEDJ, NEEDE> O;
+        double al[PMAX + 1];
+#pragma unroll
+        for (int k = 0; k <= PMAX; ++k) al[k] = a[k];
+        int s = 0;
+        integrateOut<BASIS, POS, PMAX, NEEDJ, NEEDE>(al, P, xd, &Q, &bc, nugget, &O, &s);
+        R = O;
+        st |= s;
+    } else {
+        integrate<BASIS, POS, PMAX, NEEDJ, NEEDE>(a, P, xd, Q, bc, nugget, R, st);
+    }
+}
+
 // Value-only integral for the inverse solver.
 template <int BASIS, int POS, int PMAX>
 __device__ __forceinline__ double integrateValue(const double* a, int P, double xd, const QuadParams& Q,
@@ -624,7 +801,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                 const bool needT = (flags & (kFlagEval | kFlagCoefDenseT | kFlagKL)) != 0 ||
                                    (NEEDJ && (flags & (kFlagCoefReduced | kFlagInput))) || NEEDE == 2;
                 if (needT && active) {
-                    integrate<BASIS, POS, PMAX, NEEDJ, NEEDE>(a, P, xd, prm.quad, prm.bc, prm.nugget, R, st);
+                    integratePoint<BASIS, POS, PMAX, NEEDJ, NEEDE>(a, P, xd, prm.quad, prm.bc, prm.nugget, R, st);
                     // the point's cost in this component, a sort key for the next call
                     if (!BATCH && prm.costKey) prm.costKey[(long long)ci * prm.costStride + i] = 0.125 * R.nInt;
                 }
