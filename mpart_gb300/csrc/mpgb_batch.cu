@@ -118,7 +118,7 @@ __global__ void segScatterKernel(const SortSeg* segs, const int* chunkSeg, const
     for (int c = 0; c < kChunk / 32; ++c) {
         const long long i = base + c * 32 + lane;
         const bool active = i < sg.N;
-        const int key = active ? bucketOf(sg.xd[i * sg.stride]) : kBuckets + lane;
+        const int key = active ? bucketOf(x[c]) : kBuckets + lane;
         const unsigned grp = __match_any_sync(0xffffffffu, key);
         const int rank = __popc(grp & lt);
         int slot = 0;
@@ -139,12 +139,10 @@ struct GatherSeg {
     int off, nSlots;
 };
 
-__global__ void gatherSegKernel(const GatherSeg* g, double* cm) {
-    const GatherSeg s = g[blockIdx.y];
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= s.nSlots) return;
-    const int t = s.slotTerm[j];
-    cm[s.off + j] = t >= 0 ? s.src[t] : 0.0;
+__global__ void __launch_bounds__(512) gatherSegKernel(const GatherSeg* g, double* cm, int2* cmFx, int* scale) {
+    const GatherSeg s = g[blockIdx.x];
+    gatherComponent(s.src, s.slotTerm, s.nSlots, cm + s.off, cmFx ? cmFx + s.off : nullptr, scale + blockIdx.x,
+                    kNoLimbs);
 }
 
 // Fixed-order reduction of each component's partial rows (the single-map
@@ -261,7 +259,8 @@ public:
                 nBmax_ = std::max(nBmax_, pg->nB);
                 depthMax_ = std::max(depthMax_, pg->maxDepth);
                 pclass_ = std::max(pclass_, batchOrderClass(pg->P));
-                if (pg->nSlots + pg->nNodes <= kStageCap) stageNeed_ = std::max(stageNeed_, pg->nSlots + pg->nNodes);
+                maxCNodes_ = std::max(maxCNodes_, pg->nCNodes);
+                stageNeed_ = std::max(stageNeed_, std::max(kStageMin, std::min(kStageCap, pg->nSlots + 2 * (pg->nNodes + 2))));
             }
         }
         totalSlots_ = slot;
@@ -277,6 +276,8 @@ public:
             c.coeffOffset = (int)part.mapCoeffOffset; c.slotOffset = bc.slotOffset; c.cSegs = p.cSegs;
             c.nodeA = p.dNodeA; c.nodeSlot = p.dNodeSlot; c.nodeC = p.dNodeC; c.nodeCRows = p.dNodeCRows;
             c.slotTerm = p.dSlotTerm; c.leadDeg = p.dLeadDeg; c.rowOff = p.dRowOff;
+            c.nodeCIdx = p.dNodeCIdx;
+            c.nodeCRow = p.dNodeCRow;
             cd.push_back(c);
         }
         compDesc_.ensure(cd.size() * sizeof(CompDesc));
@@ -450,16 +451,17 @@ private:
         }
         // Coefficient gather.
         std::vector<GatherSeg> g;
-        int maxSlots = 1;
         for (auto& bc : comps_) {
             const auto& part = maps_[bc.map]->Parts()[bc.part];
             part.owner->CheckCoefficients("MapBatch");
             g.push_back({part.owner->Coeffs() + part.coeffOffset, bc.prog->dSlotTerm, bc.slotOffset, bc.prog->nSlots});
-            maxSlots = std::max(maxSlots, bc.prog->nSlots);
         }
         upload(gatherBuf_, g, s);
         cm_.ensure(std::max(1, totalSlots_) * sizeof(double));
-        gatherSegKernel<<<dim3((maxSlots + 255) / 256, nC), 256, 0, s>>>(gatherBuf_.as<GatherSeg>(), cm_.as<double>());
+        cmFx_.ensure((totalSlots_ + 1) * sizeof(int2));
+        cmScale_.ensure(nC * sizeof(int));
+        gatherSegKernel<<<nC, 512, 0, s>>>(gatherBuf_.as<GatherSeg>(), cm_.as<double>(),
+                                           limbMap(basis_, 1) ? cmFx_.as<int2>() : nullptr, cmScale_.as<int>());
         MPGB_CUDA(cudaGetLastError());
         countLaunches(s, 1);
 
@@ -571,6 +573,8 @@ private:
         FusedParams p{};
         p.comps = compDesc_.as<CompDesc>();
         p.cm = cm_.as<double>();
+        p.cmFx = limbMap(basis_, 1) ? cmFx_.as<int2>() : nullptr;  // (per component: orders up to 6)
+        p.cmScale = cmScale_.as<int>();
         p.N = 0;
         p.flags = kFlagEval | kFlagLogDet | kFlagCoefReduced;
         p.tpb = tpb_;
@@ -597,14 +601,30 @@ private:
         p.items = itemBuf_.as<WorkItem>();
         const size_t smem = fusedSmemBytes(tpb_, dmax_, nBmax_, depthMax_, pclass_, false);
         if (smem > 227 * 1024) throw std::invalid_argument("MapBatch: components too large for the shared-memory tile.");
-        // Phase A's inputs staged in shared memory for the components that fit
-        // kStageCap, when that leaves the blocks per SM unchanged (the batch
-        // kernel's register budget: 4 blocks for order classes up to 4, 2 above).
+        // Phase A's inputs staged in shared memory: as for single maps (the
+        // batch kernel's register budget: 4 blocks for order classes up to 4, 2
+        // above).
         {
-            const size_t base = smem + 1024, with = base + (size_t)stageNeed_ * sizeof(double);
+            const size_t base = smem + 2048;
             const size_t lb = pclass_ <= 4 ? 4 : 2;
             auto blocks = [&](size_t b) { return std::min<size_t>(lb, (size_t)smemPerSM_ / b); };
-            p.stageDoubles = (stageNeed_ > 0 && with <= 227 * 1024 && blocks(with) == blocks(base)) ? stageNeed_ : 0;
+            auto fits = [&](int n) {
+                const size_t with = base + (size_t)n * sizeof(double);
+                return with <= 227 * 1024 && blocks(with) == blocks(base);
+            };
+            int n = stageNeed_;
+            while (n >= kStageMin && !fits(n)) n /= 2;
+            if (n < kStageMin) n = base + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
+            p.stageDoubles = n;
+        }
+        // The kept products of a tile, one cache per resident block (at most
+        // 512 threads an SM); above 2 GiB the reduction forms them again in FP64.
+        p.rcStride = (long long)maxCNodes_ * tpb_;
+        const long long blocks = std::min<long long>((long long)items.size(), (512LL / tpb_) * numSMs_);
+        if (p.rcStride * blocks * (long long)sizeof(double) <= (2LL << 30)) {
+            rcache_.ensure((size_t)(p.rcStride * blocks) * sizeof(double));
+            p.rcache = rcache_.as<double>();
+            p.rcBlocks = (int)blocks;
         }
         MPGB_CUDA(launchBatch(basis_, pos_, p, (int)items.size(), pclass_, counter_.as<int>(), s));
     }
@@ -691,7 +711,7 @@ private:
     int basis_ = 0, pos_ = 0;
     QuadParams quad_{};
     BasisConsts bc_{};
-    int dmax_ = 1, nBmax_ = 0, depthMax_ = 0, pclass_ = 2, totalSlots_ = 0, numSMs_ = 1, stageNeed_ = 0,
+    int dmax_ = 1, nBmax_ = 0, depthMax_ = 0, pclass_ = 2, totalSlots_ = 0, numSMs_ = 1, stageNeed_ = 0, maxCNodes_ = 0,
         smemPerSM_ = 0;
     int tpb_ = 128;
     std::map<std::pair<int, int>, int> tiles_;
@@ -701,7 +721,7 @@ private:
     std::vector<LogdetSeg> logdet_;
     long long maxN_ = 1;
     double lsensScale_ = 0.0;
-    Buf compDesc_, status_, gatherBuf_, cm_, logdetRows_, perm_, ioBuf_, segBuf_, chunkSegBuf_, hist_, partials_,
+    Buf compDesc_, status_, gatherBuf_, cm_, cmFx_, cmScale_, rcache_, logdetRows_, perm_, ioBuf_, segBuf_, chunkSegBuf_, hist_, partials_,
         rowBaseBuf_, itemBuf_, counter_, reduceBuf_, logdetBuf_;
 };
 

@@ -39,6 +39,8 @@ constexpr int kFusedBlocksPerSM = 4;
 // Largest phase-A staging (coefficient doubles plus table words) a fused
 // launch keeps in shared memory.
 constexpr int kStageCap = 2048;
+// Smallest staging the fixed-point phase A works with (its chunks of nodes).
+constexpr int kStageMin = 256;
 // Inverse: doubles of a saved root-solver state (RootSolve::save).
 constexpr int kSolveStateDoubles = 14;
 // Inverse warp pass: lanes per deferred point (32 / kWarpGroup points per warp).
@@ -178,6 +180,58 @@ __device__ __forceinline__ double prefixProduct(int depth, const int* r, const d
         }
     }
     return phi;
+}
+
+// One block gathers a component's coefficients into its slots, as doubles (cm)
+// and, unless limbs is null, as limbs scaled by 2^-s (see kNoLimbs).  The
+// first kGatherKeep values of a thread stay in registers between the two.
+__device__ __forceinline__ void gatherComponent(const double* src, const int32_t* slotTerm, int nSlots, double* cm,
+                                                int2* limbs, int* scale, int noLimbs) {
+    constexpr int kGatherKeep = 4;
+    __shared__ double red[32];
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5, step = blockDim.x;
+    double s = 0.0, v[kGatherKeep];
+    bool bad = false;
+#pragma unroll
+    for (int q = 0; q < kGatherKeep; ++q) {
+        const int j = threadIdx.x + q * step;
+        const int t = j < nSlots ? slotTerm[j] : -1;
+        v[q] = t >= 0 ? src[t] : 0.0;
+    }
+#pragma unroll
+    for (int q = 0; q < kGatherKeep; ++q) {
+        const int j = threadIdx.x + q * step;
+        if (j < nSlots) cm[j] = v[q];
+        s = fmax(s, fabs(v[q]));
+        bad |= !(fabs(v[q]) < 0x1p900);
+    }
+    for (int j = threadIdx.x + kGatherKeep * step; j < nSlots; j += step) {
+        const int t = slotTerm[j];
+        const double x = t >= 0 ? src[t] : 0.0;
+        cm[j] = x;
+        s = fmax(s, fabs(x));
+        bad |= !(fabs(x) < 0x1p900);
+    }
+    if (!limbs) return;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) s = fmax(s, __shfl_xor_sync(0xffffffffu, s, o));
+    if (lane == 0) red[wp] = s;
+    bad = __syncthreads_or(bad);
+    s = 0.0;
+    for (int q = 0; q < nw; ++q) s = fmax(s, red[q]);
+    const bool ok = !bad && (s == 0.0 || s > 0x1p-900);
+    const int e = s == 0.0 ? 0 : fx::expBound(s) + 2;
+    if (threadIdx.x == 0) *scale = ok ? e : noLimbs;
+    if (!ok) return;
+    auto put = [&](int j, double x) {
+        const long long f = fx::toFixed(x, 58 - e);
+        const long long h = (f + (1ll << 27)) >> 28;
+        limbs[j] = make_int2((int)h, (int)(f - (h << 28)));
+    };
+#pragma unroll
+    for (int q = 0; q < kGatherKeep; ++q)
+        if ((int)threadIdx.x + q * step < nSlots) put(threadIdx.x + q * step, v[q]);
+    for (int j = threadIdx.x + kGatherKeep * step; j < nSlots; j += step) put(j, cm[j]);
 }
 
 // Sort bucket of a point by |x_D| (256 buckets): width 1/32 below 4, width 1/4

@@ -17,9 +17,7 @@
 #pragma once
 #include <cstdint>
 
-#if defined(__CUDA_ARCH__)
-#define MPGB_FX_TABLE __device__ const
-#elif defined(__CUDACC__)
+#ifdef __CUDACC__
 #define MPGB_FX_TABLE __device__ const
 #else
 #define MPGB_FX_TABLE static const
@@ -28,7 +26,7 @@
 #include "mpgb_fixed_tables.h"
 
 #ifdef __CUDACC__
-#define MPGB_HD __host__ __device__ __forceinline__
+#define MPGB_HD __device__ __forceinline__
 #else
 #define MPGB_HD inline
 #endif
@@ -38,31 +36,52 @@ namespace fx {
 
 MPGB_HD uint32_t hi32(uint64_t x) { return (uint32_t)(x >> 32); }
 MPGB_HD uint32_t lo32(uint64_t x) { return (uint32_t)x; }
-MPGB_HD uint64_t wide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+// a b + c of 32-bit factors and a 64-bit addend: one IMAD.WIDE each.
+#ifdef __CUDA_ARCH__
+MPGB_HD uint64_t mulWide(uint32_t a, uint32_t b) {
+    uint64_t r;
+    asm("mul.wide.u32 %0, %1, %2;" : "=l"(r) : "r"(a), "r"(b));
+    return r;
+}
+MPGB_HD uint64_t madWide(uint32_t a, uint32_t b, uint64_t c) {
+    uint64_t r;
+    asm("mad.wide.u32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+MPGB_HD int64_t madWideS(int32_t a, int32_t b, int64_t c) {
+    int64_t r;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(r) : "r"(a), "r"(b), "l"(c));
+    return r;
+}
+#else
+MPGB_HD uint64_t mulWide(uint32_t a, uint32_t b) { return (uint64_t)a * b; }
+MPGB_HD uint64_t madWide(uint32_t a, uint32_t b, uint64_t c) { return (uint64_t)a * b + c; }
+MPGB_HD int64_t madWideS(int32_t a, int32_t b, int64_t c) { return (int64_t)a * b + c; }
+#endif
 
 // floor(a b / 2^64) less at most 1 (the product of the low words is left
 // out), for a + b <= 2^64.
 MPGB_HD uint64_t mulhi(uint64_t a, uint64_t b) {
-    const uint64_t mid = wide(hi32(a), lo32(b)) + wide(lo32(a), hi32(b));
-    return wide(hi32(a), hi32(b)) + hi32(mid);
+    const uint64_t mid = madWide(hi32(a), lo32(b), mulWide(lo32(a), hi32(b)));
+    return madWide(hi32(a), hi32(b), hi32(mid));
 }
 
 // The same for any a, b (less at most 2).
 MPGB_HD uint64_t mulhiAny(uint64_t a, uint64_t b) {
-    const uint64_t m1 = wide(lo32(a), hi32(b)), m2 = wide(hi32(a), lo32(b));
-    return wide(hi32(a), hi32(b)) + hi32(m1) + hi32(m2);
+    const uint64_t m1 = mulWide(lo32(a), hi32(b)), m2 = mulWide(hi32(a), lo32(b));
+    return madWide(hi32(a), hi32(b), hi32(m1)) + hi32(m2);
 }
 
 // floor(a b / 2^32).
-MPGB_HD uint64_t mul32(uint64_t a, uint32_t b) { return wide(hi32(a), b) + hi32(wide(lo32(a), b)); }
+MPGB_HD uint64_t mul32(uint64_t a, uint32_t b) { return madWide(hi32(a), b, hi32(mulWide(lo32(a), b))); }
 
 // a b / 2^32, rounded.
 MPGB_HD uint64_t mul32Round(uint64_t a, uint32_t b) {
-    return wide(hi32(a), b) + hi32(wide(lo32(a), b) + 0x80000000ull);
+    return madWide(hi32(a), b, hi32(madWide(lo32(a), b, 0x80000000ull)));
 }
 
 // a b / 2^32 of two 32-bit numbers, rounded.
-MPGB_HD uint32_t hi(uint32_t a, uint32_t b) { return hi32(wide(a, b) + 0x80000000ull); }
+MPGB_HD uint32_t hi(uint32_t a, uint32_t b) { return hi32(madWide(a, b, 0x80000000ull)); }
 
 MPGB_HD uint64_t shr(uint64_t x, int n) { return n < 64 ? x >> n : 0; }
 // x / 2^n rounded to nearest, n >= 0.
@@ -178,6 +197,48 @@ MPGB_HD int64_t toFixed58(double x, bool& bad) {
     const int sh = 1027 - e;  // (subnormal x: shifted out)
     const int64_t v = (sh >= 0 && sh < 64) ? (int64_t)(m >> sh) : 0;
     return (b >> 63) ? -v : v;
+}
+
+// x 2^sc rounded to an integer, for |x| 2^sc < 2^62; finite x.
+MPGB_HD int64_t toFixed(double x, int sc) {
+#ifdef __CUDA_ARCH__
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t b;
+    __builtin_memcpy(&b, &x, 8);
+#endif
+    const int e = (int)((b >> 52) & 0x7ff);
+    const int sh = 1084 - e - sc;  // (62 - the product's exponent) - 1
+    if (e == 0 || sh > 62) return 0;  // below half a unit (subnormals too)
+    const uint64_t m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
+    const int64_t v = sh < 0 ? (int64_t)m : (int64_t)(((m >> sh) + 1) >> 1);
+    return (b >> 63) ? -v : v;
+}
+
+// The exponent bound of a double: |x| < 2^expBound(x) (finite x; a very small
+// number for 0); 1025 for infinities and NaN.
+MPGB_HD int expBound(double x) {
+#ifdef __CUDA_ARCH__
+    const uint32_t h = (uint32_t)__double2hiint(x);
+#else
+    uint64_t b;
+    __builtin_memcpy(&b, &x, 8);
+    const uint32_t h = (uint32_t)(b >> 32);
+#endif
+    return (int)((h >> 20) & 0x7ff) - 1022;
+}
+
+// Products of leading-basis values in fixed point: phi = (h 2^27 + l) 2^-57,
+// 0 <= l < 2^27, |phi| <= 1, times a basis value (bh 2^31 + bl) 2^-58, |B| < 16.
+// The constant is the mean of what the shift and the left-out product of the
+// low words drop.
+struct Limbs {
+    int32_t h, l;
+};
+MPGB_HD Limbs limbMul(Limbs p, int32_t bh, int32_t bl) {
+    const int64_t m = madWideS(p.l << 4, bh, madWideS(p.h, bl, 3ll << 29));
+    const int64_t v = madWideS(p.h, bh, m >> 31);
+    return {(int32_t)(v >> 27), (int32_t)v & 0x07ffffff};
 }
 
 // The adaptive rule in fixed point: three coarse and five fine nodes (-1, 0, 1

@@ -313,7 +313,7 @@ struct KLPlan {
 };
 
 struct MapWorkspace {
-    DevBuf comps, cm, gather, items, partials, rowBase, lossPart, lossSlots, logdetRows, status, reduceDesc;
+    DevBuf comps, cm, cmFx, cmScale, gather, items, partials, rowBase, lossPart, lossSlots, logdetRows, status, reduceDesc;
     DevBuf stage[8];
     std::vector<CompDesc> hostComps;
     std::vector<GatherDescHost> hostGather;
@@ -344,14 +344,11 @@ struct MapWorkspace {
 
 // Coefficient gather over several components (separate translation unit needs no kernel here).
 namespace mpgb {
-__global__ void gatherMultiKernel(const GatherDescHost* descs, int nComps, double* cm) {
-    const int c = blockIdx.y;
-    if (c >= nComps) return;
-    const GatherDescHost g = descs[c];
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < g.nSlots; s += gridDim.x * blockDim.x) {
-        const int t = g.slotTerm[s];
-        cm[g.slotOffset + s] = (t >= 0) ? g.src[t] : 0.0;
-    }
+__global__ void __launch_bounds__(512) gatherMultiKernel(const GatherDescHost* descs, double* cm, int2* cmFx,
+                                                         int* scale) {
+    const GatherDescHost g = descs[blockIdx.x];
+    gatherComponent(g.src, g.slotTerm, g.nSlots, cm + g.slotOffset, cmFx ? cmFx + g.slotOffset : nullptr,
+                    scale + blockIdx.x, kNoLimbs);
 }
 
 __global__ void sumRowsKernel(const double* rows, int nRows, long long N, double* out, long long outStride) {
@@ -620,13 +617,14 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
             c.sigC = p.dSigC; c.sigW = p.dSigW; c.sigWt = p.dSigWt; c.sigStart = p.dSigStart;
             c.sigN = (int)p.sigC.size(); c.sigNStarts = (int)p.sigStart.size(); c.rectify = p.kind == 1 ? 1 : 0;
             c.nodeCIdx = p.dNodeCIdx;
+            c.nodeCRow = p.dNodeCRow;
             W.hostComps.push_back(c);
             slotOff += p.nSlots;
             pm = std::max(pm, p.P);
             W.dmax = std::max(W.dmax, p.D);
             W.nBmax = std::max(W.nBmax, p.nB);
             W.depthMax = std::max(W.depthMax, p.maxDepth);
-            if (p.kind == 0 && p.nSlots + p.nNodes <= kStageCap) W.stageNeed = std::max(W.stageNeed, p.nSlots + p.nNodes);
+            if (p.kind == 0) W.stageNeed = std::max(W.stageNeed, std::max(kStageMin, std::min(kStageCap, p.nSlots + 2 * (p.nNodes + 2))));
         }
         MPGB_CUDA(cudaDeviceGetAttribute(&W.smemPerSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
         W.totalSlots = slotOff;
@@ -642,6 +640,8 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
         MPGB_CUDA(cudaMemcpy(W.comps.p, W.hostComps.data(), W.hostComps.size() * sizeof(CompDesc),
                              cudaMemcpyHostToDevice));
         W.cm.ensure(std::max(1, W.totalSlots) * sizeof(double), stream);
+        W.cmFx.ensure((W.totalSlots + 1) * sizeof(int2), stream);
+        W.cmScale.ensure(W.hostComps.size() * sizeof(int), stream);
         W.status.ensure(sizeof(int) * 4, stream);
         MPGB_CUDA(cudaMemset(W.status.p, 0, sizeof(int) * 4));
         W.built = true;
@@ -663,10 +663,9 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
         MPGB_CUDA(cudaStreamSynchronize(stream));
         W.hostGather = g;
     }
-    int maxSlots = 1;
-    for (auto& x : g) maxSlots = std::max(maxSlots, x.nSlots);
-    dim3 grid((maxSlots + 255) / 256, (unsigned)g.size());
-    gatherMultiKernel<<<grid, 256, 0, stream>>>(W.gather.as<GatherDescHost>(), (int)g.size(), W.cm.as<double>());
+    const bool limbs = limbMap(W.basis, W.pmax);
+    gatherMultiKernel<<<(unsigned)g.size(), 512, 0, stream>>>(W.gather.as<GatherDescHost>(), W.cm.as<double>(),
+                                                              limbs ? W.cmFx.as<int2>() : nullptr, W.cmScale.as<int>());
     MPGB_CUDA(cudaGetLastError());
     countLaunches(stream, 1);
 }
@@ -759,6 +758,8 @@ void checkMatrix(const StridedMatrix& m, int64_t rows, int64_t cols, const char*
 static void baseParams(MapWorkspace& W, const MapOptions& o, FusedParams& p, long long N) {
     p.comps = W.comps.as<CompDesc>();
     p.cm = W.cm.as<double>();
+    p.cmFx = limbMap(W.basis, W.pmax) ? W.cmFx.as<int2>() : nullptr;
+    p.cmScale = W.cmScale.as<int>();
     p.N = N;
     p.tpb = kTpb;
     p.nugget = o.nugget;
@@ -865,14 +866,21 @@ static void orderPoints(MapWorkspace& W, const std::vector<MonotoneMapBase::Part
     p.permStride = N;
 }
 
-// Phase A's inputs are staged in shared memory (FusedParams::stageDoubles)
-// when the staging does not lower the number of blocks an SM holds.
+// Phase A's inputs are staged in shared memory (FusedParams::stageDoubles):
+// the largest of the full need, halves of it and kStageMin that does not lower
+// the number of blocks an SM holds (phaseALimbs takes a component in chunks),
+// or kStageMin all the same.
 static int stageDoubles(const MapWorkspace& W, const FusedParams& p, bool input) {
     if (W.stageNeed == 0 || W.smemPerSM <= 0) return 0;
-    const size_t base = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, input) + 1024;
-    const size_t with = base + (size_t)W.stageNeed * sizeof(double);
+    const size_t base = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, input) + 2048;
     auto blocks = [&](size_t b) { return std::min<size_t>(kFusedBlocksPerSM, (size_t)W.smemPerSM / b); };
-    return (with <= 227 * 1024 && blocks(with) == blocks(base)) ? W.stageNeed : 0;
+    auto fits = [&](int n) {
+        const size_t with = base + (size_t)n * sizeof(double);
+        return with <= 227 * 1024 && blocks(with) == blocks(base);
+    };
+    for (int n = W.stageNeed; n >= kStageMin; n /= 2)
+        if (fits(n)) return n;
+    return base + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
 }
 
 static void launch(MapWorkspace& W, const MapOptions& o, FusedParams& p, int nItems, int needJ, int needE,

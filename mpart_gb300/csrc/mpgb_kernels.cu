@@ -334,7 +334,7 @@ void countLaunches(cudaStream_t stream, long long n) {
 long long launchCount() { return g_launches.load(std::memory_order_relaxed); }
 
 size_t fusedSmemBytes(int tpb, int dmax, int nBmax, int depthMax, int pmax, bool input) {
-    size_t n = (size_t)dmax * tpb + (size_t)nBmax * (tpb + 1) + (size_t)(depthMax + 1) * tpb +
+    size_t n = (size_t)dmax * tpb + (size_t)nBmax * (tpb + 1) + 1 + (size_t)(depthMax + 1) * tpb +
                (size_t)(pmax + 1) * tpb;
     if (input) {
         n += (size_t)nBmax * (tpb + 1) + (size_t)dmax * tpb +

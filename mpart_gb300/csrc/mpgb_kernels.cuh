@@ -370,9 +370,6 @@ struct NodePoly {
     }
 };
 
-// Largest last-input order the fixed-point quadrature is built for.
-constexpr int kFxMaxOrder = 6;
-
 // The quadrature of `integrate` in 64-bit fixed point (fx::integrate): the
 // coefficients a_k become those of d_D f(t x_D) as a polynomial in t, the
 // traversal integrates g and, for adjoints, the moments of g' t^j, and J and
@@ -547,10 +544,16 @@ struct SmemLayout {
     int bstride;
 };
 
+// The leading-basis table, rounded up so that what follows is 16-byte aligned
+// (reduceLimbs reads pairs of weights).
+__host__ __device__ inline size_t leadDoubles(int tpb, int nBmax) {
+    return ((size_t)nBmax * (tpb + 1) + 1) & ~(size_t)1;
+}
+
 __host__ __device__ inline size_t smemBytes(int tpb, int dmax, int nBmax, int depthMax, int pmax, bool input,
                                             int stageDoubles = 0) {
     const int sw = (depthMax + 1 > pmax + 1) ? depthMax + 1 : pmax + 1;
-    size_t n = (size_t)dmax * tpb + (size_t)nBmax * (tpb + 1) + (size_t)sw * tpb;
+    size_t n = (size_t)dmax * tpb + leadDoubles(tpb, nBmax) + (size_t)sw * tpb;
     if (input) {
         n += (size_t)dmax * tpb + (size_t)((depthMax + 1) * (depthMax + 2) / 2) * tpb;
     }
@@ -563,7 +566,7 @@ __device__ inline SmemLayout carveSmem(double* base, int tpb, int dmax, int nBma
     L.bstride = tpb + 1;
     double* p = base;
     L.X = p; p += (size_t)dmax * tpb;
-    L.B = p; p += (size_t)nBmax * (tpb + 1);
+    L.B = p; p += leadDoubles(tpb, nBmax);
     L.S = p;
     L.W = p;
     p += (size_t)((depthMax + 1 > pmax + 1) ? depthMax + 1 : pmax + 1) * tpb;
@@ -651,6 +654,254 @@ __device__ __forceinline__ void phaseAStaged(const CompDesc& c, const SmemLayout
 }
 
 // --------------------------------------------------------------------------
+// Phase A and the reduced adjoint in fixed point.
+//
+// Both are sums of products over a few hundred prefix nodes: 1.5 DFMA per node
+// each and a DMUL for the product, 1,380 of the 1,560 FP64 instructions a dim-8
+// order-4 point took once its quadrature was in fixed point.  A product of
+// limbs is three IMAD.WIDE and two shifts, a multiply-add three IMAD.WIDE.
+// A point's products are scaled by 2^-e with 2^e above any of them, so they
+// carry 57 fraction bits below that bound; points with e > kFxMaxScale or a
+// basis value of 16 or more ("outliers": far tails) keep FP64 products.
+// --------------------------------------------------------------------------
+constexpr int kFxMaxScale = 5;
+
+template <int BASIS, int PMAX>
+__host__ __device__ constexpr bool limbBasis() {
+    return limbMap(BASIS, PMAX);
+}
+
+// The leading-basis table of one point as limbs (int2 in the table's slots),
+// or as doubles (returns true) for an outlier; e as above.
+template <int BASIS>
+__device__ __forceinline__ bool fillLeadLimbs(const CompDesc& c, const SmemLayout& L, int tid, const BasisConsts& bc,
+                                              int& e) {
+    fillLead<BASIS>(c, L, tid, bc);
+    e = 0;
+    int top = 0;
+    for (int d = 0; d < c.D - 1; ++d) {
+        const int p = __ldg(&c.leadDeg[d]), r = __ldg(&c.rowOff[d]);
+        int ed = 0;
+        for (int k = 0; k < p; ++k) ed = max(ed, fx::expBound(L.B[(r + k) * L.bstride + tid]));
+        top = max(top, ed);
+        e += ed;
+    }
+    if (top > 4) return true;
+    if (e > kFxMaxScale) {
+        // The bound over the tree itself (a low-order term set has far smaller
+        // products than all inputs' largest values together).
+        int* E = reinterpret_cast<int*>(L.S + tid);  // (this thread's column of the stack)
+        E[0] = 0;
+        e = 0;
+        for (int n = 1; n < c.nNodes; ++n) {
+            const uint32_t w = __ldg(&c.nodeA[n]);
+            const int depth = w & 31;
+            const int x = E[(depth - 1) * 2 * (int)blockDim.x] + fx::expBound(L.B[(int)(w >> 18) * L.bstride + tid]);
+            E[depth * 2 * (int)blockDim.x] = x;
+            e = max(e, x);
+        }
+        if (e > kFxMaxScale) return true;
+    }
+    bool bad = false;
+    for (int r = 0; r < c.nB; ++r) {
+        double* b = &L.B[r * L.bstride + tid];
+        const long long v = fx::toFixed58(*b, bad);
+        *reinterpret_cast<int2*>(b) = make_int2((int)(v >> 31), (int)v & 0x7fffffff);
+    }
+    return false;
+}
+
+// Phase A of a tile from the points' limb tables.  The tree is staged in
+// shared memory in chunks that fit `room` doubles: per node one int4 (byte
+// offsets of its basis row, of its parent's stack row and of its first
+// coefficient, and nk), then the chunk's coefficient limbs.  The walk is a
+// chain (stack, product, stack), so the next node's operands are loaded while
+// the current product is formed, and a first child takes its parent from
+// registers.  Sums of 16 nodes in hh (2^-60) and m (2^-88), whose products
+// stay below 2^59 each, are folded into 96-bit totals: no bound on the whole
+// sum is needed.  out: see phaseA (limbs, one row per term-carrying node in
+// tree order).  Every thread of the block calls it; outliers only stage.
+template <int PMAX>
+__device__ __forceinline__ void phaseALimbs(const CompDesc& c, const SmemLayout& L, int tid, const int2* cl, int room,
+                                            bool outlier, int e, int scale, double* a, double* pc) {
+    const int tpb = blockDim.x;
+    const int rowB = tpb * 8;
+    long long hh[PMAX + 1], m[PMAX + 1];
+    unsigned long long lo[PMAX + 1];
+    int up[PMAX + 1];
+    fx::Limbs phi{1 << (30 - e), 0};
+#pragma unroll
+    for (int k = 0; k <= PMAX; ++k) { hh[k] = 0; m[k] = 1ll << 27; lo[k] = 0; up[k] = 0; }
+    auto fold = [&]() {
+#pragma unroll
+        for (int k = 0; k <= PMAX; ++k) {
+            const long long s = hh[k] + (m[k] >> 28);
+            lo[k] += (unsigned long long)s;
+            up[k] += (int)(s >> 63) + (lo[k] < (unsigned long long)s ? 1 : 0);
+            hh[k] = 0;
+            m[k] = 1ll << 27;
+        }
+    };
+    auto term = [&](int k, int2 w) {
+        hh[k] = fx::madWideS(phi.h, w.x, hh[k]);
+        m[k] = fx::madWideS(phi.h, w.y, m[k]);
+        m[k] = fx::madWideS(phi.l << 1, w.x, m[k]);
+    };
+    const char* Bb = reinterpret_cast<const char*>(L.B + tid);
+    char* Sb = reinterpret_cast<char*>(L.S + tid);
+    int2* out = reinterpret_cast<int2*>(pc) + tid;
+    auto ld2 = [](const char* q) { return *reinterpret_cast<const int2*>(q); };
+    // The root (phi = 1).
+    *reinterpret_cast<int2*>(Sb) = make_int2(phi.h, phi.l);
+    {
+        const int nk = (__ldg(&c.nodeA[0]) >> 5) & 31;
+        if (nk && pc) {
+            *out = make_int2(phi.h, phi.l);
+            out += tpb;
+        }
+#pragma unroll
+        for (int k = 0; k <= PMAX; ++k)
+            if (k < nk) term(k, __ldg(&cl[k]));
+    }
+    int4* tab = reinterpret_cast<int4*>(L.stage);
+    const int left = c.nNodes - 1;
+    // (two look-ahead entries, and a coefficient past the last)
+    const int chunk = (2 * (left + 3) + c.nSlots <= room) ? left : max(1, (room - 6) / (2 + PMAX + 1));
+    for (int n0 = 1; n0 < c.nNodes; n0 += chunk) {
+        const int cnt = min(chunk, c.nNodes - n0);
+        const int s0 = (int)__ldg(&c.nodeSlot[n0]);
+        const int s1 = n0 + cnt < c.nNodes ? (int)__ldg(&c.nodeSlot[n0 + cnt]) : c.nSlots;
+        char* cs = reinterpret_cast<char*>(tab + cnt + 2);
+        __syncthreads();
+        for (int j = tid; j < cnt + 2; j += tpb) {
+            const int n = n0 + min(j, cnt - 1);  // (two more entries for the look-ahead)
+            const uint32_t w = __ldg(&c.nodeA[n]);
+            tab[j] = make_int4((int)(w >> 18) * L.bstride * 8, ((int)(w & 31) - 1) * rowB,
+                               ((int)__ldg(&c.nodeSlot[n]) - s0) * 8, (int)(w >> 5) & 31);
+        }
+        for (int j = tid; j < s1 - s0; j += tpb) reinterpret_cast<int2*>(cs)[j] = __ldg(&cl[s0 + j]);
+        __syncthreads();
+        if (outlier) continue;
+        int4 tA = tab[0], tB = tab[1];
+        int2 b = ld2(Bb + tA.x), par = ld2(Sb + tA.y), c0 = ld2(cs + tA.z);
+#pragma unroll 4
+        for (int i = 0; i < cnt; ++i) {
+            const int4 tC = tab[i + 2];
+            const int2 bN = ld2(Bb + tB.x), pN = ld2(Sb + tB.y), cN = ld2(cs + tB.z);
+            phi = fx::limbMul({par.x, par.y}, b.x, b.y);
+            const int own = tA.y + rowB;
+            *reinterpret_cast<int2*>(Sb + own) = make_int2(phi.h, phi.l);
+            const int nk = tA.w;
+            if (nk) {
+                if (pc) {
+                    *out = make_int2(phi.h, phi.l);
+                    out += tpb;
+                }
+                term(0, c0);
+                const char* ck = cs + tA.z;
+#define MPGB_TERM(K) if constexpr (K <= PMAX) if (nk > K) { term(K, ld2(ck + 8 * K));
+                MPGB_TERM(1) MPGB_TERM(2) MPGB_TERM(3) MPGB_TERM(4) MPGB_TERM(5) MPGB_TERM(6)
+                }}}}}}
+#undef MPGB_TERM
+            }
+            if ((i & 15) == 15) fold();
+            par = tB.y == own ? make_int2(phi.h, phi.l) : pN;
+            tA = tB;
+            tB = tC;
+            b = bN;
+            c0 = cN;
+        }
+        fold();
+    }
+    if (outlier) return;
+    fold();
+    const double sc = ldexp(1.0, e + scale - 60);
+#pragma unroll
+    for (int k = 0; k <= PMAX; ++k) {
+        double v = (double)(long long)lo[k];
+        // (a total beyond 64 bits)
+        if (up[k] != (int)((long long)lo[k] >> 63)) v = fma((double)up[k], 0x1p64, (double)lo[k]);
+        a[k] = v * sc;
+    }
+}
+
+// Sum over the tile's points of phi_n W_k for the nodes of one component, from
+// the products kept by phaseALimbs (rc) and the weights' limbs W ((h 2^30 + l)
+// 2^-59 2^sE[k], |l| <= 2^29), added to the partial row.  Eight lanes share a
+// node (nodes sorted by nk: the orders of a warp's four nodes run together),
+// two points each at a time: 16-byte loads, whole lines of rc, the next
+// nodes' lines in flight during the sums.
+template <int PMAX>
+__device__ __forceinline__ void reduceLimbs(const CompDesc& c, const double* rc, const double* W, const int* sE,
+                                            double* part) {
+    const int tid = threadIdx.x, tpb = blockDim.x;
+    const int lane = tid & 31, q = lane & 7;
+    const int perNode = tpb >> 1;  // int4 per row (8 lanes x 4 or 8)
+    const bool two = perNode > 32;
+    const int4* Wl = reinterpret_cast<const int4*>(W) + q;
+    const int step = tpb >> 3;
+    uint32_t w = 0;
+    int4 p[8], nx[8];
+    auto fetch = [&](int n, int4* v) {
+        w = n < c.nCNodes ? __ldg(&c.nodeC[n]) : 0;
+        const int4* row =
+            reinterpret_cast<const int4*>(rc + (long long)(n < c.nCNodes ? (int)__ldg(&c.nodeCRow[n]) : 0) * tpb) + q;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) v[u] = (u < 4 || two) ? row[8 * u] : make_int4(0, 0, 0, 0);
+    };
+    int n0 = (tid >> 5) * 4;
+    if (n0 < c.nCNodes) fetch(n0 + (lane >> 3), nx);
+    for (; n0 < c.nCNodes; n0 += step) {
+        const int nk = (w >> 5) & 31, slot = w >> 10;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) p[u] = nx[u];
+        if (n0 + step < c.nCNodes) fetch(n0 + step + (lane >> 3), nx);
+        const int nkm = __reduce_max_sync(0xffffffffu, nk);
+        long long mine = 0;
+#pragma unroll
+        for (int k = 0; k <= PMAX; ++k) {
+            if (k < nkm) {
+                long long hh = 0, m1 = 0, m2 = 0;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    if (u == 4) {
+                        if (!two) break;
+                        hh += m1 >> 30;  // (eight points: m1 below 2^62)
+                        m1 &= (1ll << 30) - 1;
+                    }
+                    const int4 x = Wl[k * perNode + 8 * u], v = p[u];
+                    hh = fx::madWideS(v.x, x.x, hh);
+                    m1 = fx::madWideS(v.x, x.y, m1);
+                    m2 = fx::madWideS(v.y, x.x, m2);
+                    hh = fx::madWideS(v.z, x.z, hh);
+                    m1 = fx::madWideS(v.z, x.w, m1);
+                    m2 = fx::madWideS(v.w, x.z, m2);
+                }
+                // Eight lanes' sums need three more bits: the low ones, and
+                // eight of the fraction, apart.  Rounded once, ties to even:
+                // halves up in every sum would add to several of its ulps at
+                // 1M points.
+                m1 += m2 << 3;
+                long long s = hh + (m1 >> 30);
+                int low = ((int)s & 7) << 8 | ((int)(m1 >> 22) & 255);
+                s >>= 3;
+#pragma unroll
+                for (int o = 1; o < 8; o <<= 1) {
+                    s += __shfl_xor_sync(0xffffffffu, s, o);
+                    low += __shfl_xor_sync(0xffffffffu, low, o);
+                }
+                s += (low + 1023 + (int)((s + (low >> 11)) & 1)) >> 11;
+                if (q == k) mine = s;
+            }
+        }
+        if (q < nk) {
+            const int t = __ldg(&c.slotTerm[slot + q]);
+            if (t >= 0) part[t] += (double)mine * ldexp(1.0, sE[q] - 56);
+        }
+    }
+}
+
+// --------------------------------------------------------------------------
 // Sigmoid expansions (no quadrature).
 // --------------------------------------------------------------------------
 // Phase A of a sigmoid expansion: a_0 = sum_m c_(m,0) Phi_m and, for k >= 1,
@@ -730,14 +981,48 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
             const CompDesc& c = prm.comps[ci];
             const double* cm = prm.cm + c.slotOffset;
             const int P = c.P;
-            fillLead<BASIS>(c, L, tid, prm.bc);
+            // The reduced adjoint adds to the item's partial rows.
+            if ((flags & kFlagCoefReduced) && tj == 0)
+                for (long long k = tid; k < (long long)c.cSegs * c.numTerms; k += tpb)
+                    prm.partials[item.partialBase + k] = 0.0;
+            // Fixed-point phase A (and reduction): launches that need neither
+            // per-term outputs nor input gradients, which read the FP64 table.
+            constexpr bool kLimbs = limbBasis<BASIS, PMAX>();
+            bool limbs = false, outlier = false;
+            int phiScale = 0, cScale = 0;
+            if constexpr (kLimbs) {
+                if (prm.cmFx && prm.stageDoubles >= kStageMin && !(flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput))) {
+                    cScale = __ldg(&prm.cmScale[ci]);
+                    limbs = cScale != kNoLimbs;
+                }
+            }
+            if (limbs) {
+                outlier = fillLeadLimbs<BASIS>(c, L, tid, prm.bc, phiScale);
+                // A warp with an outlier walks the tree twice: with more than
+                // one per warp on average the whole tile takes FP64.
+                if (__syncthreads_count(outlier) > (tpb >> 5)) {
+                    limbs = false;
+                    if (!outlier) fillLead<BASIS>(c, L, tid, prm.bc);
+                    outlier = false;
+                }
+            } else {
+                fillLead<BASIS>(c, L, tid, prm.bc);
+            }
 
             double a[PMAX + 1];
             // (sigmoid expansions: the rectified products R(Phi_m) of this tile,
             // kept for the reduction below)
             // (monotone components: the products of the deeper prefix nodes)
-            double* rc = (prm.rcache && (flags & kFlagCoefReduced)) ? prm.rcache + item.rcBase : nullptr;
-            if constexpr (BASIS == kBasisSigmoid) {
+            double* rc = (prm.rcache && (flags & kFlagCoefReduced))
+                             ? prm.rcache + (BATCH ? blockIdx.x * prm.rcStride : item.rcBase)
+                             : nullptr;
+            if (kLimbs && limbs) {
+                if constexpr (kLimbs) {
+                    phaseALimbs<PMAX>(c, L, tid, prm.cmFx + c.slotOffset, prm.stageDoubles, outlier, phiScale, cScale, a,
+                                      rc);
+                    if (outlier) phaseA<PMAX>(c, L, tid, cm, a, nullptr);
+                }
+            } else if constexpr (BASIS == kBasisSigmoid) {
                 phaseARect<PMAX, POS>(c, L, tid, cm, a, rc);
             } else if (c.nSlots + c.nNodes <= prm.stageDoubles) {
                 // The tree walk reads a coefficient and two table words per
@@ -949,12 +1234,90 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                 if (!(flags & kFlagImplicit)) *g += gxd;  // implicit mode keeps lambda there
             }
 
-            // Reduced combined adjoint: owner-computes over the block's points.
-            if (flags & kFlagCoefReduced) {
+            // Reduced combined adjoint in fixed point; outliers and points
+            // with weights that are not finite follow in FP64, eight at a time
+            // in the order of the tile.
+            if (kLimbs && limbs && rc) {
+                if constexpr (kLimbs) {
+                    constexpr int kRound = 8;
+                    __shared__ int sMax[PMAX + 1];
+                    __shared__ unsigned sOut[4];
+                    __shared__ double sOutW[kRound][PMAX + 1];
+                    __shared__ int sOutIdx[kRound];
+                    double w[PMAX + 1];
+                    bool skip = outlier;
+#pragma unroll
+                    for (int k = 0; k <= PMAX; ++k) {
+                        w[k] = wT[k] + wL[k];
+                        skip |= fx::expBound(w[k]) > 1024;
+                    }
+                    if (skip && !outlier) fillLead<BASIS>(c, L, tid, prm.bc);
+                    if (tid <= PMAX) sMax[tid] = -4096;
+                    __syncthreads();
+#pragma unroll
+                    for (int k = 0; k <= PMAX; ++k) {
+                        const int b = __reduce_max_sync(0xffffffffu, skip ? -4096 : fx::expBound(w[k]) + phiScale + 1);
+                        if ((tid & 31) == 0) atomicMax(&sMax[k], b);
+                    }
+                    const unsigned om = __ballot_sync(0xffffffffu, skip);
+                    if ((tid & 31) == 0) sOut[tid >> 5] = om;
+                    __syncthreads();
+#pragma unroll
+                    for (int k = 0; k <= PMAX; ++k) {
+                        const long long v = skip ? 0 : fx::toFixed(w[k], phiScale + 59 - sMax[k]);
+                        const long long h = (v + (1ll << 29)) >> 30;
+                        reinterpret_cast<int2*>(L.W)[k * tpb + tid] = make_int2((int)h, (int)(v - (h << 30)));
+                    }
+                    __syncthreads();
+                    double* part = prm.partials + item.partialBase;
+                    reduceLimbs<PMAX>(c, rc, L.W, sMax, part);
+                    int nOut = 0, rank = 0;
+                    for (int q = 0; q < (tpb >> 5); ++q) {
+                        const unsigned x = sOut[q];
+                        nOut += __popc(x);
+                        if (q < (tid >> 5)) rank += __popc(x);
+                        else if (q == (tid >> 5)) rank += __popc(x & ((1u << (tid & 31)) - 1u));
+                    }
+                    for (int r0 = 0; r0 < nOut; r0 += kRound) {
+                        __syncthreads();
+                        if (skip && rank >= r0 && rank < r0 + kRound) {
+                            sOutIdx[rank - r0] = tid;
+#pragma unroll
+                            for (int k = 0; k <= PMAX; ++k) sOutW[rank - r0][k] = w[k];
+                        }
+                        __syncthreads();
+                        const int m = min(kRound, nOut - r0);
+                        for (int n = tid; n < c.nCNodes; n += tpb) {
+                            const uint32_t nw = __ldg(&c.nodeC[n]);
+                            const int depth = nw & 31, nk = (nw >> 5) & 31, slot = nw >> 10;
+                            const uint16_t* rows = c.nodeCRows + (size_t)n * kMaxDepth;
+                            double acc[PMAX + 1];
+#pragma unroll
+                            for (int k = 0; k <= PMAX; ++k) acc[k] = 0.0;
+                            for (int o = 0; o < m; ++o) {
+                                double phi = 1.0;
+                                for (int d = 0; d < depth; ++d)
+                                    phi *= L.B[(int)__ldg(&rows[d]) * L.bstride + sOutIdx[o]];
+                                accumSlots<PMAX>(nk, phi, sOutW[o], 1, acc);
+                            }
+#pragma unroll
+                            for (int k = 0; k <= PMAX; ++k) {
+                                if (k < nk) {
+                                    const int t = __ldg(&c.slotTerm[slot + k]);
+                                    if (t >= 0) part[t] += acc[k];
+                                }
+                            }
+                        }
+                    }
+                    __syncthreads();
+                }
+            } else if (flags & kFlagCoefReduced) {
+                // Owner-computes over the block's points, in FP64 (no room for
+                // the kept products, or no limbs).
+                if (limbs && !outlier) fillLead<BASIS>(c, L, tid, prm.bc);
 #pragma unroll
                 for (int k = 0; k <= PMAX; ++k) L.W[k * tpb + tid] = wT[k] + wL[k];
                 __syncthreads();
-                const bool first = (tj == 0);
                 // Units (node, point segment); consecutive threads share a node.
                 const int S = c.cSegs;
                 const int segLen = tpb / S;
@@ -1007,7 +1370,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                             const int t = __ldg(&c.slotTerm[slot + k]);
                             if (t >= 0) {
                                 double* dst = part + t;
-                                *dst = first ? acc[k] : (*dst + acc[k]);
+                                *dst += acc[k];
                             }
                         }
                     }
@@ -1050,7 +1413,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
 
 template <int BASIS, int POS, int PMAX, bool NEEDJ, int NEEDE>
 __global__ void __launch_bounds__(128, kFusedBlocksPerSM) fusedKernel(const __grid_constant__ FusedParams prm) {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     fusedBody<BASIS, POS, PMAX, NEEDJ, NEEDE, false>(prm, prm.items[blockIdx.x], smem);
 }
 
@@ -1068,7 +1431,7 @@ __global__ void __launch_bounds__(128, kFusedBlocksPerSM) fusedKernel(const __gr
 template <int BASIS, int POS, int MAXC>
 __global__ void __launch_bounds__(128, (MAXC <= 4) ? 4 : 2) batchKernel(const __grid_constant__ FusedParams prm,
                                                                        int nItems, int* counter) {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     __shared__ int next;
     for (;;) {
         if (threadIdx.x == 0) next = atomicAdd(counter, 1);
@@ -1363,7 +1726,7 @@ __device__ __forceinline__ void solveLockstep(bool need, const F& f, double yd, 
 
 template <int BASIS, int POS, int PMAX>
 __global__ void __launch_bounds__(256) inverseKernel(const __grid_constant__ InverseParams prm) {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     const int tid = threadIdx.x;
     const int tpb = blockDim.x;
     const SmemLayout L = carveSmem(smem, tpb, prm.dmax, prm.nBmax, prm.depthMax, PMAX, false);
@@ -1949,7 +2312,7 @@ __global__ void __launch_bounds__(128) inverseWarpKernel(const __grid_constant__
 // to the range [0, x] they integrate, which the estimate predicts.
 template <int BASIS, int POS, int PMAX>
 __global__ void __launch_bounds__(256) inverseKeyKernel(const __grid_constant__ InverseParams prm) {
-    extern __shared__ double smem[];
+    extern __shared__ __align__(16) double smem[];
     const int tid = threadIdx.x;
     const int tpb = blockDim.x;
     const SmemLayout L = carveSmem(smem, tpb, prm.dmax, prm.nBmax, prm.depthMax, PMAX, false);
@@ -2024,7 +2387,8 @@ cudaError_t launchBatchP(const FusedParams& prm, int nItems, int pmaxClass, int*
     if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, prm.tpb, smem)) != cudaSuccess) return e;
     if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
     if ((e = cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
-    const int grid = std::max(1, std::min(nItems, std::max(1, perSM) * nSM));
+    int grid = std::max(1, std::min(nItems, std::max(1, perSM) * nSM));
+    if (prm.rcache) grid = std::min(grid, prm.rcBlocks);
     kern<<<grid, prm.tpb, smem, stream>>>(prm, nItems, counter);
     e = cudaGetLastError();
     countLaunches(stream, 1);

@@ -87,14 +87,9 @@ struct GatherDesc {
     int nSlots;
 };
 
-__global__ void gatherNA(const GatherDesc* descs, int nComps, double* cm) {
-    const int c = blockIdx.y;
-    if (c >= nComps) return;
-    const GatherDesc g = descs[c];
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < g.nSlots; s += gridDim.x * blockDim.x) {
-        const int t = g.slotTerm[s];
-        cm[g.slotOffset + s] = (t >= 0) ? g.src[t] : 0.0;
-    }
+__global__ void __launch_bounds__(512) gatherNA(const GatherDesc* descs, double* cm, int2* cmFx, int* scale) {
+    const GatherDesc g = descs[blockIdx.x];
+    gatherComponent(g.src, g.slotTerm, g.nSlots, cm + g.slotOffset, cmFx + g.slotOffset, scale + blockIdx.x, kNoLimbs);
 }
 
 // Bump allocator over the static array (offsets only; nothing is allocated).
@@ -201,6 +196,8 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
     const size_t oItems = cv.take(std::max<size_t>(1, items.size()) * sizeof(WorkItem));
     const size_t oRows = cv.take(std::max<size_t>(1, rowBase.size()) * sizeof(long long));
     const size_t oCm = cv.take(std::max(1, slotOff) * sizeof(double));
+    const size_t oCmFx = cv.take((slotOff + 1) * sizeof(int2));
+    const size_t oScale = cv.take(nComps * sizeof(int));
     const size_t oPart = cv.take(std::max<long long>(1, partBase) * sizeof(double));
     if (cv.used > kNoAllocScratchBytes) {
         std::ostringstream os;
@@ -217,9 +214,8 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         MPGB_CUDA(cudaMemcpyAsync(base + oRows, rowBase.data(), rowBase.size() * sizeof(long long), cudaMemcpyHostToDevice, stream));
     }
     double* cm = (double*)(base + oCm);
-    int maxSlots = 1;
-    for (auto& g : gather) maxSlots = std::max(maxSlots, g.nSlots);
-    gatherNA<<<dim3((maxSlots + 255) / 256, nComps), 256, 0, stream>>>((const GatherDesc*)(base + oGather), nComps, cm);
+    gatherNA<<<nComps, 512, 0, stream>>>((const GatherDesc*)(base + oGather), cm, (int2*)(base + oCmFx),
+                                         (int*)(base + oScale));
     MPGB_CUDA(cudaGetLastError());
     countLaunches(stream, 1);
 
@@ -229,6 +225,8 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         p.comps = (const CompDesc*)(base + oComps);
         p.items = (const WorkItem*)(base + oItems);
         p.cm = cm;
+        p.cmFx = limbMap(o.basisType == BasisTypes::HermiteFunctions ? kBasisHermiteFunctions : kBasisProbHermite, pmax) ? (const int2*)(base + oCmFx) : nullptr;
+        p.cmScale = (const int*)(base + oScale);
         p.N = N;
         p.tpb = kTpbNA;
         p.pts = pts.data; p.ptsRs = pts.row_stride; p.ptsCs = pts.col_stride;
@@ -262,6 +260,7 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         buildLaunchConstants(o, p.quad, p.bc);
         const size_t smem = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, pmax, false);
         if (smem > 227 * 1024) throw std::invalid_argument("component too large for the shared-memory tile");
+        p.stageDoubles = smem + 2048 + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
         const int basis = o.basisType == BasisTypes::HermiteFunctions ? kBasisHermiteFunctions : kBasisProbHermite;
         const int pos = o.posFuncType == PosFuncTypes::Exp ? kPosExp : kPosSoftPlus;
         if (p.flags) MPGB_CUDA(launchFused(basis, pos, pmax, p, (int)items.size(), needJ, 0, stream));

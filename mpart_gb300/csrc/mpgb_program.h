@@ -86,10 +86,10 @@ struct ComponentProgram {
     int D = 0, P = 0, nB = 0, nNodes = 0, nSlots = 0, nCNodes = 0, maxDepth = 0, numTerms = 0;
     std::vector<uint32_t> nodeA, nodeSlot, nodeC;
     std::vector<uint16_t> nodeCRows;
-    std::vector<int32_t> slotTerm, leadDeg, rowOff, nodeCIdx;
+    std::vector<int32_t> slotTerm, leadDeg, rowOff, nodeCIdx, nodeCRow;
     uint32_t *dNodeA = nullptr, *dNodeSlot = nullptr, *dNodeC = nullptr;
     uint16_t* dNodeCRows = nullptr;
-    int32_t *dSlotTerm = nullptr, *dLeadDeg = nullptr, *dRowOff = nullptr, *dNodeCIdx = nullptr;
+    int32_t *dSlotTerm = nullptr, *dLeadDeg = nullptr, *dRowOff = nullptr, *dNodeCIdx = nullptr, *dNodeCRow = nullptr;
     // Work per point (FP64 operations of phases A and C), for load balancing.
     double weight = 1.0;
     // Integrand dimension of the reference component's quadrature object,
@@ -220,7 +220,12 @@ struct ComponentProgram {
         {
             std::vector<int> cOf(tn.size(), -1);
             for (int j = 0; j < nCNodes; ++j) cOf[cn[j]] = j;
-            for (int n : order) nodeCIdx.push_back(cOf[n]);
+            nodeCRow.assign(nCNodes, 0);
+            int rank = 0;
+            for (int n : order) {
+                nodeCIdx.push_back(cOf[n]);
+                if (cOf[n] >= 0) nodeCRow[cOf[n]] = rank++;
+            }
         }
         nodeCRows.assign((size_t)nCNodes * kMaxDepth, 0);
         double opsA = 0, opsC = 0;
@@ -244,6 +249,7 @@ struct ComponentProgram {
         dLeadDeg = toDevice(leadDeg);
         dRowOff = toDevice(rowOff);
         dNodeCIdx = toDevice(nodeCIdx);
+        dNodeCRow = toDevice(nodeCRow);
         reserveNoAllocScratch();
     }
     ~ComponentProgram() {
@@ -255,6 +261,7 @@ struct ComponentProgram {
         cudaFree(dLeadDeg);
         cudaFree(dRowOff);
         cudaFree(dNodeCIdx);
+        cudaFree(dNodeCRow);
         cudaFree(dSigC);
         cudaFree(dSigW);
         cudaFree(dSigWt);
