@@ -115,6 +115,14 @@ __global__ void segScatterKernel(const SortSeg* segs, const int* chunkSeg, const
     __syncwarp();
     const long long base = (long long)(blockIdx.x - sg.chunk0) * kChunk;
     const unsigned lt = (1u << lane) - 1u;
+    // (the chunk's keys in flight together)
+    double x[kChunk / 32];
+#pragma unroll
+    for (int c = 0; c < kChunk / 32; ++c) {
+        const long long i = base + c * 32 + lane;
+        x[c] = i < sg.N ? sg.xd[i * sg.stride] : 0.0;
+    }
+#pragma unroll
     for (int c = 0; c < kChunk / 32; ++c) {
         const long long i = base + c * 32 + lane;
         const bool active = i < sg.N;

@@ -844,6 +844,27 @@ static void uploadItems(MapWorkspace& W, const std::vector<WorkItem>& items, cud
                               stream));
 }
 
+// Sorts every component's points (or onlyComp's) by |x_D| of its own last
+// coordinate into perm + c * N: one launch set when the last coordinates are
+// consecutive rows, as in a triangular map.
+static cudaError_t sortComponents(const std::vector<MonotoneMapBase::Part>& parts, StridedMatrix const& pts,
+                                  int onlyComp, int* hist, int* perm, cudaStream_t stream) {
+    const long long N = pts.cols;
+    bool rows = onlyComp < 0;
+    for (size_t c = 0; c < parts.size(); ++c) rows = rows && parts[c].prog->D == parts[0].prog->D + (int)c;
+    if (rows)
+        return launchSortByLastSegments(pts.data + (int64_t)(parts[0].prog->D - 1) * pts.rowStride, pts.colStride,
+                                        pts.rowStride, (int)parts.size(), N, hist, perm, N, stream);
+    for (size_t c = 0; c < parts.size(); ++c) {
+        if (onlyComp >= 0 && (int)c != onlyComp) continue;
+        const cudaError_t e =
+            launchSortByLast(pts.data + (int64_t)(parts[c].prog->D - 1) * pts.rowStride, pts.colStride, N, hist,
+                             perm + c * (size_t)N, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
 // Processing order for per-component launches: each component's points
 // sorted (stably) by |x_D| of its own last coordinate.
 static void orderPoints(MapWorkspace& W, const std::vector<MonotoneMapBase::Part>& parts, StridedMatrix const& pts,
@@ -855,13 +876,8 @@ static void orderPoints(MapWorkspace& W, const std::vector<MonotoneMapBase::Part
     if (!W.ordering || N < 2 * kTpb || W.basis == kBasisSigmoid) return;
     const size_t nComps = parts.size();
     W.perm.ensure(nComps * (size_t)N * sizeof(int), stream);
-    W.sortHist.ensure(sortScratchInts(N) * sizeof(int), stream);
-    for (size_t c = 0; c < nComps; ++c) {
-        if (onlyComp >= 0 && (int)c != onlyComp) continue;
-        const double* xd = pts.data + (int64_t)(parts[c].prog->D - 1) * pts.rowStride;
-        MPGB_CUDA(launchSortByLast(xd, pts.colStride, N, W.sortHist.as<int>(), W.perm.as<int>() + c * (size_t)N,
-                                   stream));
-    }
+    W.sortHist.ensure(nComps * sortScratchInts(N) * sizeof(int), stream);
+    MPGB_CUDA(sortComponents(parts, pts, onlyComp, W.sortHist.as<int>(), W.perm.as<int>(), stream));
     p.perm = W.perm.as<int>();
     p.permStride = N;
 }
@@ -1419,12 +1435,7 @@ static void orderPointsKL(MapWorkspace& W, KLPlan& P, const std::vector<Monotone
         // room for the step's all-component cost-order sort as well, which
         // runs inside graph capture and so cannot allocate
         W.sortHist.ensure(nComps * sortScratchInts(N) * sizeof(int), stream);
-        for (size_t c = 0; c < nComps; ++c) {
-            if (onlyComp >= 0 && (int)c != onlyComp) continue;
-            const double* xd = pts.data + (int64_t)(parts[c].prog->D - 1) * pts.rowStride;
-            MPGB_CUDA(launchSortByLast(xd, pts.colStride, N, W.sortHist.as<int>(), P.perm.as<int>() + c * (size_t)N,
-                                       stream));
-        }
+        MPGB_CUDA(sortComponents(parts, pts, onlyComp, W.sortHist.as<int>(), P.perm.as<int>(), stream));
         cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
         MPGB_CUDA(cudaStreamIsCapturing(stream, &cs));
         if (cs == cudaStreamCaptureStatusNone) {

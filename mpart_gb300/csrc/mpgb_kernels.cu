@@ -57,8 +57,9 @@ constexpr int kSortChunk = 1024;
 
 __device__ __forceinline__ int sortKey(double x) { return sortBucket(x); }
 
-// Segment blockIdx.y of a multi-segment sort: keys at xd + y * keySeg,
-// histogram at hist + y * histSeg, permutation at perm + y * permSeg.
+// Segment blockIdx.y of a multi-segment sort: keys at xd + y * keySeg, counts
+// at hist + y * histSeg (bucket-major, [bucket][chunk], then the 256 bucket
+// totals), permutation at perm + y * permSeg.
 __global__ void keyHistKernel(const double* xd, long long stride, long long N, int* hist, long long keySeg,
                               long long histSeg) {
     xd += blockIdx.y * keySeg;
@@ -72,36 +73,36 @@ __global__ void keyHistKernel(const double* xd, long long stride, long long N, i
         if (i < N) atomicAdd(&h[sortKey(xd[i * stride])], 1);
     }
     __syncthreads();
-    for (int t = threadIdx.x; t < kSortBuckets; t += blockDim.x) hist[(long long)blockIdx.x * kSortBuckets + t] = h[t];
+    for (int t = threadIdx.x; t < kSortBuckets; t += blockDim.x) hist[(long long)t * gridDim.x + blockIdx.x] = h[t];
 }
 
-// One block of kSortBuckets threads: hist[blk][b] -> first output slot of (blk, b).
+// One warp per bucket: its chunk counts -> exclusive sums over the chunks, and
+// the bucket's total.  (One block walking all chunks of 256 buckets in turn
+// took 62 of the sort's 104 us at 1M points.)
 __global__ void keyScanKernel(int* hist, int nBlk, long long histSeg) {
-    hist += blockIdx.x * histSeg;  // one block per segment
-    __shared__ int tot[kSortBuckets];
-    const int b = threadIdx.x;
-    int s = 0;
-    for (int k = 0; k < nBlk; ++k) s += hist[(long long)k * kSortBuckets + b];
-    tot[b] = s;
-    __syncthreads();
-    if (b == 0) {
-        int run = 0;
-        for (int q = 0; q < kSortBuckets; ++q) {
-            const int v = tot[q];
-            tot[q] = run;
-            run += v;
+    hist += blockIdx.y * histSeg;
+    const int lane = threadIdx.x & 31;
+    const int b = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    int* row = hist + (long long)b * nBlk;
+    int run = 0;
+    for (int k0 = 0; k0 < nBlk; k0 += 32) {
+        const int k = k0 + lane;
+        const int v = k < nBlk ? row[k] : 0;
+        int s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += x;
         }
+        if (k < nBlk) row[k] = run + s - v;
+        run += __shfl_sync(0xffffffffu, s, 31);
     }
-    __syncthreads();
-    int run = tot[b];
-    for (int k = 0; k < nBlk; ++k) {
-        const int v = hist[(long long)k * kSortBuckets + b];
-        hist[(long long)k * kSortBuckets + b] = run;
-        run += v;
-    }
+    if (lane == 0) hist[(long long)kSortBuckets * nBlk + b] = run;
 }
 
-// One warp per chunk, chunk order kept within each bucket.
+// One warp per chunk, chunk order kept within each bucket.  The chunk's keys
+// are loaded together (a lane's loads one after another left the warp waiting
+// for memory 32 times: 30 us at any size).
 __global__ void keyScatterKernel(const double* xd, long long stride, long long N, const int* off, int* perm,
                                  long long keySeg, long long histSeg, long long permSeg) {
     xd += blockIdx.y * keySeg;
@@ -109,21 +110,50 @@ __global__ void keyScatterKernel(const double* xd, long long stride, long long N
     perm += blockIdx.y * permSeg;
     __shared__ int cnt[kSortBuckets];
     const int lane = threadIdx.x;
-    for (int t = lane; t < kSortBuckets; t += 32) cnt[t] = 0;
-    __syncwarp();
+    const int nBlk = gridDim.x;
     const long long base = (long long)blockIdx.x * kSortChunk;
+    double x[kSortChunk / 32];
+#pragma unroll
+    for (int c = 0; c < kSortChunk / 32; ++c) {
+        const long long i = base + c * 32 + lane;
+        x[c] = i < N ? xd[i * stride] : 0.0;
+    }
+    // First slot of (bucket, this chunk): eight buckets per lane.
+    {
+        int t[kSortBuckets / 32], s = 0;
+#pragma unroll
+        for (int q = 0; q < kSortBuckets / 32; ++q) {
+            t[q] = off[(long long)kSortBuckets * nBlk + lane * (kSortBuckets / 32) + q];
+            s += t[q];
+        }
+        int incl = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        int run = incl - s;
+#pragma unroll
+        for (int q = 0; q < kSortBuckets / 32; ++q) {
+            const int b = lane * (kSortBuckets / 32) + q;
+            cnt[b] = run + off[(long long)b * nBlk + blockIdx.x];
+            run += t[q];
+        }
+    }
+    __syncwarp();
     const unsigned lt = (1u << lane) - 1u;
+#pragma unroll
     for (int c = 0; c < kSortChunk / 32; ++c) {
         const long long i = base + c * 32 + lane;
         const bool active = i < N;
-        const int key = active ? sortKey(xd[i * stride]) : kSortBuckets + lane;
+        const int key = active ? sortKey(x[c]) : kSortBuckets + lane;
         const unsigned grp = __match_any_sync(0xffffffffu, key);
         const int rank = __popc(grp & lt);
         int slot = 0;
         if (active) slot = cnt[key];
         __syncwarp();
         if (active) {
-            perm[off[(long long)blockIdx.x * kSortBuckets + key] + slot + rank] = (int)i;
+            perm[slot + rank] = (int)i;
             if (rank == 0) cnt[key] = slot + __popc(grp);
         }
         __syncwarp();
@@ -381,7 +411,7 @@ cudaError_t launchSumLoss(const double* lossPart, const int* slots, int n, doubl
     return e;
 }
 
-size_t sortScratchInts(long long N) { return (size_t)((N + kSortChunk - 1) / kSortChunk) * kSortBuckets; }
+size_t sortScratchInts(long long N) { return (size_t)((N + kSortChunk - 1) / kSortChunk + 1) * kSortBuckets; }
 
 cudaError_t launchSortByLast(const double* xd, long long stride, long long N, int* hist, int* perm,
                              cudaStream_t stream) {
@@ -394,7 +424,7 @@ cudaError_t launchSortByLastSegments(const double* keys, long long stride, long 
     const int nBlk = (int)((N + kSortChunk - 1) / kSortChunk);
     const long long histSeg = (long long)sortScratchInts(N);
     keyHistKernel<<<dim3(nBlk, nSeg), 256, 0, stream>>>(keys, stride, N, hist, keySeg, histSeg);
-    keyScanKernel<<<nSeg, kSortBuckets, 0, stream>>>(hist, nBlk, histSeg);
+    keyScanKernel<<<dim3(kSortBuckets / 8, nSeg), 256, 0, stream>>>(hist, nBlk, histSeg);
     keyScatterKernel<<<dim3(nBlk, nSeg), 32, 0, stream>>>(keys, stride, N, hist, perm, keySeg, histSeg, permSeg);
     const cudaError_t e = cudaGetLastError();
     countLaunches(stream, 3);
