@@ -355,6 +355,75 @@ struct Threshold {
     int E;
 };
 
+// One interval of the rule from its five nodes (ends A, B, middle M, inner V,
+// W): the nodes' g on one exponent E (Exp), the fine sum ih (per unit width) and
+// whether |ih - ic| < max(relTol ic, (absTol / |x_D|) 2^level).
+struct Interval {
+    uint64_t a, b, m, v, w, ih;
+    int E;
+    bool small;
+};
+template <bool EXPR>
+MPGB_HD Interval intervalSums(const Node& A, const Node& B, const Node& V, const Node& M, const Node& W,
+                              const Rule& Q, Threshold thr, int level) {
+    Interval o;
+    o.a = A.g;
+    o.b = B.g;
+    o.m = M.g;
+    o.v = V.g;
+    o.w = W.g;
+    o.E = 0;
+    if constexpr (EXPR) {
+        int E = A.E > B.E ? A.E : B.E;
+        E = M.E > E ? M.E : E;
+        E = V.E > E ? V.E : E;
+        E = W.E > E ? W.E : E;
+        o.E = E;
+        o.a = shr(o.a, E - A.E);
+        o.b = shr(o.b, E - B.E);
+        o.m = shr(o.m, E - M.E);
+        o.v = shr(o.v, E - V.E);
+        o.w = shr(o.w, E - W.E);
+    }
+    const uint64_t ab = o.a + o.b, vw = o.v + o.w;
+    const uint64_t ic = mulhi(ab, Q.c0) + mulhi(o.m, Q.cM) + 1;
+    o.ih = mulhi(ab, Q.w0) + mulhi(o.m, Q.wM) + mulhi(vw, Q.w1) + 2;
+    const uint64_t err = o.ih > ic ? o.ih - ic : ic - o.ih;
+    uint64_t tol = mulhi(ic, Q.rel), ta;
+    if constexpr (EXPR) {
+        const int sh = o.E - thr.E - level;
+        ta = sh < 0 ? ~0ull : shr(thr.m, sh);
+    } else {
+        ta = (thr.m >> (63 - level)) ? ~0ull : thr.m << level;
+    }
+    tol = ta > tol ? ta : tol;
+    o.small = err < tol;
+    return o;
+}
+
+// Adds an accepted interval's fine sum to the value g 2^E (SoftPlus: E unused).
+// Exp: the exponent follows the largest contribution (the interval's exponent
+// less its level), so a narrow peak keeps its bits.
+template <bool EXPR>
+MPGB_HD void addValue(uint64_t ih, int E, int level, uint64_t& g, int& gE) {
+    int dn = level;
+    if constexpr (EXPR) {
+        const int e = E - level;
+        if (e > gE) {
+            g = shr(g, e - gE);
+            gE = e;
+        }
+        dn = gE - e;
+    }
+    g += shrRound(ih, dn);
+    if constexpr (EXPR) {
+        if (g >> 62) {
+            g >>= 1;
+            ++gE;
+        }
+    }
+}
+
 // The adaptive traversal of `integrate` (depth first, left first; the same
 // rule, accept test and order of accepted sums) on [0, 1].  An interval is
 // (lo, level), lo with 32 fraction bits and width 2^-level; the pending right
@@ -380,43 +449,13 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
         const uint64_t mid = ((uint64_t)lo << 32) + (0x8000000000000000ull >> level);
         const uint64_t dr = Q.rho >> (level + 1);
         const Node V = nodeAt<EXPR, D>(p, mid - dr), M = nodeAt<EXPR, D>(p, mid), W = nodeAt<EXPR, D>(p, mid + dr);
-        uint64_t a = A.g, b = B.g, m = M.g, v = V.g, w = W.g;
-        int E = 0;
-        if constexpr (EXPR) {
-            // One exponent for the interval's nodes.
-            E = A.E > B.E ? A.E : B.E;
-            E = M.E > E ? M.E : E;
-            E = V.E > E ? V.E : E;
-            E = W.E > E ? W.E : E;
-            a = shr(a, E - A.E);
-            b = shr(b, E - B.E);
-            m = shr(m, E - M.E);
-            v = shr(v, E - V.E);
-            w = shr(w, E - W.E);
-        }
-        const uint64_t ab = a + b, vw = v + w;
-        const uint64_t ic = mulhi(ab, Q.c0) + mulhi(m, Q.cM) + 1;
-        const uint64_t ih = mulhi(ab, Q.w0) + mulhi(m, Q.wM) + mulhi(vw, Q.w1) + 2;
-        const uint64_t err = ih > ic ? ih - ic : ic - ih;
-        // err < max(relTol ic, (absTol / |x_D|) 2^level)
-        uint64_t tol = mulhi(ic, Q.rel);
-        {
-            uint64_t ta;
-            if constexpr (EXPR) {
-                const int sh = E - thr.E - level;
-                ta = sh < 0 ? ~0ull : shr(thr.m, sh);
-            } else {
-                ta = (thr.m >> (63 - level)) ? ~0ull : thr.m << level;
-            }
-            tol = ta > tol ? ta : tol;
-        }
-        const bool accept = (err < tol || level == maxSub - 1) && level >= minSub;
+        const Interval q = intervalSums<EXPR>(A, B, V, M, W, Q, thr, level);
+        const uint64_t a = q.a, b = q.b, m = q.m, v = q.v, w = q.w, ih = q.ih;
+        const int E = q.E;
+        const bool accept = (q.small || level == maxSub - 1) && level >= minSub;
         ++count;
         if (accept) {
-            // Exp: the sums' exponent follows the largest contribution (the
-            // interval's exponent less its level), so a narrow peak keeps its
-            // bits.
-            int dn = level;
+            int dn = level;  // (exponents as in addValue)
             if constexpr (EXPR) {
                 const int e = E - level;
                 if (e > R.E) {

@@ -1724,6 +1724,130 @@ __device__ __forceinline__ void solveLockstep(bool need, const F& f, double yd, 
     }
 }
 
+// --------------------------------------------------------------------------
+// Inverse in fixed point.
+// --------------------------------------------------------------------------
+// What T(x_<D, x) - f(x_<D, 0) needs of a point: d_D f(x_<D, y) in powers of
+// y (times the envelope, plus a1, for Hermite functions) and the integrand's
+// node at t = 0, which no x_D changes.
+template <int BASIS, int POS, int PMAX>
+struct FixedPoint {
+    static constexpr bool EXPR = POS == kPosExp, ENV = BASIS == kBasisHermiteFunctions;
+    double s[PMAX], a1;
+    fx::Node A0;
+
+    // False: the point keeps FP64 (see integrateFixed).
+    __device__ bool init(const double* a, int P, const BasisConsts& bc) {
+        constexpr NodePoly<BASIS, PMAX> U;
+        double as[PMAX + 1];
+        scaleCoeffs<BASIS, PMAX>(a, P, bc, as);
+#pragma unroll
+        for (int j = 0; j < PMAX; ++j) {
+            double v = 0.0;
+#pragma unroll
+            for (int k = 0; k < PMAX; ++k) {
+                const double u = ENV ? (k >= 1 ? U.c[k >= 1 ? k - 1 : 0][j] : 0.0) : U.c[k][j];
+                if (u != 0.0) v = fma(u, as[k + 1], v);
+            }
+            s[j] = v;
+        }
+        a1 = ENV ? as[1] : 0.0;
+        bool bad = false;
+        fx::Poly<PMAX, ENV> p;
+        const long long q = fx::toFixed58(s[0], bad), q1 = fx::toFixed58(a1, bad);
+        bad |= q > (15ll << 58) || q < -(15ll << 58) || q1 > (15ll << 58) || q1 < -(15ll << 58);
+        if (!EXPR) bad |= q + q1 < -(4ll << 58);
+        if (bad) return false;
+#pragma unroll
+        for (int j = 0; j < PMAX; ++j) p.c[j] = 0x8000000000000000ull;
+        p.c[0] = (uint64_t)q + 0x8000000000000000ull;
+        p.a = (uint64_t)q1 + 0x8000000000000000ull;
+        p.Z = 0;
+        A0 = fx::nodeEnd<EXPR, false>(p, false);
+        return true;
+    }
+    // The quadrature at x: false where its range does not hold.
+    __device__ bool setup(double x, const QuadParams& Q, fx::Poly<PMAX, ENV>& p, fx::Threshold& thr) const {
+        bool bad = !(fabs(x) < 1e100);
+        uint32_t sum = 0;
+        double xp = 1.0;
+#pragma unroll
+        for (int j = 0; j < PMAX; ++j) {
+            const long long v = fx::toFixed58(j == 0 ? s[0] : s[j] * xp, bad);
+            xp = j == 0 ? x : xp * x;
+            sum += (uint32_t)((v < 0 ? -v : v) >> 35) + 1;
+            p.c[j] = (uint64_t)v + 0x8000000000000000ull;
+        }
+        p.a = p.Z = 0;
+        if constexpr (ENV) {
+            const long long v = fx::toFixed58(a1, bad);
+            sum += (uint32_t)((v < 0 ? -v : v) >> 35) + 1;
+            p.a = (uint64_t)v + 0x8000000000000000ull;
+            const double z = (x * x) * 0.72134752044448170368;
+            bad |= !(z < 126.0);
+            p.Z = bad ? 0 : (uint64_t)(z * 0x1p57);
+        }
+        bad |= sum > (31u << 23);
+        const double ta = Q.absTol / fabs(x);
+        if constexpr (EXPR) {
+            const uint64_t t = (uint64_t)__double_as_longlong(ta);
+            thr.m = ((t & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
+            thr.E = (int)(t >> 52) - 1023;
+        } else {
+            thr.m = ta < 32.0 ? (uint64_t)(ta * 0x1p57) : 1ull << 62;
+            thr.E = 0;
+        }
+        return !bad;
+    }
+    // The value of an integral, and of a node (the slope of T at t = 1).
+    static __device__ double value(uint64_t g, int E) {
+        if constexpr (EXPR) return (double)g * __longlong_as_double((long long)(E - 62 + 1023) << 52);
+        else return (double)g * 0x1p-57;
+    }
+};
+
+// T(x) of a monotone component for the lockstep solver: the fixed-point
+// quadrature wherever it holds at x, FP64 elsewhere -- the same function of x
+// in every inverse kernel, so that a root does not depend on which one found it.
+template <int BASIS, int POS, int PMAX>
+__device__ __noinline__ bool fixedValueNI(const FixedPoint<BASIS, POS, PMAX>* F, double x, const QuadParams* Q, double* I,
+                                          double* slope, int* st) {
+    using FP = FixedPoint<BASIS, POS, PMAX>;
+    fx::Poly<PMAX, FP::ENV> p;
+    fx::Threshold thr;
+    if (!F->setup(x, *Q, p, thr)) return false;
+    fx::Sums<0> S;
+    fx::integrate<FP::EXPR, PMAX, FP::ENV, 0>(p, Q->fx, Q->maxSub, Q->minSub, (int)Q->maxIntervals, thr, S);
+    if (S.over) {
+        *st |= kStatusBudget;
+        *I = __longlong_as_double(0x7ff8000000000000ULL);
+    } else {
+        *I = __dmul_rn(x, FP::value(S.g, S.E));  // (no contraction with the caller's sum)
+    }
+    const fx::Node B = fx::nodeEnd<FP::EXPR, false>(p, true);
+    *slope = FP::value(B.g, B.E);
+    return true;
+}
+
+template <int BASIS, int POS, int PMAX>
+struct InverseEvalFixed {
+    InverseEval<BASIS, POS, PMAX> f;
+    FixedPoint<BASIS, POS, PMAX> F;
+    bool ok;  // the point's fixed-point form holds
+    mutable bool known;
+    mutable double s;
+    __device__ double operator()(double x) const {
+        double I = 0.0, sl = 0.0;
+        int st = 0;
+        known = ok && fixedValueNI<BASIS, POS, PMAX>(&F, x, f.Q, &I, &sl, &st);
+        if (!known) return f(x);
+        *f.st |= st;
+        s = sl;
+        return I + f.f0;
+    }
+    __device__ double slope(double x) const { return known ? s : f.slope(x); }
+};
+
 template <int BASIS, int POS, int PMAX>
 __global__ void __launch_bounds__(256) inverseKernel(const __grid_constant__ InverseParams prm) {
     extern __shared__ __align__(16) double smem[];
@@ -1793,7 +1917,13 @@ __global__ void __launch_bounds__(256) inverseKernel(const __grid_constant__ Inv
             for (int k = 0; k <= PMAX; ++k) f0 = fma(A.a[k], prm.bc.v0[k], f0);
             int st = 0;
             InverseEval<BASIS, POS, PMAX> f{A, c.P, f0, &prm.quad, &prm.bc, prm.nugget, &st};
-            solveLockstep(mine && !hasNan, f, yd, x0, prm.xtol, prm.ytol, budget, prm.method, result, info);
+            if constexpr (PMAX <= kFxMaxOrder) {
+                InverseEvalFixed<BASIS, POS, PMAX> ff{f, {}, false, false, 0.0};
+                if (mine && prm.quad.fx.ok && prm.nugget == 0.0) ff.ok = ff.F.init(A.a, c.P, prm.bc);
+                solveLockstep(mine && !hasNan, ff, yd, x0, prm.xtol, prm.ytol, budget, prm.method, result, info);
+            } else {
+                solveLockstep(mine && !hasNan, f, yd, x0, prm.xtol, prm.ytol, budget, prm.method, result, info);
+            }
             stAll |= st;
         }
         if (!mine) continue;
@@ -2087,6 +2217,168 @@ __global__ void __launch_bounds__(128) inverseQueueKernel(const __grid_constant_
     if (prm.statusWord && stAll) atomicOr(prm.statusWord, stAll);
 }
 
+// Lanes of a warp that may still be in their quadratures when the others take
+// a solver step.  A step is some 60 FP64 instructions, as long on the SM as
+// three intervals of a whole warp, so it waits for most lanes; waiting for all
+// leaves lanes idle behind the widest quadrature.
+constexpr int kStepLanes = 8;
+
+// Inverse of one monotone component (compBegin) from the queue of points, in
+// fixed point: the solver of inverseQueueKernel (one point per lane, expensive
+// ones first), its quadratures traversed interval by interval on integers
+// (fx::integrate's arithmetic).  A point or an iterate out of the fixed-point
+// range, a quadrature of wideQuad intervals and a solve of nodeBudget nodes go,
+// with the solver's state, to the warp pass.
+template <int BASIS, int POS, int PMAX>
+__global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_constant__ InverseParams prm) {
+    using FP = FixedPoint<BASIS, POS, PMAX>;
+    constexpr bool EXPR = FP::EXPR, ENV = FP::ENV;
+    const QuadParams& Q = prm.quad;
+    const int comp = prm.compBegin;
+    const CompDesc& c = prm.comps[comp];
+    const int D = c.D, P = c.P;
+    const long long N = prm.N;
+    const int lane = threadIdx.x & 31;
+    const unsigned kFull = 0xffffffffu;
+    const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+
+    bool have = false, need = true, start = false, running = false, done = false;
+    long long i = 0;
+    double yd = 0.0, f0 = 0.0;
+    FP F;
+    RootSolve rs;
+    rs.phase = RootSolve::kDone;
+    fx::Poly<PMAX, ENV> p;
+    fx::Threshold thr{0, 0};
+    fx::Node A{}, B{}, E1{};
+    uint64_t G = 0;
+    int GE = 0, level = 0, nInt = 0, nodes = 0, stAll = 0;
+    uint32_t lo = 0, pend = 0;
+    uint64_t stG[32];
+    int stE[EXPR ? 32 : 1];
+    auto defer = [&]() {
+        const int slot = atomicAdd(prm.deferCount, 1);
+        prm.deferList[slot] = (int)i;
+        if (prm.deferState && slot < prm.deferStateCap)
+            rs.save(prm.deferState + (long long)slot * RootSolve::kSaveDoubles);
+        have = running = done = start = false;
+        need = true;
+    };
+
+    for (;;) {
+        const unsigned needMask = __ballot_sync(kFull, need);
+        if (needMask) {
+            const int leader = __ffs(needMask) - 1;
+            int base = 0;
+            if (lane == leader) base = atomicAdd(prm.queue, __popc(needMask));
+            base = __shfl_sync(kFull, base, leader);
+            if (need) {
+                const long long slot = (long long)base + __popc(needMask & ((1u << lane) - 1u));
+                need = false;
+                if (slot < N) {
+                    i = prm.perm ? (long long)prm.perm[N - 1 - slot] : slot;
+                    // fullOut = [x1; outputs so far] (TriangularMap.cpp:146-184); the
+                    // last coordinate is the initial guess.
+                    const long long xi = (prm.x1Cols == 1) ? 0 : i;
+                    bool hasNan = false;
+                    double x0 = 0.0;
+                    for (int d = 0; d < D; ++d) {
+                        double v = 0.0;
+                        if (d < prm.x1Rows) v = prm.x1[d * prm.x1Rs + xi * prm.x1Cs];
+                        else if (d - prm.extra < comp) v = prm.out[(long long)(d - prm.extra) * prm.outRs + i * prm.outCs];
+                        hasNan |= isnan(v);
+                        x0 = v;
+                    }
+                    if (hasNan) {
+                        // (MonotoneComponent.h:407-413)
+                        prm.out[(long long)comp * prm.outRs + i * prm.outCs] = nan;
+                        if (prm.info) prm.info[(long long)comp * prm.infoStride + i] = 0;
+                        need = true;
+                    } else {
+                        yd = prm.r[(long long)comp * prm.rRs + i * prm.rCs];
+                        double a[PMAX + 1];
+                        f0 = 0.0;
+#pragma unroll
+                        for (int k = 0; k <= PMAX; ++k) {
+                            a[k] = prm.acoef[(long long)k * N + i];
+                            f0 = fma(a[k], prm.bc.v0[k], f0);
+                        }
+                        rs.start(x0);
+                        nodes = 0;
+                        have = start = true;
+                        if (!F.init(a, P, prm.bc)) defer();
+                    }
+                }
+            }
+        }
+        if (!__any_sync(kFull, have || need)) break;
+        if (start) {
+            start = false;
+            if (F.setup(rs.x, Q, p, thr)) {
+                A = F.A0;
+                E1 = B = fx::nodeEnd<EXPR, false>(p, true);
+                G = 0;
+                GE = -200;
+                lo = pend = 0;
+                level = nInt = 0;
+                running = true;
+            } else {
+                defer();
+            }
+        }
+        // Intervals, until few lanes are still in their quadratures.
+        for (;;) {
+            if (running) {
+                const uint64_t mid = ((uint64_t)lo << 32) + (0x8000000000000000ull >> level);
+                const uint64_t dr = Q.fx.rho >> (level + 1);
+                const fx::Node V = fx::nodeAt<EXPR, false>(p, mid - dr), M = fx::nodeAt<EXPR, false>(p, mid),
+                               W = fx::nodeAt<EXPR, false>(p, mid + dr);
+                const fx::Interval q = fx::intervalSums<EXPR>(A, B, V, M, W, Q.fx, thr, level);
+                nodes += 3;
+                ++nInt;
+                if ((q.small || level == Q.maxSub - 1) && level >= Q.minSub) {
+                    fx::addValue<EXPR>(q.ih, q.E, level, G, GE);
+                    if (pend == 0) {
+                        running = false;
+                        done = true;
+                    } else {
+                        const int up = 31 - __clz((int)pend);
+                        pend ^= 1u << up;
+                        lo += 1u << (32 - level);
+                        level = up;
+                        A = B;
+                        B.g = stG[up];
+                        if constexpr (EXPR) B.E = stE[up];
+                    }
+                } else {
+                    ++level;
+                    pend |= 1u << level;
+                    stG[level] = B.g;
+                    if constexpr (EXPR) stE[level] = B.E;
+                    B = M;
+                }
+                if (running && (nInt >= prm.wideQuad || nodes > prm.nodeBudget)) defer();
+            }
+            if (__popc(__ballot_sync(kFull, running)) <= kStepLanes) break;
+        }
+        if (done) {
+            done = false;
+            const double T = __dmul_rn(rs.x, FP::value(G, GE));
+            rs.step_(T + f0, yd, KnownSlope{FP::value(E1.g, E1.E)}, prm.xtol, prm.ytol, kBracketIts, prm.method);
+            if (rs.phase == RootSolve::kDone) {
+                prm.out[(long long)comp * prm.outRs + i * prm.outCs] = rs.result;
+                if (prm.info) prm.info[(long long)comp * prm.infoStride + i] = rs.info;
+                if (rs.info < 0) stAll |= kStatusNoBracket;
+                have = false;
+                need = true;
+            } else {
+                start = true;
+            }
+        }
+    }
+    if (prm.statusWord && stAll) atomicOr(prm.statusWord, stAll);
+}
+
 // Inverse of the points the queue pass left over (deferList), one group of
 // G lanes per point (G = kWarpGroup; 32 / G points per warp), each solve
 // continuing from the state the queue pass saved for it (deferState).  The solver
@@ -2175,6 +2467,10 @@ __global__ void __launch_bounds__(128) inverseWarpKernel(const __grid_constant__
         }
         int dummy = 0;
         const InverseEval<BASIS, POS, PMAX> f{A, P, f0, &prm.quad, &prm.bc, nugget, &dummy};
+        constexpr bool kFixed = PMAX <= kFxMaxOrder;
+        FixedPoint<BASIS, POS, kFixed ? PMAX : 1> F;
+        bool fixedPt = false;
+        if constexpr (kFixed) fixedPt = Q.fx.ok && nugget == 0.0 && F.init(A.a, P, prm.bc);
         RootSolve rs;
         if (prm.deferState && k < prm.deferStateCap) rs.load(prm.deferState + (long long)k * RootSolve::kSaveDoubles);
         else rs.start(x0);
@@ -2184,6 +2480,88 @@ __global__ void __launch_bounds__(128) inverseWarpKernel(const __grid_constant__
             int qst = 0;
             double Ih = 0.0;  // (group lane 0)
             bool failed = false;
+            if constexpr (kFixed) {
+                fx::Poly<PMAX, decltype(F)::ENV> p;
+                fx::Threshold thr;
+                if (fixedPt && F.setup(xd, Q, p, thr)) {
+                    // The same rounds on integers (entries reuse the stack's space).
+                    constexpr bool EXPR = decltype(F)::EXPR;
+                    FxEntry* fst = reinterpret_cast<FxEntry*>(stk);
+                    const fx::Node NB = fx::nodeEnd<EXPR, false>(p, true);
+                    uint64_t Gs = 0;
+                    int GE = -200, sp = 1;
+                    if (gl == 0) fst[0] = FxEntry{F.A0.g, NB.g, 0, 0, 0, F.A0.E, NB.E};
+                    __syncwarp(gmask);
+                    long long processed = 0;
+                    while (sp > 0) {
+                        int m = min(G, sp);
+                        if (sp + m > cap - kMaxSubCap - 2) m = 1;
+                        const bool has = gl < m;
+                        FxEntry e{0, 0, 0, 0, 1, 0, 0};
+                        if (has) e = fst[sp - 1 - gl];
+                        __syncwarp(gmask);
+                        const bool pend = has && !e.done;
+                        bool accept = false;
+                        fx::Interval q{};
+                        fx::Node M{};
+                        if (pend) {
+                            const uint64_t mid = ((uint64_t)e.lo << 32) + (0x8000000000000000ull >> e.level);
+                            const uint64_t dr = Q.fx.rho >> (e.level + 1);
+                            fx::Node NA{}, NE{};
+                            NA.g = e.gA; NA.E = e.EA; NE.g = e.gB; NE.E = e.EB;
+                            const fx::Node V = fx::nodeAt<EXPR, false>(p, mid - dr);
+                            M = fx::nodeAt<EXPR, false>(p, mid);
+                            const fx::Node W = fx::nodeAt<EXPR, false>(p, mid + dr);
+                            q = fx::intervalSums<EXPR>(NA, NE, V, M, W, Q.fx, thr, e.level);
+                            accept = (q.small || e.level == Q.maxSub - 1) && e.level >= Q.minSub;
+                        }
+                        processed += __popc(__ballot_sync(gmask, pend) & gmask);
+                        if (processed > Q.maxIntervals) {
+                            qst |= kStatusBudget;
+                            failed = true;
+                            break;
+                        }
+                        const int nout = !has ? 0 : ((pend && !accept) ? 2 : 1);
+                        int incl = nout;  // sum over the group's lanes >= this one
+#pragma unroll
+                        for (int off = 1; off < G; off <<= 1) {
+                            const int v = __shfl_down_sync(gmask, incl, off, G);
+                            if (gl + off < G) incl += v;
+                        }
+                        const int total = __shfl_sync(gmask, incl, 0, G);
+                        const int base = sp - m + (incl - nout);
+                        if (has) {
+                            const int lv = e.level + 1;
+                            if (!pend) {
+                                fst[base] = e;
+                            } else if (accept) {
+                                fst[base] = FxEntry{q.ih, 0, e.lo, (short)e.level, 1, q.E, 0};
+                            } else {
+                                fst[base] = FxEntry{M.g, e.gB, e.lo + (0x80000000u >> e.level), (short)lv, 0, M.E, e.EB};
+                                fst[base + 1] = FxEntry{e.gA, M.g, e.lo, (short)lv, 0, e.EA, M.E};
+                            }
+                        }
+                        sp = sp - m + total;
+                        __syncwarp(gmask);
+                        if (gl == 0) {
+                            while (sp > 0) {
+                                const FxEntry t = fst[sp - 1];
+                                if (!t.done) break;
+                                fx::addValue<EXPR>(t.gA, t.EA, t.level, Gs, GE);
+                                --sp;
+                            }
+                        }
+                        sp = __shfl_sync(gmask, sp, 0, G);
+                        __syncwarp(gmask);
+                    }
+                    stAll |= qst;
+                    double T = __shfl_sync(gmask, __dmul_rn(xd, decltype(F)::value(Gs, GE)), 0, G);
+                    if (failed) T = nan;
+                    rs.step_(T + f0, yd, KnownSlope{decltype(F)::value(NB.g, NB.E)}, prm.xtol, prm.ytol, kBracketIts,
+                             prm.method);
+                    continue;
+                }
+            }
             if (fixed) {
                 // one fixed rule: the group's first lane alone
                 if (gl == 0) {
@@ -2432,6 +2810,9 @@ cudaError_t launchInverseP(const InverseParams& prm, int nBlocks, cudaStream_t s
             if (prm.tpb != 128 || !prm.queue || !prm.acoef) return cudaErrorInvalidValue;
             if (prm.nodeBudget > 0 && (!prm.deferList || !prm.deferCount)) return cudaErrorInvalidValue;
             kern = inverseQueueKernel<BASIS, POS, PMAX>;
+            if constexpr (PMAX <= kFxMaxOrder) {
+                if (prm.quad.fx.ok && prm.nugget == 0.0 && prm.nodeBudget > 0) kern = inverseFixedKernel<BASIS, POS, PMAX>;
+            }
             int perSM = 0, dev = 0, nSM = 0;
             cudaError_t e;
             if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, 128, 0)) != cudaSuccess) return e;

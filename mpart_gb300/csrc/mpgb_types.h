@@ -173,6 +173,16 @@ struct QEntry {
     int level, done;
 };
 
+// The same in fixed point (an accepted interval: its fine sum and exponent in
+// gA, EA); lo with 32 fraction bits.
+struct FxEntry {
+    uint64_t gA, gB;
+    uint32_t lo;
+    short level, done;
+    int EA, EB;
+};
+static_assert(sizeof(FxEntry) == sizeof(QEntry), "the two share the stack's space");
+
 struct InverseParams {
     const CompDesc* comps;
     int nComps;
