@@ -1500,6 +1500,14 @@ struct InverseEval {
     }
 };
 
+// The slope of T from the integrand's node at t = 1, formed when asked for.
+template <class F>
+struct NodeSlope {
+    uint64_t g;
+    int E;
+    __device__ double slope(double) const { return F::value(g, E); }
+};
+
 // The slope at the point just evaluated, read off its quadrature's t = 1 node.
 struct KnownSlope {
     double s;
@@ -1531,9 +1539,37 @@ struct SigmoidInverseEval {
     }
 };
 
-// 2^e for the integer-valued (or infinite / NaN) exponents of the ITP
-// truncation, exactly as pow(2.0, e) gives them.
-__device__ __forceinline__ double exp2Int(double e) {
+// Comparisons of doubles on their bits: a DSETP holds the FP64 pipe as long as
+// a DFMA, and a solver step compares as often as it multiplies.  (A NaN that
+// arithmetic makes has its sign bit clear: it is above every number.)
+__device__ __forceinline__ bool absLess(double x, double tol) {  // |x| < tol, tol >= 0
+    return (__double_as_longlong(x) & 0x7fffffffffffffffLL) < __double_as_longlong(tol);
+}
+__device__ __forceinline__ bool lessPos(double x, double tol) {  // x < tol, tol >= 0
+    return __double_as_longlong(x) < __double_as_longlong(tol);
+}
+__device__ __forceinline__ bool isPos(double x) {  // x > 0
+    const long long b = __double_as_longlong(x);
+    return b > 0 && b <= 0x7ff0000000000000LL;
+}
+__device__ __forceinline__ double minAbs(double x, double y) {  // fmin(x, |y|)
+    const long long a = __double_as_longlong(x), b = __double_as_longlong(y) & 0x7fffffffffffffffLL;
+    return __longlong_as_double(a < b ? a : b);
+}
+
+// 2^(nhalf + 1 - it) for the integer-valued (or infinite / NaN) nhalf of the
+// ITP truncation, exactly as pow(2.0, e) gives it.
+__device__ __forceinline__ double itpPow(double nhalf, unsigned it) {
+    const long long b = __double_as_longlong(nhalf);
+    const int ex = (int)((b >> 52) & 0x7ff) - 1023;
+    if (ex < 10) {
+        // |nhalf| < 1024: its integer from the bits.
+        const long long m = (b & 0x000fffffffffffffLL) | 0x0010000000000000LL;
+        const int v = ex < 0 ? 0 : (int)(m >> (52 - ex));
+        const int e = (b < 0 ? -v : v) + 1 - (int)it;
+        if (e > -1022 && e < 1024) return __longlong_as_double((long long)(e + 1023) << 52);
+    }
+    const double e = __dsub_rn(__dadd_rn(nhalf, 1.0), (double)it);
     if (isnan(e)) return e;
     if (e > 4096.0) return __longlong_as_double(0x7ff0000000000000ULL);
     if (e < -4096.0) return 0.0;
@@ -1544,18 +1580,18 @@ __device__ __forceinline__ double exp2Int(double e) {
 // constants of InverseSingleBracket (k1 = 0.1, k2 = 2, n0 = 1, :145-149), in
 // the reference's operation order and without FMA contraction, so that the
 // iterates are those of the reference's host build.  pow(w, 2) is w * w
-// (libm's pow returns the correctly rounded square).
-__device__ __forceinline__ double itpPoint(double xlb, double xub, double ylb, double yub, double nhalf, unsigned it,
-                                           double xtol) {
+// (libm's pow returns the correctly rounded square); a product by the sign
+// sigma is a sign change.  w = xub - xlb.
+__device__ __forceinline__ double itpPoint(double xlb, double xub, double ylb, double yub, double w, double nhalf,
+                                           unsigned it, double xtol) {
     const double xb = __dmul_rn(0.5, __dadd_rn(xub, xlb));
     double xf = __ddiv_rn(__dsub_rn(__dmul_rn(xub, ylb), __dmul_rn(xlb, yub)), __dsub_rn(ylb, yub));
-    const double sigma = (__dsub_rn(xb, xf) > 0) ? 1.0 : -1.0;
-    const double w = __dsub_rn(xub, xlb);
-    const double delta = fmin(__dmul_rn(0.1, __dmul_rn(w, w)), fabs(__dsub_rn(xb, xf)));
-    xf = __dadd_rn(xf, __dmul_rn(delta, sigma));
-    const double p2 = exp2Int(__dsub_rn(__dadd_rn(nhalf, 1.0), (double)it));
-    const double rho = fmin(__dsub_rn(__dmul_rn(xtol, p2), __dmul_rn(0.5, w)), fabs(__dsub_rn(xf, xb)));
-    return __dsub_rn(xb, __dmul_rn(sigma, rho));
+    const double gap = __dsub_rn(xb, xf);
+    const long long sign = isPos(gap) ? 0LL : (long long)0x8000000000000000ULL;
+    const double delta = minAbs(__dmul_rn(0.1, __dmul_rn(w, w)), gap);
+    xf = __dadd_rn(xf, __longlong_as_double(__double_as_longlong(delta) ^ sign));
+    const double rho = minAbs(__dsub_rn(__dmul_rn(xtol, itpPow(nhalf, it)), __dmul_rn(0.5, w)), __dsub_rn(xf, xb));
+    return __dsub_rn(xb, __longlong_as_double(__double_as_longlong(rho) ^ sign));
 }
 
 // Root of f(x) = yd for a monotone f (MonotoneComponent::InverseImpl with
@@ -1612,7 +1648,7 @@ struct RootSolve {
         if ((ylb > yd) || (yub < yd)) { finish(__longlong_as_double(0x7ff8000000000000ULL), -2); return; }
         nhalf = ceil(log2(__ddiv_rn(__dmul_rn(0.5, __dsub_rn(xub, xlb)), xtol)));
         it = 0;
-        x = itpPoint(xlb, xub, ylb, yub, nhalf, it, xtol);
+        x = itpPoint(xlb, xub, ylb, yub, __dsub_rn(xub, xlb), nhalf, it, xtol);
         phase = kITP;
     }
     // The bracket is found: the checks before the solver loop and its first point.
@@ -1637,13 +1673,14 @@ struct RootSolve {
         const double nan = __longlong_as_double(0x7ff8000000000000ULL);
         if (phase == kITP) {
             // One iteration of InverseSingleBracket's loop (RootFinding.h:152-170).
-            const double xc = x;
-            if (fabs(y - yd) < ftol) { finish(xc, 0); return; }
-            if (y > yd) { xub = xc; yub = y; }
+            const double xc = x, d = __dsub_rn(y, yd);
+            if (absLess(d, ftol)) { finish(xc, 0); return; }
+            if (isPos(d)) { xub = xc; yub = y; }
             else { xlb = xc; ylb = y; }
-            if (((xub - xlb) < xtol) || ((yub - ylb) < ftol)) { finish(0.5 * (xub + xlb), 0); return; }
+            const double w = __dsub_rn(xub, xlb);
+            if (lessPos(w, xtol) || lessPos(__dsub_rn(yub, ylb), ftol)) { finish(0.5 * (xub + xlb), 0); return; }
             if (++it >= 10000u) { finish(0.5 * (xub + xlb), 0); return; }
-            x = itpPoint(xlb, xub, ylb, yub, nhalf, it, xtol);
+            x = itpPoint(xlb, xub, ylb, yub, w, nhalf, it, xtol);
             return;
         }
         if (phase == kStart) {
@@ -1788,7 +1825,18 @@ struct FixedPoint {
             p.Z = bad ? 0 : (uint64_t)(z * 0x1p57);
         }
         bad |= sum > (31u << 23);
-        const double ta = Q.absTol / fabs(x);
+        // absTol / |x|: the accept test's threshold, to 2^-44 (the test's own
+        // integers carry fewer bits) by one Newton step from the 2^-23
+        // reciprocal; a true division is three times as long on the FP64 pipe.
+        double ta;
+        {
+            const double ax = fabs(x);
+            double r;
+            asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(ax));
+            const double e = fma(-ax, r, 1.0);
+            ta = Q.absTol * fma(r, e, r);
+            if (!(ax > 1e-200)) ta = __longlong_as_double(0x7ff0000000000000ULL);
+        }
         if constexpr (EXPR) {
             const uint64_t t = (uint64_t)__double_as_longlong(ta);
             thr.m = ((t & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
@@ -2217,19 +2265,21 @@ __global__ void __launch_bounds__(128) inverseQueueKernel(const __grid_constant_
     if (prm.statusWord && stAll) atomicOr(prm.statusWord, stAll);
 }
 
-// Lanes of a warp that may still be in their quadratures when the others take
-// a solver step.  A step is some 60 FP64 instructions, as long on the SM as
-// three intervals of a whole warp, so it waits for most lanes; waiting for all
-// leaves lanes idle behind the widest quadrature.
-constexpr int kStepLanes = 8;
-
 // Inverse of one monotone component (compBegin) from the queue of points, in
 // fixed point: the solver of inverseQueueKernel (one point per lane, expensive
 // ones first), its quadratures traversed interval by interval on integers
 // (fx::integrate's arithmetic).  A point or an iterate out of the fixed-point
 // range, a quadrature of wideQuad intervals and a solve of nodeBudget nodes go,
 // with the solver's state, to the warp pass.
-template <int BASIS, int POS, int PMAX>
+//
+// A solver step is some 60 FP64 instructions, as long on the SM as three
+// intervals of a whole warp, so it waits until at most a quarter of the warp's
+// solves are still in their quadratures (waiting for all leaves lanes idle
+// behind the widest; spreading few points over more, part-filled warps repeats
+// the FP64 steps: 40k targets 18.6 -> 23.0 ms).  LANES = 4 gives a point four lanes, which evaluate an interval's
+// three nodes side by side: for launches too small to fill the device, where a
+// solve's own chain of intervals is the time.
+template <int BASIS, int POS, int PMAX, int LANES>
 __global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_constant__ InverseParams prm) {
     using FP = FixedPoint<BASIS, POS, PMAX>;
     constexpr bool EXPR = FP::EXPR, ENV = FP::ENV;
@@ -2238,7 +2288,8 @@ __global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_consta
     const CompDesc& c = prm.comps[comp];
     const int D = c.D, P = c.P;
     const long long N = prm.N;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, q4 = lane % LANES;
+    const unsigned gmask = LANES == 1 ? 0xffffffffu : ((1u << LANES) - 1u) << (lane - q4);
     const unsigned kFull = 0xffffffffu;
     const double nan = __longlong_as_double(0x7ff8000000000000ULL);
 
@@ -2257,23 +2308,25 @@ __global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_consta
     uint64_t stG[32];
     int stE[EXPR ? 32 : 1];
     auto defer = [&]() {
-        const int slot = atomicAdd(prm.deferCount, 1);
-        prm.deferList[slot] = (int)i;
-        if (prm.deferState && slot < prm.deferStateCap)
-            rs.save(prm.deferState + (long long)slot * RootSolve::kSaveDoubles);
+        if (q4 == 0) {
+            const int slot = atomicAdd(prm.deferCount, 1);
+            prm.deferList[slot] = (int)i;
+            if (prm.deferState && slot < prm.deferStateCap)
+                rs.save(prm.deferState + (long long)slot * RootSolve::kSaveDoubles);
+        }
         have = running = done = start = false;
         need = true;
     };
 
     for (;;) {
-        const unsigned needMask = __ballot_sync(kFull, need);
+        const unsigned needMask = __ballot_sync(kFull, need && q4 == 0);
         if (needMask) {
             const int leader = __ffs(needMask) - 1;
             int base = 0;
             if (lane == leader) base = atomicAdd(prm.queue, __popc(needMask));
             base = __shfl_sync(kFull, base, leader);
             if (need) {
-                const long long slot = (long long)base + __popc(needMask & ((1u << lane) - 1u));
+                const long long slot = (long long)base + __popc(needMask & ((1u << (lane - q4)) - 1u));
                 need = false;
                 if (slot < N) {
                     i = prm.perm ? (long long)prm.perm[N - 1 - slot] : slot;
@@ -2291,8 +2344,10 @@ __global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_consta
                     }
                     if (hasNan) {
                         // (MonotoneComponent.h:407-413)
-                        prm.out[(long long)comp * prm.outRs + i * prm.outCs] = nan;
-                        if (prm.info) prm.info[(long long)comp * prm.infoStride + i] = 0;
+                        if (q4 == 0) {
+                            prm.out[(long long)comp * prm.outRs + i * prm.outCs] = nan;
+                            if (prm.info) prm.info[(long long)comp * prm.infoStride + i] = 0;
+                        }
                         need = true;
                     } else {
                         yd = prm.r[(long long)comp * prm.rRs + i * prm.rCs];
@@ -2331,8 +2386,23 @@ __global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_consta
             if (running) {
                 const uint64_t mid = ((uint64_t)lo << 32) + (0x8000000000000000ull >> level);
                 const uint64_t dr = Q.fx.rho >> (level + 1);
-                const fx::Node V = fx::nodeAt<EXPR, false>(p, mid - dr), M = fx::nodeAt<EXPR, false>(p, mid),
-                               W = fx::nodeAt<EXPR, false>(p, mid + dr);
+                fx::Node V, M, W;
+                if constexpr (LANES == 1) {
+                    V = fx::nodeAt<EXPR, false>(p, mid - dr);
+                    M = fx::nodeAt<EXPR, false>(p, mid);
+                    W = fx::nodeAt<EXPR, false>(p, mid + dr);
+                } else {
+                    const fx::Node o = fx::nodeAt<EXPR, false>(p, q4 == 0 ? mid - dr : (q4 == 1 ? mid : mid + dr));
+                    V.g = __shfl_sync(gmask, o.g, 0, LANES);
+                    M.g = __shfl_sync(gmask, o.g, 1, LANES);
+                    W.g = __shfl_sync(gmask, o.g, 2, LANES);
+                    V.E = M.E = W.E = 0;
+                    if constexpr (EXPR) {
+                        V.E = __shfl_sync(gmask, o.E, 0, LANES);
+                        M.E = __shfl_sync(gmask, o.E, 1, LANES);
+                        W.E = __shfl_sync(gmask, o.E, 2, LANES);
+                    }
+                }
                 const fx::Interval q = fx::intervalSums<EXPR>(A, B, V, M, W, Q.fx, thr, level);
                 nodes += 3;
                 ++nInt;
@@ -2359,15 +2429,17 @@ __global__ void __launch_bounds__(128, 4) inverseFixedKernel(const __grid_consta
                 }
                 if (running && (nInt >= prm.wideQuad || nodes > prm.nodeBudget)) defer();
             }
-            if (__popc(__ballot_sync(kFull, running)) <= kStepLanes) break;
+            if (4 * __popc(__ballot_sync(kFull, running)) <= __popc(__ballot_sync(kFull, have))) break;
         }
         if (done) {
             done = false;
             const double T = __dmul_rn(rs.x, FP::value(G, GE));
-            rs.step_(T + f0, yd, KnownSlope{FP::value(E1.g, E1.E)}, prm.xtol, prm.ytol, kBracketIts, prm.method);
+            rs.step_(T + f0, yd, NodeSlope<FP>{E1.g, E1.E}, prm.xtol, prm.ytol, kBracketIts, prm.method);
             if (rs.phase == RootSolve::kDone) {
-                prm.out[(long long)comp * prm.outRs + i * prm.outCs] = rs.result;
-                if (prm.info) prm.info[(long long)comp * prm.infoStride + i] = rs.info;
+                if (q4 == 0) {
+                    prm.out[(long long)comp * prm.outRs + i * prm.outCs] = rs.result;
+                    if (prm.info) prm.info[(long long)comp * prm.infoStride + i] = rs.info;
+                }
                 if (rs.info < 0) stAll |= kStatusNoBracket;
                 have = false;
                 need = true;
@@ -2557,8 +2629,7 @@ __global__ void __launch_bounds__(128) inverseWarpKernel(const __grid_constant__
                     stAll |= qst;
                     double T = __shfl_sync(gmask, __dmul_rn(xd, decltype(F)::value(Gs, GE)), 0, G);
                     if (failed) T = nan;
-                    rs.step_(T + f0, yd, KnownSlope{decltype(F)::value(NB.g, NB.E)}, prm.xtol, prm.ytol, kBracketIts,
-                             prm.method);
+                    rs.step_(T + f0, yd, NodeSlope<decltype(F)>{NB.g, NB.E}, prm.xtol, prm.ytol, kBracketIts, prm.method);
                     continue;
                 }
             }
@@ -2810,14 +2881,26 @@ cudaError_t launchInverseP(const InverseParams& prm, int nBlocks, cudaStream_t s
             if (prm.tpb != 128 || !prm.queue || !prm.acoef) return cudaErrorInvalidValue;
             if (prm.nodeBudget > 0 && (!prm.deferList || !prm.deferCount)) return cudaErrorInvalidValue;
             kern = inverseQueueKernel<BASIS, POS, PMAX>;
-            if constexpr (PMAX <= kFxMaxOrder) {
-                if (prm.quad.fx.ok && prm.nugget == 0.0 && prm.nodeBudget > 0) kern = inverseFixedKernel<BASIS, POS, PMAX>;
-            }
             int perSM = 0, dev = 0, nSM = 0;
             cudaError_t e;
-            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, 128, 0)) != cudaSuccess) return e;
             if ((e = cudaGetDevice(&dev)) != cudaSuccess) return e;
             if ((e = cudaDeviceGetAttribute(&nSM, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+            if constexpr (PMAX <= kFxMaxOrder) {
+                if (prm.quad.fx.ok && prm.nugget == 0.0 && prm.nodeBudget > 0) {
+                    // Four lanes a point while that leaves the points side by
+                    // side on the device (4 blocks an SM); see the kernel.
+                    const bool four = prm.N * 4 <= (long long)nSM * 4 * 128;
+                    kern = four ? inverseFixedKernel<BASIS, POS, PMAX, 4> : inverseFixedKernel<BASIS, POS, PMAX, 1>;
+                    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, 128, 0)) != cudaSuccess) return e;
+                    const long long perWarp = four ? 8 : 32;
+                    const long long blocks = (prm.N + 4 * perWarp - 1) / (4 * perWarp);
+                    kern<<<(int)std::min(blocks, (long long)std::max(1, perSM) * nSM), 128, 0, stream>>>(prm);
+                    e = cudaGetLastError();
+                    countLaunches(stream, 1);
+                    return e;
+                }
+            }
+            if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&perSM, kern, 128, 0)) != cudaSuccess) return e;
             const long long need = (prm.N + 127) / 128;
             const int grid = (int)std::max(1LL, std::min(need, (long long)std::max(1, perSM) * nSM));
             kern<<<grid, 128, 0, stream>>>(prm);
