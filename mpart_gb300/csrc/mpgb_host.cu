@@ -312,8 +312,34 @@ struct KLPlan {
     long long rcTotal = 0;  // rectifier cache of sigmoid expansions (doubles)
 };
 
+// Work items and reduction tables of a launch: they depend on the map and the
+// number of points alone, so a call with a size seen before uploads nothing.
+enum class PlanStyle { AllComps, PerComp, Reduced };
+struct LaunchPlan {
+    long long N = -1;
+    PlanStyle style = PlanStyle::AllComps;
+    int onlyComp = -1;
+    bool uploaded = false;  // false after a build inside a stream capture (the copies have not run)
+    bool captured = false;  // a captured graph may read it: kept as long as the map
+    long long used = 0;     // call counter of the last use
+    std::vector<WorkItem> items;
+    std::vector<long long> rows;       // partial rows, by component
+    std::vector<KLReduceDesc> reduce;  // per component
+    int maxTerms = 0;
+    size_t partialDoubles = 1;
+    long long rcTotal = 0;
+    DevBuf dItems, dRows, dReduce;
+};
+constexpr size_t kMaxPlans = 48;
+
 struct MapWorkspace {
-    DevBuf comps, cm, cmFx, cmScale, gather, items, partials, rowBase, lossPart, lossSlots, logdetRows, status, reduceDesc;
+    std::vector<std::unique_ptr<LaunchPlan>> plans;
+    long long planClock = 0;
+    int* hostStatus = nullptr;  // pinned: a pageable copy is staged by the driver
+    ~MapWorkspace() {
+        if (hostStatus) cudaFreeHost(hostStatus);
+    }
+    DevBuf comps, cm, cmFx, cmScale, gather, partials, lossPart, logdetRows, status;
     DevBuf stage[8];
     std::vector<CompDesc> hostComps;
     std::vector<GatherDescHost> hostGather;
@@ -700,10 +726,11 @@ double* MonotoneMapBase::StagingBuffer(int slot, size_t bytes, cudaStream_t stre
 int MonotoneMapBase::CheckStatus(cudaStream_t stream) {
     MapWorkspace& W = *ws_;
     if (!W.status.p) return 0;
-    int st = 0;
-    MPGB_CUDA(cudaMemcpyAsync(&st, W.status.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    if (!W.hostStatus) MPGB_CUDA(cudaMallocHost(&W.hostStatus, sizeof(int)));
+    MPGB_CUDA(cudaMemcpyAsync(W.hostStatus, W.status.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     MPGB_CUDA(cudaStreamSynchronize(stream));
-    MPGB_CUDA(cudaMemsetAsync(W.status.p, 0, sizeof(int), stream));
+    const int st = *W.hostStatus;
+    if (st) MPGB_CUDA(cudaMemsetAsync(W.status.p, 0, sizeof(int), stream));
     return st;
 }
 
@@ -838,10 +865,81 @@ static double* rectCache(MapWorkspace& W, long long rcTotal, cudaStream_t stream
     return W.rcache.as<double>();
 }
 
-static void uploadItems(MapWorkspace& W, const std::vector<WorkItem>& items, cudaStream_t stream) {
-    W.items.ensure(items.size() * sizeof(WorkItem), stream);
-    MPGB_CUDA(cudaMemcpyAsync(W.items.p, items.data(), items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice,
-                              stream));
+// The plan for (N, style, onlyComp), built on first use.  At most kMaxPlans are
+// kept; the least recently used makes room (after a device synchronisation:
+// launches in flight may still read it).
+static LaunchPlan& launchPlan(MapWorkspace& W, const std::vector<MonotoneMapBase::Part>& parts, long long N,
+                              PlanStyle style, int onlyComp, cudaStream_t stream) {
+    LaunchPlan* P = nullptr;
+    for (auto& p : W.plans)
+        if (p->N == N && p->style == style && p->onlyComp == onlyComp) P = p.get();
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    MPGB_CUDA(cudaStreamIsCapturing(stream, &cs));
+    const bool capturing = cs != cudaStreamCaptureStatusNone;
+    if (P) P->captured = P->captured || capturing;
+    if (P && P->uploaded) {
+        P->used = ++W.planClock;
+        return *P;
+    }
+    if (!P) {
+        if (W.plans.size() >= kMaxPlans && !capturing) {
+            auto old = std::min_element(W.plans.begin(), W.plans.end(), [](auto const& x, auto const& y) {
+                return x->captured != y->captured ? y->captured : x->used < y->used;
+            });
+            if (!(*old)->captured) {
+                MPGB_CUDA(cudaDeviceSynchronize());
+                W.plans.erase(old);
+            }
+        }
+        auto fresh = std::make_unique<LaunchPlan>();
+        LaunchPlan& q = *fresh;
+        q.N = N;
+        q.style = style;
+        q.onlyComp = onlyComp;
+        q.captured = capturing;
+        if (style == PlanStyle::AllComps) {
+            q.items = itemsAllComps(N, (int)parts.size());
+        } else {
+            std::vector<std::vector<int>> itemsOf;
+            const bool reduced = style == PlanStyle::Reduced;
+            q.items = itemsPerComp(parts, N, W.numSMs, reduced, nullptr, &itemsOf, onlyComp, &q.rcTotal);
+            for (int c = 0; reduced && c < (int)parts.size(); ++c) {
+                const ComponentProgram& g = *parts[c].prog;
+                KLReduceDesc d{};
+                d.rowOff = (int)q.rows.size();
+                for (int id : itemsOf[c])
+                    for (int sg = 0; sg < g.cSegs; ++sg)
+                        q.rows.push_back(q.items[id].partialBase + (long long)sg * g.numTerms);
+                d.nRows = (int)q.rows.size() - d.rowOff;
+                d.nTerms = g.numTerms;
+                d.outOff = (int)parts[c].mapCoeffOffset;
+                d.comp = c;
+                q.reduce.push_back(d);
+                q.maxTerms = std::max(q.maxTerms, d.nTerms);
+            }
+            if (reduced)
+                for (auto& it : q.items)
+                    q.partialDoubles = std::max<size_t>(
+                        q.partialDoubles, (size_t)it.partialBase +
+                                              (size_t)parts[it.c0].prog->numTerms * parts[it.c0].prog->cSegs);
+        }
+        W.plans.push_back(std::move(fresh));
+        P = W.plans.back().get();
+    }
+    P->used = ++W.planClock;
+    auto put = [&](DevBuf& d, const void* h, size_t bytes) {
+        d.ensure(std::max<size_t>(bytes, 8), stream);
+        if (bytes) MPGB_CUDA(cudaMemcpyAsync(d.p, h, bytes, cudaMemcpyHostToDevice, stream));
+    };
+    put(P->dItems, P->items.data(), P->items.size() * sizeof(WorkItem));
+    put(P->dRows, P->rows.data(), P->rows.size() * sizeof(long long));
+    put(P->dReduce, P->reduce.data(), P->reduce.size() * sizeof(KLReduceDesc));
+    if (!capturing) {
+        // (the next call may use the plan on another stream)
+        MPGB_CUDA(cudaStreamSynchronize(stream));
+        P->uploaded = true;
+    }
+    return *P;
 }
 
 // Sorts every component's points (or onlyComp's) by |x_D| of its own last
@@ -899,9 +997,10 @@ static int stageDoubles(const MapWorkspace& W, const FusedParams& p, bool input)
     return base + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
 }
 
-static void launch(MapWorkspace& W, const MapOptions& o, FusedParams& p, int nItems, int needJ, int needE,
+static void launch(MapWorkspace& W, const MapOptions& o, FusedParams& p, const LaunchPlan& plan, int needJ, int needE,
                    cudaStream_t stream) {
-    p.items = W.items.as<WorkItem>();
+    const int nItems = (int)plan.items.size();
+    p.items = plan.dItems.as<WorkItem>();
     if (nItems == 0) return;
     const size_t smem = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, (p.flags & kFlagInput) != 0);
     if (smem > 227 * 1024) throw std::invalid_argument("Component too large for the shared-memory tile.");
@@ -942,8 +1041,7 @@ void MonotoneMapBase::EvaluateImpl(StridedMatrix const& pts, StridedMatrix const
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    auto items = itemsPerComp(parts_, N, W.numSMs, false, nullptr, nullptr);
-    uploadItems(W, items, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, -1, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     // The reference's EvaluateImpl calls EvaluateSingle without the nugget
@@ -954,7 +1052,7 @@ void MonotoneMapBase::EvaluateImpl(StridedMatrix const& pts, StridedMatrix const
     p.pts = pts.data; p.ptsRs = pts.rowStride; p.ptsCs = pts.colStride;
     p.outEval = output.data; p.evalRs = output.rowStride; p.evalCs = output.colStride;
     orderPoints(W, parts_, pts, p, -1, stream);
-    launch(W, opts_, p, (int)items.size(), 0, 0, stream);
+    launch(W, opts_, p, plan, 0, 0, stream);
     Finish(stream, "Evaluate");
 }
 
@@ -967,15 +1065,14 @@ void MonotoneMapBase::LogDeterminantImpl(StridedMatrix const& pts, StridedMatrix
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    auto items = itemsAllComps(N, (int)parts_.size());
-    uploadItems(W, items, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::AllComps, -1, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagLogDet;
     p.pts = pts.data; p.ptsRs = pts.rowStride; p.ptsCs = pts.colStride;
     p.outLogDet = output.data;
     p.logDetStride = (output.rows == 1) ? output.colStride : output.rowStride;
-    launch(W, opts_, p, (int)items.size(), 0, 0, stream);
+    launch(W, opts_, p, plan, 0, 0, stream);
     Finish(stream, "LogDeterminant");
 }
 
@@ -990,8 +1087,7 @@ void MonotoneMapBase::CoeffGradImpl(StridedMatrix const& pts, StridedMatrix cons
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    auto items = itemsPerComp(parts_, N, W.numSMs, false, nullptr, nullptr);
-    uploadItems(W, items, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, -1, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagCoefDenseT;
@@ -999,7 +1095,7 @@ void MonotoneMapBase::CoeffGradImpl(StridedMatrix const& pts, StridedMatrix cons
     p.sens = sens.data; p.sensRs = sens.rowStride; p.sensCs = sens.colStride;
     p.outDense = output.data; p.denseRs = output.rowStride; p.denseCs = output.colStride;
     orderPoints(W, parts_, pts, p, -1, stream);
-    launch(W, opts_, p, (int)items.size(), 1, 0, stream);
+    launch(W, opts_, p, plan, 1, 0, stream);
     Finish(stream, "CoeffGrad");
 }
 
@@ -1013,14 +1109,13 @@ void MonotoneMapBase::LogDeterminantCoeffGradImpl(StridedMatrix const& pts, Stri
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    auto items = itemsPerComp(parts_, N, W.numSMs, false, nullptr, nullptr);
-    uploadItems(W, items, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, -1, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagCoefDenseL;
     p.pts = pts.data; p.ptsRs = pts.rowStride; p.ptsCs = pts.colStride;
     p.outDense = output.data; p.denseRs = output.rowStride; p.denseCs = output.colStride;
-    launch(W, opts_, p, (int)items.size(), 0, 0, stream);
+    launch(W, opts_, p, plan, 0, 0, stream);
     Finish(stream, "LogDeterminantCoeffGrad");
 }
 
@@ -1035,8 +1130,7 @@ void MonotoneMapBase::GradientImpl(StridedMatrix const& pts, StridedMatrix const
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    auto items = itemsAllComps(N, (int)parts_.size());
-    uploadItems(W, items, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::AllComps, -1, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagInput;
@@ -1044,7 +1138,7 @@ void MonotoneMapBase::GradientImpl(StridedMatrix const& pts, StridedMatrix const
     p.sens = sens.data; p.sensRs = sens.rowStride; p.sensCs = sens.colStride;
     p.lsens = nullptr; p.lsensScale = 0.0;
     p.outInput = output.data; p.inputRs = output.rowStride; p.inputCs = output.colStride;
-    launch(W, opts_, p, (int)items.size(), 1, 1, stream);
+    launch(W, opts_, p, plan, 1, 1, stream);
     Finish(stream, "Gradient");
 }
 
@@ -1059,8 +1153,7 @@ void MonotoneMapBase::LogDeterminantInputGradImpl(StridedMatrix const& pts, Stri
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    auto items = itemsAllComps(N, (int)parts_.size());
-    uploadItems(W, items, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::AllComps, -1, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagInput;
@@ -1068,7 +1161,7 @@ void MonotoneMapBase::LogDeterminantInputGradImpl(StridedMatrix const& pts, Stri
     p.sens = nullptr;
     p.lsens = nullptr; p.lsensScale = 1.0;
     p.outInput = output.data; p.inputRs = output.rowStride; p.inputCs = output.colStride;
-    launch(W, opts_, p, (int)items.size(), 0, 0, stream);
+    launch(W, opts_, p, plan, 0, 0, stream);
     Finish(stream, "LogDeterminantInputGrad");
 }
 
@@ -1258,16 +1351,13 @@ void MonotoneMapBase::FusedForwardAdjoint(StridedMatrix const& pts, StridedMatri
     const bool wantCoef = coeffGrad != nullptr;
     const bool wantLogDet = !outLogDet.empty();
     if (wantCoef || !outEval.empty() || wantLogDet) {
-        std::vector<long long> rowBase;
-        std::vector<std::vector<int>> itemsOf;
-        long long rcTotal = 0;
-        auto items = itemsPerComp(parts_, N, W.numSMs, wantCoef, &rowBase, &itemsOf, -1, &rcTotal);
-        uploadItems(W, items, stream);
+        LaunchPlan& plan =
+            launchPlan(W, parts_, N, wantCoef ? PlanStyle::Reduced : PlanStyle::PerComp, -1, stream);
         FusedParams p{};
         baseParams(W, opts_, p, N);
         p.pts = pts.data; p.ptsRs = pts.rowStride; p.ptsCs = pts.colStride;
         p.flags = 0;
-        if (wantCoef) p.rcache = rectCache(W, rcTotal, stream);
+        if (wantCoef) p.rcache = rectCache(W, plan.rcTotal, stream);
         orderPoints(W, parts_, pts, p, -1, stream);
         if (!outEval.empty()) {
             p.flags |= kFlagEval;
@@ -1286,13 +1376,7 @@ void MonotoneMapBase::FusedForwardAdjoint(StridedMatrix const& pts, StridedMatri
             p.flags |= kFlagCoefReduced;
             p.sens = sens.data; p.sensRs = sens.rowStride; p.sensCs = sens.colStride;
             p.lsens = logdetSens.data; p.lsensStride = ldStrideL; p.lsensScale = logdetSensScale;
-            size_t nPart = rowBase.empty() ? 1 : (size_t)(rowBase.back() + parts_[items.back().c0].prog->numTerms);
-            size_t tot = 0;
-            for (auto& it : items)
-                tot = std::max<size_t>(tot, (size_t)it.partialBase +
-                                                (size_t)parts_[it.c0].prog->numTerms * parts_[it.c0].prog->cSegs);
-            nPart = std::max(nPart, tot);
-            W.partials.ensure(nPart * sizeof(double), stream);
+            W.partials.ensure(plan.partialDoubles * sizeof(double), stream);
             p.partials = W.partials.as<double>();
             needJ = sens.empty() ? 0 : 1;
         }
@@ -1300,54 +1384,27 @@ void MonotoneMapBase::FusedForwardAdjoint(StridedMatrix const& pts, StridedMatri
             // One component per item: each writes its component's row of the
             // scratch, summed in component order below.
             p.logDetCompStride = N;
-            launch(W, opts_, p, (int)items.size(), needJ, 0, stream);
+            launch(W, opts_, p, plan, needJ, 0, stream);
             sumRowsKernel<<<(unsigned)((N + 255) / 256), 256, 0, stream>>>(
                 W.logdetRows.as<double>(), nComps, N, outLogDet.data,
                 (outLogDet.rows == 1) ? outLogDet.colStride : outLogDet.rowStride);
             MPGB_CUDA(cudaGetLastError());
             countLaunches(stream, 1);
         } else {
-            launch(W, opts_, p, (int)items.size(), needJ, 0, stream);
+            launch(W, opts_, p, plan, needJ, 0, stream);
         }
         if (wantCoef) {
-            // Fixed-order reduction of each component's partial rows.
-            std::vector<long long> rb;
-            W.rowBase.ensure(sizeof(long long) * std::max<size_t>(1, rowBase.size()), stream);
-            for (int c = 0; c < nComps; ++c) {
-                for (int id : itemsOf[c])
-                    for (int sg = 0; sg < parts_[c].prog->cSegs; ++sg)
-                        rb.push_back(items[id].partialBase + (long long)sg * parts_[c].prog->numTerms);
-            }
-            MPGB_CUDA(cudaMemcpyAsync(W.rowBase.p, rb.data(), rb.size() * sizeof(long long), cudaMemcpyHostToDevice,
-                                      stream));
-            // Every component's rows in one launch.
-            std::vector<KLReduceDesc> rd(nComps);
-            int off = 0, maxTerms = 0;
-            for (int c = 0; c < nComps; ++c) {
-                KLReduceDesc& q = rd[c];
-                q = KLReduceDesc{};
-                q.rowOff = off;
-                q.nRows = (int)itemsOf[c].size() * parts_[c].prog->cSegs;
-                q.nTerms = parts_[c].prog->numTerms;
-                q.outOff = (int)parts_[c].mapCoeffOffset;
-                q.comp = c;
-                off += q.nRows;
-                maxTerms = std::max(maxTerms, q.nTerms);
-            }
-            W.reduceDesc.ensure(rd.size() * sizeof(KLReduceDesc), stream);
-            MPGB_CUDA(cudaMemcpyAsync(W.reduceDesc.p, rd.data(), rd.size() * sizeof(KLReduceDesc),
-                                      cudaMemcpyHostToDevice, stream));
-            MPGB_CUDA(launchKLReduce(W.partials.as<double>(), W.rowBase.as<long long>(),
-                                     W.reduceDesc.as<KLReduceDesc>(), nComps, maxTerms, coeffGrad, nullptr, nullptr,
-                                     1.0, nullptr, stream));
+            // Fixed-order reduction of every component's partial rows.
+            MPGB_CUDA(launchKLReduce(W.partials.as<double>(), plan.dRows.as<long long>(),
+                                     plan.dReduce.as<KLReduceDesc>(), nComps, plan.maxTerms, coeffGrad, nullptr,
+                                     nullptr, 1.0, nullptr, stream));
         }
     }
     // Pass 2: input gradient (sums over components per point).
     if (!inputGrad.empty()) {
         if (!opts_.contDeriv && (logdetSens.data || logdetSensScale != 0.0))
             throw std::invalid_argument("Discrete derivative version is not implemented yet (To Do)");
-        auto items = itemsAllComps(N, nComps);
-        uploadItems(W, items, stream);
+        LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::AllComps, -1, stream);
         FusedParams p{};
         baseParams(W, opts_, p, N);
         p.flags = kFlagInput;
@@ -1356,7 +1413,7 @@ void MonotoneMapBase::FusedForwardAdjoint(StridedMatrix const& pts, StridedMatri
         p.lsens = logdetSens.data; p.lsensStride = ldStrideL; p.lsensScale = logdetSensScale;
         p.outInput = inputGrad.data; p.inputRs = inputGrad.rowStride; p.inputCs = inputGrad.colStride;
         const int nj = sens.empty() ? 0 : 1;
-        launch(W, opts_, p, (int)items.size(), nj, nj, stream);
+        launch(W, opts_, p, plan, nj, nj, stream);
     }
     Finish(stream, "FusedForwardAdjoint");
 }
@@ -1583,14 +1640,11 @@ void MonotoneMapBase::InverseCoeffGrad(StridedMatrix const& pts, StridedMatrix c
     const bool wantCoef = coeffGrad != nullptr;
     for (size_t q = 0; q < order.size(); ++q) {
         const int c = order[q];
-        std::vector<long long> rowBase;
-        std::vector<std::vector<int>> itemsOf;
-        long long rcTotal = 0;
-        auto items = itemsPerComp(parts_, N, W.numSMs, wantCoef, &rowBase, &itemsOf, c, &rcTotal);
-        uploadItems(W, items, stream);
+        LaunchPlan& plan =
+            launchPlan(W, parts_, N, wantCoef ? PlanStyle::Reduced : PlanStyle::PerComp, c, stream);
         FusedParams p{};
         baseParams(W, opts_, p, N);
-        if (wantCoef) p.rcache = rectCache(W, rcTotal, stream);
+        if (wantCoef) p.rcache = rectCache(W, plan.rcTotal, stream);
         p.flags = kFlagInput | kFlagImplicit | (q == 0 ? kFlagImplicitFirst : 0) | (wantCoef ? kFlagCoefReduced : 0);
         p.pts = pts.data; p.ptsRs = pts.rowStride; p.ptsCs = pts.colStride;
         p.sens = w.data; p.sensRs = w.rowStride; p.sensCs = w.colStride;
@@ -1598,20 +1652,13 @@ void MonotoneMapBase::InverseCoeffGrad(StridedMatrix const& pts, StridedMatrix c
         p.outInput = G.data; p.inputRs = G.rowStride; p.inputCs = G.colStride;
         p.negRows = (q + 1 == order.size()) ? extra : 0;
         if (wantCoef) {
-            size_t nPart = 1;
-            for (auto& it : items)
-                nPart = std::max<size_t>(nPart, (size_t)it.partialBase +
-                                                    (size_t)parts_[c].prog->numTerms * parts_[c].prog->cSegs);
-            W.partials.ensure(nPart * sizeof(double), stream);
+            W.partials.ensure(plan.partialDoubles * sizeof(double), stream);
             p.partials = W.partials.as<double>();
         }
         orderPoints(W, parts_, pts, p, c, stream);
-        launch(W, opts_, p, (int)items.size(), 1, 0, stream);
+        launch(W, opts_, p, plan, 1, 0, stream);
         if (wantCoef) {
-            W.rowBase.ensure(sizeof(long long) * std::max<size_t>(1, rowBase.size()), stream);
-            MPGB_CUDA(cudaMemcpyAsync(W.rowBase.p, rowBase.data(), rowBase.size() * sizeof(long long),
-                                      cudaMemcpyHostToDevice, stream));
-            MPGB_CUDA(launchReduceRows(W.partials.as<double>(), W.rowBase.as<long long>(), (int)rowBase.size(),
+            MPGB_CUDA(launchReduceRows(W.partials.as<double>(), plan.dRows.as<long long>(), (int)plan.rows.size(),
                                        parts_[c].prog->numTerms, -1.0, coeffGrad + parts_[c].mapCoeffOffset, 0,
                                        stream));
         }
