@@ -985,13 +985,18 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
             if ((flags & kFlagCoefReduced) && tj == 0)
                 for (long long k = tid; k < (long long)c.cSegs * c.numTerms; k += tpb)
                     prm.partials[item.partialBase + k] = 0.0;
-            // Fixed-point phase A (and reduction): launches that need neither
-            // per-term outputs nor input gradients, which read the FP64 table.
+            // Fixed-point phase A (and reduction).  Per-term outputs and input
+            // gradients walk the tree again with the FP64 table: alone they
+            // keep it from the start (filling it twice costs more than phase A
+            // gains: 4-D order-4 dense gradients 198 -> 214 us), with a reduced
+            // adjoint beside them (the implicit gradient) they do not.
             constexpr bool kLimbs = limbBasis<BASIS, PMAX>();
             bool limbs = false, outlier = false;
             int phiScale = 0, cScale = 0;
             if constexpr (kLimbs) {
-                if (prm.cmFx && prm.stageDoubles >= kStageMin && !(flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput))) {
+                if (prm.cmFx && prm.stageDoubles >= kStageMin &&
+                    (!(flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) ||
+                     ((flags & kFlagCoefReduced) && prm.rcache))) {
                     cScale = __ldg(&prm.cmScale[ci]);
                     limbs = cScale != kNoLimbs;
                 }
@@ -1021,6 +1026,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                     phaseALimbs<PMAX>(c, L, tid, prm.cmFx + c.slotOffset, prm.stageDoubles, outlier, phiScale, cScale, a,
                                       rc);
                     if (outlier) phaseA<PMAX>(c, L, tid, cm, a, nullptr);
+                    else if (flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) fillLead<BASIS>(c, L, tid, prm.bc);
                 }
             } else if constexpr (BASIS == kBasisSigmoid) {
                 phaseARect<PMAX, POS>(c, L, tid, cm, a, rc);
@@ -1251,7 +1257,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                         w[k] = wT[k] + wL[k];
                         skip |= fx::expBound(w[k]) > 1024;
                     }
-                    if (skip && !outlier) fillLead<BASIS>(c, L, tid, prm.bc);
+                    if (skip && !outlier && !(flags & kFlagInput)) fillLead<BASIS>(c, L, tid, prm.bc);
                     if (tid <= PMAX) sMax[tid] = -4096;
                     __syncthreads();
 #pragma unroll
