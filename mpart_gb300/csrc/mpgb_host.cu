@@ -286,6 +286,7 @@ struct GatherDescHost {
 struct KLPlan {
     long long N = -1;
     int onlyComp = -2;
+    int tpb = 128;
     int nItems = 0;
     std::vector<std::vector<int>> itemsOf;
     std::vector<int> rowOff;   // first row of each component in rowBase
@@ -319,6 +320,7 @@ struct LaunchPlan {
     long long N = -1;
     PlanStyle style = PlanStyle::AllComps;
     int onlyComp = -1;
+    int tpb = 128;
     bool uploaded = false;  // false after a build inside a stream capture (the copies have not run)
     bool captured = false;  // a captured graph may read it: kept as long as the map
     long long used = 0;     // call counter of the last use
@@ -800,9 +802,21 @@ static void baseParams(MapWorkspace& W, const MapOptions& o, FusedParams& p, lon
 
 static int posCode(const MapOptions& o) { return o.posFuncType == PosFuncTypes::Exp ? kPosExp : kPosSoftPlus; }
 
+// Points per block.  A launch with too few 128-point tiles for the SMs takes
+// smaller ones: the FP64 part of a tile holds its SM's one FP64 pipe, so 4,096
+// points finish sooner as 128 one-warp blocks than as 32 blocks of four warps.
+// Reduced launches keep at least 64 (their sums share a node's row among lanes).
+// The rule goes by the number of points alone, so that batched and
+// per-component launches cut the same tiles.
+static int tileSize(long long N, int numSMs, bool reduced) {
+    const long long sms = std::max(1, numSMs);
+    if (!reduced && N <= 32 * sms * 2) return 32;
+    return N <= 64 * sms ? 64 : kTpb;
+}
+
 // Items of style "all components per tile" (per-point sums across components).
-static std::vector<WorkItem> itemsAllComps(long long N, int nComps) {
-    long long nTiles = (N + kTpb - 1) / kTpb;
+static std::vector<WorkItem> itemsAllComps(long long N, int nComps, int tpb) {
+    long long nTiles = (N + tpb - 1) / tpb;
     std::vector<WorkItem> v;
     v.reserve(nTiles);
     for (long long t = 0; t < nTiles; ++t) v.push_back({0, nComps, (int)t, 1, 0, 0, 1});
@@ -817,11 +831,11 @@ static std::vector<WorkItem> itemsAllComps(long long N, int nComps) {
 // in order of |x_D| (quadrature cost grows with it), and striding gives every
 // item the same mix of cheap and expensive tiles.
 static std::vector<WorkItem> itemsPerComp(const std::vector<MonotoneMapBase::Part>& parts, long long N, int numSMs,
-                                          bool reduced, std::vector<long long>* rowBaseOut,
+                                          bool reduced, int tpb, std::vector<long long>* rowBaseOut,
                                           std::vector<std::vector<int>>* itemsOfComp, int onlyComp = -1,
                                           long long* rcTotal = nullptr) {
     const int nComps = (int)parts.size();
-    const long long nTiles = (N + kTpb - 1) / kTpb;
+    const long long nTiles = (N + tpb - 1) / tpb;
     std::vector<int> order;
     for (int c = 0; c < nComps; ++c)
         if (onlyComp < 0 || c == onlyComp) order.push_back(c);
@@ -841,7 +855,7 @@ static std::vector<WorkItem> itemsPerComp(const std::vector<MonotoneMapBase::Par
                 w.lossSlot = (int)v.size();
                 if (rcTotal) {
                     w.rcBase = *rcTotal;
-                    *rcTotal += (long long)parts[c].prog->nCNodes * kTpb;
+                    *rcTotal += (long long)parts[c].prog->nCNodes * tpb;
                 }
                 for (int sg = 0; sg < parts[c].prog->cSegs; ++sg) {
                     if (rowBaseOut) rowBaseOut->push_back(base);
@@ -897,12 +911,13 @@ static LaunchPlan& launchPlan(MapWorkspace& W, const std::vector<MonotoneMapBase
         q.style = style;
         q.onlyComp = onlyComp;
         q.captured = capturing;
+        q.tpb = tileSize(N, W.numSMs, style == PlanStyle::Reduced);
         if (style == PlanStyle::AllComps) {
-            q.items = itemsAllComps(N, (int)parts.size());
+            q.items = itemsAllComps(N, (int)parts.size(), q.tpb);
         } else {
             std::vector<std::vector<int>> itemsOf;
             const bool reduced = style == PlanStyle::Reduced;
-            q.items = itemsPerComp(parts, N, W.numSMs, reduced, nullptr, &itemsOf, onlyComp, &q.rcTotal);
+            q.items = itemsPerComp(parts, N, W.numSMs, reduced, q.tpb, nullptr, &itemsOf, onlyComp, &q.rcTotal);
             for (int c = 0; reduced && c < (int)parts.size(); ++c) {
                 const ComponentProgram& g = *parts[c].prog;
                 KLReduceDesc d{};
@@ -1000,6 +1015,7 @@ static int stageDoubles(const MapWorkspace& W, const FusedParams& p, bool input)
 static void launch(MapWorkspace& W, const MapOptions& o, FusedParams& p, const LaunchPlan& plan, int needJ, int needE,
                    cudaStream_t stream) {
     const int nItems = (int)plan.items.size();
+    p.tpb = plan.tpb;
     p.items = plan.dItems.as<WorkItem>();
     if (nItems == 0) return;
     const size_t smem = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, (p.flags & kFlagInput) != 0);
@@ -1429,7 +1445,8 @@ static KLPlan& klPlan(MapWorkspace& W, const std::vector<MonotoneMapBase::Part>&
     P.N = N;
     P.onlyComp = onlyComp;
     std::vector<long long> rowBase;
-    auto items = itemsPerComp(parts, N, W.numSMs, true, &rowBase, &P.itemsOf, onlyComp, &P.rcTotal);
+    P.tpb = tileSize(N, W.numSMs, true);
+    auto items = itemsPerComp(parts, N, W.numSMs, true, P.tpb, &rowBase, &P.itemsOf, onlyComp, &P.rcTotal);
     P.nItems = (int)items.size();
     for (auto& it : items)
         P.partialDoubles = std::max<size_t>(P.partialDoubles, (size_t)it.partialBase + (size_t)parts[it.c0].prog->numTerms *
@@ -1551,6 +1568,7 @@ void MonotoneMapBase::KLObjective(StridedMatrix const& pts, double* lossPerComp,
     p.partials = W.partials.as<double>();
     p.lossPartials = W.lossPart.as<double>();
     p.items = P.items.as<WorkItem>();
+    p.tpb = P.tpb;
     p.rcache = rectCache(W, P.rcTotal, stream);
     orderPointsKL(W, P, parts_, pts, p, onlyComp, stream);
     const bool costOrder = p.perm != nullptr;
@@ -1640,8 +1658,9 @@ void MonotoneMapBase::InverseCoeffGrad(StridedMatrix const& pts, StridedMatrix c
     const bool wantCoef = coeffGrad != nullptr;
     for (size_t q = 0; q < order.size(); ++q) {
         const int c = order[q];
-        LaunchPlan& plan =
-            launchPlan(W, parts_, N, wantCoef ? PlanStyle::Reduced : PlanStyle::PerComp, c, stream);
+        // (the same tiles with and without the coefficient gradient: the same
+        // input gradient to the bit)
+        LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::Reduced, c, stream);
         FusedParams p{};
         baseParams(W, opts_, p, N);
         if (wantCoef) p.rcache = rectCache(W, plan.rcTotal, stream);

@@ -988,15 +988,15 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
             // Fixed-point phase A (and reduction).  Per-term outputs and input
             // gradients walk the tree again with the FP64 table: alone they
             // keep it from the start (filling it twice costs more than phase A
-            // gains: 4-D order-4 dense gradients 198 -> 214 us), with a reduced
-            // adjoint beside them (the implicit gradient) they do not.
+            // gains: 4-D order-4 dense gradients 198 -> 214 us); the implicit
+            // gradient, with its reduced adjoint, does not (and takes the same
+            // a_k when no coefficient gradient is asked for).
             constexpr bool kLimbs = limbBasis<BASIS, PMAX>();
             bool limbs = false, outlier = false;
             int phiScale = 0, cScale = 0;
             if constexpr (kLimbs) {
                 if (prm.cmFx && prm.stageDoubles >= kStageMin &&
-                    (!(flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) ||
-                     ((flags & kFlagCoefReduced) && prm.rcache))) {
+                    (!(flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) || (flags & kFlagImplicit))) {
                     cScale = __ldg(&prm.cmScale[ci]);
                     limbs = cScale != kNoLimbs;
                 }
