@@ -59,16 +59,17 @@ MPGB_HD uint64_t madWide(uint32_t a, uint32_t b, uint64_t c) { return (uint64_t)
 MPGB_HD int64_t madWideS(int32_t a, int32_t b, int64_t c) { return (int64_t)a * b + c; }
 #endif
 
-// floor(a b / 2^64) less at most 1 (the product of the low words is left
-// out), for a + b <= 2^64.
+// a b / 2^64 rounded, for a + b <= 2^64; the product of the low words is left
+// out and its mean added with the rounding (zero stays zero).
 MPGB_HD uint64_t mulhi(uint64_t a, uint64_t b) {
-    const uint64_t mid = madWide(hi32(a), lo32(b), mulWide(lo32(a), hi32(b)));
+    const uint64_t mid = madWide(hi32(a), lo32(b), madWide(lo32(a), hi32(b), 0xC0000000ull));
     return madWide(hi32(a), hi32(b), hi32(mid));
 }
 
-// The same for any a, b (less at most 2).
+// The same for any a, b: two middle products, each with its rounding and half
+// the mean of the low one.
 MPGB_HD uint64_t mulhiAny(uint64_t a, uint64_t b) {
-    const uint64_t m1 = mulWide(lo32(a), hi32(b)), m2 = mulWide(hi32(a), lo32(b));
+    const uint64_t m1 = madWide(lo32(a), hi32(b), 0xA0000000ull), m2 = madWide(hi32(a), lo32(b), 0xA0000000ull);
     return madWide(hi32(a), hi32(b), hi32(m1)) + hi32(m2);
 }
 
@@ -84,6 +85,10 @@ MPGB_HD uint64_t mul32Round(uint64_t a, uint32_t b) {
 MPGB_HD uint32_t hi(uint32_t a, uint32_t b) { return hi32(madWide(a, b, 0x80000000ull)); }
 
 MPGB_HD uint64_t shr(uint64_t x, int n) { return n < 64 ? x >> n : 0; }
+// x / 2^n rounded to nearest (n < 0: x 2^-n).
+MPGB_HD uint64_t scaleRound(uint64_t x, int n) {
+    return n < 0 ? x << -n : (n < 64 ? (x + ((1ull << n) >> 1)) >> n : 0);
+}
 // x / 2^n rounded to nearest, n >= 0.
 MPGB_HD uint64_t shrRound(uint64_t x, int n) { return n < 64 ? (x + ((1ull << n) >> 1)) >> n : 0; }
 
@@ -121,7 +126,7 @@ MPGB_HD uint64_t exp2neg(uint64_t W, int& n) {
 // exp(-u), u with 58 fraction bits, u < 32: 63 fraction bits, below 1.
 MPGB_HD uint64_t expNeg(uint64_t u) {
     int n;
-    const uint64_t m = exp2neg(mulhiAny(u, kLog2e63) + 1, n);  // (+ 1: the mean of what mulhiAny drops)
+    const uint64_t m = exp2neg(mulhiAny(u, kLog2e63), n);
     return m >> n;
 }
 
@@ -178,7 +183,7 @@ MPGB_HD uint64_t expMant(uint64_t D, int& E) {
     // 64 - d log2(e) = (64 + 32 log2(e)) - (d + 32) log2(e), 57 fraction bits
     constexpr uint64_t kBias = (64ull << 57) + (kLog2e63 >> 1);
     int n;
-    const uint64_t m = exp2neg(kBias - mulhiAny(D, kLog2e63) - 1, n);
+    const uint64_t m = exp2neg(kBias - mulhiAny(D, kLog2e63), n);
     E = 64 - n;
     return m >> 1;
 }
@@ -195,7 +200,7 @@ MPGB_HD int64_t toFixed58(double x, bool& bad) {
     if (e > 1027) bad = true;
     const uint64_t m = ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
     const int sh = 1027 - e;  // (subnormal x: shifted out)
-    const int64_t v = (sh >= 0 && sh < 64) ? (int64_t)(m >> sh) : 0;
+    const int64_t v = sh <= 0 ? (int64_t)m : (sh < 64 ? (int64_t)(((m >> (sh - 1)) + 1) >> 1) : 0);
     return (b >> 63) ? -v : v;
 }
 
@@ -263,13 +268,13 @@ struct Poly {
 };
 
 // sum_j c_j t^j, biased; t with 64 fraction bits.  acc' = acc + 2^63 steps as
-// c_j' + t acc' - t 2^63 (c_j' rounds the truncated product back up).
+// c_j' + t acc' - t 2^63.
 template <int NB, bool ENV>
 MPGB_HD uint64_t horner(const Poly<NB, ENV>& p, uint64_t t) {
     uint64_t acc = p.c[NB - 1];
     const uint64_t th = t >> 1;
 #pragma unroll
-    for (int j = NB - 2; j >= 0; --j) acc = (p.c[j] - th) + mulhiAny(acc, t) + 1;
+    for (int j = NB - 2; j >= 0; --j) acc = (p.c[j] - th) + mulhiAny(acc, t);
     return acc;
 }
 
@@ -340,13 +345,24 @@ MPGB_HD Node nodeEnd(const Poly<NB, ENV>& p, bool one) {
 
 // Integrals over [0, 1]: g (SoftPlus: 57 fraction bits; Exp: 62, times 2^E),
 // with NM > 0 m0 = int g' (ENV; 62 fraction bits) and m[j] = int g' t^j (times
-// the envelope with ENV); Exp: all times 2^E.
+// the envelope with ENV); Exp: all times 2^E.  ENV: the moments are those of
+// (2^ms t)^j, SoftPlus times 2^ms (see momentShift).
 template <int NM>
 struct Sums {
     uint64_t g, m0, m[NM > 0 ? NM : 1];
     int E, nInt;
     bool over;
 };
+
+// ms for an envelope exp(-(x t)^2 / 2): 2^ms about |x| / 2.  The moments feed
+// polynomials in y = x t whose coefficients grow as x^j, while the envelope
+// confines t to a few 1 / |x|: unscaled, their fixed fraction would lose
+// x^j of its size (1.7e-14 in an order-5 gradient at |x| = 10).  With
+// 2^ms <= |x| / 1.41 the weights (2^ms t)^j exp(-(x t)^2 / 2) stay below 2.5.
+MPGB_HD int momentShift(double x) {
+    const int e = expBound(x * 0.70710678118654752) - 1;  // floor(log2(|x| / 1.41))
+    return e < 0 ? 0 : (e > 3 ? 3 : e);
+}
 
 // absTol / |x_D| against sums of g scaled by 2^-level: SoftPlus as an integer
 // with 57 fraction bits, Exp as m 2^(E - 62).
@@ -386,8 +402,8 @@ MPGB_HD Interval intervalSums(const Node& A, const Node& B, const Node& V, const
         o.w = shr(o.w, E - W.E);
     }
     const uint64_t ab = o.a + o.b, vw = o.v + o.w;
-    const uint64_t ic = mulhi(ab, Q.c0) + mulhi(o.m, Q.cM) + 1;
-    o.ih = mulhi(ab, Q.w0) + mulhi(o.m, Q.wM) + mulhi(vw, Q.w1) + 2;
+    const uint64_t ic = mulhi(ab, Q.c0) + mulhi(o.m, Q.cM);
+    o.ih = mulhi(ab, Q.w0) + mulhi(o.m, Q.wM) + mulhi(vw, Q.w1);
     const uint64_t err = o.ih > ic ? o.ih - ic : ic - o.ih;
     uint64_t tol = mulhi(ic, Q.rel), ta;
     if constexpr (EXPR) {
@@ -432,7 +448,7 @@ MPGB_HD void addValue(uint64_t ih, int E, int level, uint64_t& g, int& gE) {
 // about its left end and shifted to t = 0 by repeated multiply-adds with lo.
 template <bool EXPR, int NB, bool ENV, int NM>
 MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int minSub, int maxIntervals,
-                       Threshold thr, Sums<NM>& R) {
+                       Threshold thr, int ms, Sums<NM>& R) {
     constexpr bool D = NM > 0;
     uint64_t stG[32], stF[D && !EXPR ? 32 : 1], stFe[D && ENV ? 32 : 1];
     int stE[EXPR ? 32 : 1];
@@ -478,7 +494,7 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
                         fv = shr(fv, E - V.E); fw = shr(fw, E - W.E);
                         R.m0 = R.g;
                     } else {
-                        R.m0 += shrRound(mulhi(A.f + B.f, Q.w0) + mulhi(M.f, Q.wM) + mulhi(V.f + W.f, Q.w1) + 2, level);
+                        R.m0 += shrRound(mulhi(A.f + B.f, Q.w0) + mulhi(M.f, Q.wM) + mulhi(V.f + W.f, Q.w1), level);
                     }
                 } else if constexpr (EXPR) {
                     fa = a; fb = b; fm = m; fv = v; fw = w;
@@ -488,15 +504,21 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
                 uint64_t mu[NM];
                 fb = mulhi(fb, Q.w0);
                 fm = mulhi(fm, Q.wM);
-                mu[0] = mulhi(fa, Q.w0) + fb + fm + mulhi(fv + fw, Q.w1) + 3;
+                mu[0] = mulhi(fa, Q.w0) + fb + fm + mulhi(fv + fw, Q.w1);
 #pragma unroll
-                for (int j = 1; j < NM; ++j) mu[j] = fb + (fm >> j) + mulhi(fv, Q.mLo[j]) + mulhi(fw, Q.mHi[j]) + 2;
+                for (int j = 1; j < NM; ++j) mu[j] = fb + ((fm + ((1ull << j) >> 1)) >> j) + mulhi(fv, Q.mLo[j]) + mulhi(fw, Q.mHi[j]);
 #pragma unroll
-                for (int j = 0; j < NM; ++j) mu[j] = shrRound(mu[j], level * j + dn);
+                for (int j = 0; j < NM; ++j) {
+                    if constexpr (ENV) mu[j] = scaleRound(mu[j], level * j + dn - ms * (EXPR ? j : j + 1));
+                    else mu[j] = shrRound(mu[j], level * j + dn);
+                }
 #pragma unroll
                 for (int i = 0; i + 1 < NM; ++i) {
 #pragma unroll
-                    for (int j = NM - 1; j > i; --j) mu[j] += mul32Round(mu[j - 1], lo);
+                    for (int j = NM - 1; j > i; --j) {
+                        if constexpr (ENV) mu[j] += mul32Round(mu[j - 1], lo) << ms;
+                        else mu[j] += mul32Round(mu[j - 1], lo);
+                    }
                 }
 #pragma unroll
                 for (int j = 0; j < NM; ++j) R.m[j] += mu[j];

@@ -425,7 +425,7 @@ __device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd
         p.a = (uint64_t)v + 0x8000000000000000ull;
         const double z = (xd * xd) * 0.72134752044448170368;  // x_D^2 / (2 ln 2)
         bad |= !(z < 126.0);
-        p.Z = bad ? 0 : (uint64_t)(z * 0x1p57);
+        p.Z = bad ? 0 : (uint64_t)(z * 0x1p57 + 0.5);
     }
     bad |= sum > (31u << 23);
     if constexpr (!EXPR) bad |= d0 < -(4ll << 58);
@@ -441,7 +441,8 @@ __device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd
         thr.E = 0;
     }
     fx::Sums<NM> S;
-    fx::integrate<EXPR, PMAX, ENV, NM>(p, Q.fx, Q.maxSub, Q.minSub, (int)Q.maxIntervals, thr, S);
+    const int ms = ENV && NEEDJ ? fx::momentShift(xd) : 0;
+    fx::integrate<EXPR, PMAX, ENV, NM>(p, Q.fx, Q.maxSub, Q.minSub, (int)Q.maxIntervals, thr, ms, S);
     R.nInt = S.nInt;
     if (S.over) {
         st |= kStatusBudget;
@@ -455,7 +456,13 @@ __device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd
     if constexpr (NEEDJ) {
         double m[NM];
 #pragma unroll
-        for (int j = 0; j < NM; ++j) m[j] = (double)S.m[j] * sc;
+        for (int j = 0; j < NM; ++j) {
+            double f = sc;
+            // (2^-ms per power: exact)
+            if constexpr (ENV)
+                f = __longlong_as_double(__double_as_longlong(sc) - ((long long)(ms * (EXPR ? j : j + 1)) << 52));
+            m[j] = (double)S.m[j] * f;
+        }
         if constexpr (NEEDE) {
             // d/dx_D of the integrand is g + t d/dt g(d_D f(t x_D))
             double e = G;
@@ -1828,7 +1835,7 @@ struct FixedPoint {
             p.a = (uint64_t)v + 0x8000000000000000ull;
             const double z = (x * x) * 0.72134752044448170368;
             bad |= !(z < 126.0);
-            p.Z = bad ? 0 : (uint64_t)(z * 0x1p57);
+            p.Z = bad ? 0 : (uint64_t)(z * 0x1p57 + 0.5);
         }
         bad |= sum > (31u << 23);
         // absTol / |x|: the accept test's threshold, to 2^-44 (the test's own
@@ -1871,7 +1878,7 @@ __device__ __noinline__ bool fixedValueNI(const FixedPoint<BASIS, POS, PMAX>* F,
     fx::Threshold thr;
     if (!F->setup(x, *Q, p, thr)) return false;
     fx::Sums<0> S;
-    fx::integrate<FP::EXPR, PMAX, FP::ENV, 0>(p, Q->fx, Q->maxSub, Q->minSub, (int)Q->maxIntervals, thr, S);
+    fx::integrate<FP::EXPR, PMAX, FP::ENV, 0>(p, Q->fx, Q->maxSub, Q->minSub, (int)Q->maxIntervals, thr, 0, S);
     if (S.over) {
         *st |= kStatusBudget;
         *I = __longlong_as_double(0x7ff8000000000000ULL);

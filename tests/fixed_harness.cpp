@@ -96,7 +96,9 @@ void one(const double* b, double a, double Z, double xd, double tol, bool simpso
         thr.E = (int)(u >> 52) - 1023;
     }
     fx::Sums<kNM> S;
-    fx::integrate<EXPR, kNB, ENV, kNM>(p, R, 30, minSub, 1 << 16, thr, S);
+    // (the envelope 2^(-Z t^2) is that of x = sqrt(2 Z ln 2))
+    const int ms = ENV ? fx::momentShift(std::sqrt(2.0 * Z * std::log(2.0))) : 0;
+    fx::integrate<EXPR, kNB, ENV, kNM>(p, R, 30, minSub, 1 << 16, thr, ms, S);
     long double G = 0, M0 = 0, M[kNM] = {};
     struct Iv { long double lo, hi; int level; };
     std::vector<Iv> st{{0, 1, 0}};
@@ -127,11 +129,14 @@ void one(const double* b, double a, double Z, double xd, double tol, bool simpso
             st.push_back({iv.lo, m, iv.level + 1});
         }
     }
-    const long double gs = EXPR ? std::ldexp(1.0L, S.E - 62) : 0x1p-57L, ms = EXPR ? gs : 0x1p-62L;
+    const long double gs = EXPR ? std::ldexp(1.0L, S.E - 62) : 0x1p-57L, ws = EXPR ? gs : 0x1p-62L;
     const long double unit = EXPR ? G : 1.0L;
     out[0] = (double)(std::fabs(S.g * gs - G) / unit);
-    out[1] = ENV ? (double)(std::fabs(S.m0 * ms - M0) / unit) : 0.0;
-    for (int j = 0; j < kNM; ++j) out[1] = std::fmax(out[1], (double)(std::fabs(S.m[j] * ms - M[j]) / unit));
+    out[1] = ENV ? (double)(std::fabs(S.m0 * ws - M0) / unit) : 0.0;
+    for (int j = 0; j < kNM; ++j) {
+        const long double f = std::ldexp(1.0L, ENV ? -ms * (EXPR ? j : j + 1) : 0);
+        out[1] = std::fmax(out[1], (double)(std::fabs(S.m[j] * ws * f - M[j]) / unit));
+    }
     out[2] = S.over ? -1 : S.nInt;
     out[3] = n;
 }
