@@ -264,8 +264,32 @@ template <int NB, bool ENV>
 struct Poly {
     uint64_t c[NB];  // 58 fraction bits; every entry biased
     uint64_t a;      // 58 fraction bits, biased
-    uint64_t Z;      // 57 fraction bits
+    uint64_t Z;      // 57 fraction bits, or 53 where it is 126 or more (wideZ)
+    bool wideZ;
 };
+
+// The envelope 2^(-Z t^2) (63 fraction bits) for t2 = t^2, t2 = 1 by its flag.
+template <int NB>
+MPGB_HD uint64_t envelope(const Poly<NB, true>& p, uint64_t t2, bool one) {
+    uint64_t W = one ? p.Z : mulhiAny(t2, p.Z);
+    if (p.wideZ) {
+        if (W >> 60) return 0;
+        W <<= 4;
+    }
+    int n;
+    const uint64_t m = exp2neg(W, n);
+    return shr(m, n);
+}
+
+// Z and its format for |x_D| < 53 (false beyond).
+template <int NB>
+MPGB_HD bool setEnvelope(Poly<NB, true>& p, double x) {
+    const double z = (x * x) * 0.72134752044448170368;  // x^2 / (2 ln 2)
+    p.wideZ = !(z < 126.0);
+    const bool ok = z < 2000.0;
+    p.Z = ok ? (uint64_t)(z * (p.wideZ ? 0x1p53 : 0x1p57) + 0.5) : 0;
+    return ok;
+}
 
 // sum_j c_j t^j, biased; t with 64 fraction bits.  acc' = acc + 2^63 steps as
 // c_j' + t acc' - t 2^63.
@@ -307,9 +331,7 @@ MPGB_HD Node nodeAt(const Poly<NB, ENV>& p, uint64_t t) {
     Node o;
     uint64_t gp;
     if constexpr (ENV) {
-        int n;
-        const uint64_t m = exp2neg(mulhiAny(mulhiAny(t, t), p.Z), n);
-        const uint64_t e = shr(m, n);  // the envelope, 63 fraction bits
+        const uint64_t e = envelope(p, mulhiAny(t, t), false);
         rect<EXPR, DERIV>(p.a + mulhiAny(horner(p, t), e << 1) - e, o, gp);
         if constexpr (DERIV) o.fe = mulhi(gp, e);
     } else {
@@ -329,12 +351,7 @@ MPGB_HD Node nodeEnd(const Poly<NB, ENV>& p, bool one) {
     Node o;
     uint64_t gp;
     if constexpr (ENV) {
-        int n = 0;
-        uint64_t e = 0x7fffffffffffffffull;
-        if (one) {
-            const uint64_t m = exp2neg(p.Z, n);
-            e = shr(m, n);
-        }
+        const uint64_t e = one ? envelope(p, 0, true) : 0x7fffffffffffffffull;
         rect<EXPR, DERIV>(p.a + mulhiAny(q, e << 1) - e, o, gp);
         if constexpr (DERIV) o.fe = mulhi(gp, e);
     } else {
@@ -361,7 +378,7 @@ struct Sums {
 // 2^ms <= |x| / 1.41 the weights (2^ms t)^j exp(-(x t)^2 / 2) stay below 2.5.
 MPGB_HD int momentShift(double x) {
     const int e = expBound(x * 0.70710678118654752) - 1;  // floor(log2(|x| / 1.41))
-    return e < 0 ? 0 : (e > 3 ? 3 : e);
+    return e < 0 ? 0 : (e > 5 ? 5 : e);
 }
 
 // absTol / |x_D| against sums of g scaled by 2^-level: SoftPlus as an integer

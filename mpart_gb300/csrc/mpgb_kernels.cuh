@@ -375,7 +375,7 @@ struct NodePoly {
 // traversal integrates g and, for adjoints, the moments of g' t^j, and J and
 // E follow from the moments.  False (nothing done) where its range does not
 // hold: a rule it is not built for, a nugget, coefficients with
-// sum |b_j| > 31 or not finite, an envelope exponent above 126, or SoftPlus
+// sum |b_j| > 31 or not finite, Hermite functions at |x_D| > 52, or SoftPlus
 // with d_D f(0) < -4 (g' would lose relative accuracy).  The bounds hold for
 // all but the far tails of ordinary maps (dim 8, order 4, N(0, 1) points:
 // every point up to |x_D| = 5).
@@ -418,14 +418,13 @@ __device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd
         p.c[j] = (uint64_t)v + 0x8000000000000000ull;
     }
     p.a = p.Z = 0;
+    p.wideZ = false;
     if constexpr (ENV) {
         const int64_t v = fx::toFixed58(as[1], bad);
         d0 += v;
         sum += (uint32_t)((v < 0 ? -v : v) >> 35) + 1;
         p.a = (uint64_t)v + 0x8000000000000000ull;
-        const double z = (xd * xd) * 0.72134752044448170368;  // x_D^2 / (2 ln 2)
-        bad |= !(z < 126.0);
-        p.Z = bad ? 0 : (uint64_t)(z * 0x1p57 + 0.5);
+        bad |= !fx::setEnvelope(p, xd);
     }
     bad |= sum > (31u << 23);
     if constexpr (!EXPR) bad |= d0 < -(4ll << 58);
@@ -1813,6 +1812,7 @@ struct FixedPoint {
         p.c[0] = (uint64_t)q + 0x8000000000000000ull;
         p.a = (uint64_t)q1 + 0x8000000000000000ull;
         p.Z = 0;
+        p.wideZ = false;
         A0 = fx::nodeEnd<EXPR, false>(p, false);
         return true;
     }
@@ -1829,13 +1829,12 @@ struct FixedPoint {
             p.c[j] = (uint64_t)v + 0x8000000000000000ull;
         }
         p.a = p.Z = 0;
+        p.wideZ = false;
         if constexpr (ENV) {
             const long long v = fx::toFixed58(a1, bad);
             sum += (uint32_t)((v < 0 ? -v : v) >> 35) + 1;
             p.a = (uint64_t)v + 0x8000000000000000ull;
-            const double z = (x * x) * 0.72134752044448170368;
-            bad |= !(z < 126.0);
-            p.Z = bad ? 0 : (uint64_t)(z * 0x1p57 + 0.5);
+            bad |= !fx::setEnvelope(p, x);
         }
         bad |= sum > (31u << 23);
         // absTol / |x|: the accept test's threshold, to 2^-44 (the test's own

@@ -86,7 +86,8 @@ void one(const double* b, double a, double Z, double xd, double tol, bool simpso
     bool bad = false;
     for (int j = 0; j < kNB; ++j) p.c[j] = (uint64_t)fx::toFixed58(b[j], bad) + (1ull << 63);
     p.a = (uint64_t)fx::toFixed58(a, bad) + (1ull << 63);
-    p.Z = (uint64_t)(Z * 0x1p57);
+    p.wideZ = Z >= 126;
+    p.Z = (uint64_t)(Z * (p.wideZ ? 0x1p53 : 0x1p57));
     const double th = tol / xd;
     fx::Threshold thr{(uint64_t)(th * 0x1p57), 0};
     if (EXPR) {
