@@ -804,7 +804,8 @@ static int posCode(const MapOptions& o) { return o.posFuncType == PosFuncTypes::
 
 // Points per block.  A launch with too few 128-point tiles for the SMs takes
 // smaller ones: the FP64 part of a tile holds its SM's one FP64 pipe, so 4,096
-// points finish sooner as 128 one-warp blocks than as 32 blocks of four warps.
+// points finish sooner as 128 one-warp blocks than as 32 blocks of four warps
+// (KL step on 5,003 samples 243 -> 207 us, torch step of 4,096 points 1031 -> 1006).
 // Reduced launches keep at least 64 (their sums share a node's row among lanes).
 // The rule goes by the number of points alone, so that batched and
 // per-component launches cut the same tiles.
