@@ -1407,7 +1407,8 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                 const int dneed2 = prm.comps[item.c1 - 1].D;
                 for (int d = 0; d < dneed2; ++d) {
                     const double v = L.GX[d * tpb + tid];
-                    prm.outInput[d * prm.inputRs + i * prm.inputCs] = (d < prm.negRows) ? -v : v;
+                    prm.outInput[item.c0 * prm.inputCompStride + d * prm.inputRs + i * prm.inputCs] =
+                        (d < prm.negRows) ? -v : v;
                 }
             }
             if (flags & kFlagStatusArray) prm.status[i * prm.statusStride] = st;

@@ -129,6 +129,7 @@ struct FusedParams {
     long long logDetCompStride;  // items of one component c0 write row c0 (0: one row for all)
     double* outDense; long long denseRs, denseCs;   // numCoeffs x N
     double* outInput; long long inputRs, inputCs;   // inputDim x N
+    long long inputCompStride;  // items of one component c0 write from outInput + c0 * this (0: one gradient for all)
     double* partials;
     double* lossPartials;
     int* status; long long statusStride;

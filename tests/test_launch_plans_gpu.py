@@ -68,3 +68,51 @@ def test_captured_call_survives_other_sizes(gpu, warm):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(y, ref)
+
+
+@pytest.mark.parametrize("dout", [1, 2, 3])
+def test_input_gradient_by_component_and_whole(gpu, dout):
+    """Few points are cut by component, many by tile alone: the same gradients,
+    to the few roundings of adding up the components in another place."""
+    import torch
+    M = gpu
+    r = np.random.default_rng(8 + dout)
+    tm = M.CreateTriangular(3, dout, 3, M.MapOptions(quadType=M.QuadTypes.AdaptiveClenshawCurtis))
+    tm.SetCoeffs(r.normal(0.0, 0.1, tm.numCoeffs))
+    big, n = 100_000, 300
+    x = torch.as_tensor(r.standard_normal((3, big)), device="cuda")
+    s = torch.as_tensor(r.standard_normal((dout, big)), device="cuda")
+    xs, ss = x[:, :n].contiguous(), s[:, :n].contiguous()
+    for few, many in ((tm.Gradient(xs, ss), tm.Gradient(x, s)), (tm.LogDeterminantInputGrad(xs), tm.LogDeterminantInputGrad(x))):
+        many = many[:, :n]
+        assert torch.all((few - many).abs() <= 1e-13 * torch.clamp(many.abs(), min=1e-2 * float(many.abs().max())))
+
+
+def test_captured_input_gradient_survives_larger_calls(gpu):
+    """An asynchronous input gradient owns no buffer that a later, larger call replaces."""
+    import torch
+    M = gpu
+    r = np.random.default_rng(13)
+    tm = M.CreateTriangular(3, 2, 2, M.MapOptions(quadType=M.QuadTypes.AdaptiveClenshawCurtis))
+    tm.SetCoeffs(r.normal(0.0, 0.1, tm.numCoeffs))
+    x = torch.as_tensor(r.standard_normal((3, 200)), device="cuda")
+    s = torch.as_tensor(r.standard_normal((2, 200)), device="cuda")
+    g = torch.zeros(3, 200, dtype=torch.float64, device="cuda")
+    tm.GradientImpl(x, s, g)
+    ref = g.clone()
+    tm.SetAsync(True)
+    graph, side = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        tm.GradientImpl(x, s, g)
+        torch.cuda.synchronize()
+        with torch.cuda.graph(graph, stream=side):
+            tm.GradientImpl(x, s, g)
+    torch.cuda.synchronize()
+    tm.SetAsync(False)
+    for n in (400, 9000):
+        tm.Gradient(torch.as_tensor(r.standard_normal((3, n)), device="cuda"),
+                    torch.as_tensor(r.standard_normal((2, n)), device="cuda"))
+    g.zero_()
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.all((g - ref).abs() <= 1e-13 * torch.clamp(ref.abs(), min=1e-2 * float(ref.abs().max())))
