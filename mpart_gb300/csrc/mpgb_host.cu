@@ -580,12 +580,17 @@ void buildLaunchConstants(const MapOptions& o, QuadParams& q, BasisConsts& b) {
         q.absTol > 0 && std::isfinite(q.absTol)) {
         auto frac = [](double w) { return (uint64_t)std::ldexp(w, 64); };
         q.fx.ok = 1;
-        q.fx.rho = frac(q.fPts[3]);
+        // The inner nodes mirror each other; in double their positions and
+        // weights differ in the last bits.  Taking one for both made every
+        // integral 8e-17 too large, which showed in sums over points (torch
+        // step of a 6-D order-2 map, Exp: gradient 9e-16 off, 3e-16 in FP64):
+        // the mean of the two keeps the rule's own total.
+        q.fx.rho = frac(q.fPts[3]) / 2 + frac(-q.fPts[1]) / 2;
         q.fx.c0 = frac(0.5 * q.cWts[0]);
         q.fx.cM = frac(0.5 * q.cWts[1]);
         q.fx.w0 = frac(0.5 * q.fWts[0]);
         q.fx.wM = frac(0.5 * q.fWts[2]);
-        q.fx.w1 = frac(0.5 * q.fWts[3]);
+        q.fx.w1 = frac(0.25 * q.fWts[1]) + frac(0.25 * q.fWts[3]);
         q.fx.rel = frac(q.relTol);
         // Powers of the positions in 64-bit integers: in double their rounding
         // would grow with j and bias the moments.

@@ -116,3 +116,22 @@ def test_captured_input_gradient_survives_larger_calls(gpu):
     graph.replay()
     torch.cuda.synchronize()
     assert torch.all((g - ref).abs() <= 1e-13 * torch.clamp(ref.abs(), min=1e-2 * float(ref.abs().max())))
+
+
+@pytest.mark.parametrize("pos", ["SoftPlus", "Exp"])
+def test_integrals_have_no_common_bias(gpu, pos):
+    """T = x_2 g(0.1 x_1): the relative errors of many points average to the
+    rule's own (weights that sum to 2 + 5.6e-17) and the arithmetic's few 2^-58."""
+    import torch
+    M = gpu
+    o = M.MapOptions(basisType=M.BasisTypes.HermiteFunctions if pos == "Exp" else M.BasisTypes.ProbabilistHermite,
+                     posFuncType=getattr(M.PosFuncTypes, pos), quadType=M.QuadTypes.AdaptiveClenshawCurtis,
+                     basisNorm=False)
+    comp = M.CreateComponent(M.FixedMultiIndexSet.from_multis([[1, 1]]), o)
+    comp.SetCoeffs(np.array([0.1]))
+    r = np.random.default_rng(21)
+    x = r.standard_normal((2, 200_000))
+    got = comp.Evaluate(torch.as_tensor(x, device="cuda")).cpu().numpy().reshape(-1).astype(np.longdouble)
+    f = np.longdouble(0.1) * x[0].astype(np.longdouble)
+    want = x[1].astype(np.longdouble) * (np.exp(f) if pos == "Exp" else np.log1p(np.exp(f)))
+    assert abs(float((got / want - 1).mean())) <= 4e-17
