@@ -233,6 +233,18 @@ MPGB_HD int expBound(double x) {
     return (int)((h >> 20) & 0x7ff) - 1022;
 }
 
+// The significand of a double with its top bit at 2^63: |x| = this times
+// 2^(expBound(x) - 64) (not for subnormals).
+MPGB_HD uint64_t mantissa64(double x) {
+#ifdef __CUDA_ARCH__
+    const uint64_t b = (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t b;
+    __builtin_memcpy(&b, &x, 8);
+#endif
+    return ((b & 0x000fffffffffffffull) | 0x0010000000000000ull) << 11;
+}
+
 // Products of leading-basis values in fixed point: phi = (h 2^27 + l) 2^-57,
 // 0 <= l < 2^27, |phi| <= 1, times a basis value (bh 2^31 + bl) 2^-58, |B| < 16.
 // The constant is the mean of what the shift and the left-out product of the
@@ -387,10 +399,30 @@ struct Threshold {
     uint64_t m;
     int E;
 };
+// The threshold of a quadrature.  False (the point keeps FP64) where neither
+// tolerance stands 2^6 units above the sums' last bit: the integers would cut
+// a smaller one to zero, or test rounding against it, and an accept test that
+// never holds runs to the interval budget (relTol 0, absTol 5e-18, x_D = 1:
+// 255 intervals in FP64).
+constexpr double kMinRelTol = 0x1p-44;
+template <bool EXPR>
+MPGB_HD bool threshold(double ta, double relTol, Threshold& thr) {
+    const int e = expBound(ta);
+    const uint64_t M = mantissa64(ta);
+    if constexpr (EXPR) {
+        thr.m = M >> 1;
+        thr.E = e - 1;
+    } else {
+        thr.m = e > 5 ? 1ull << 62 : shr(M, 7 - e);  // (x_D = 0: infinite)
+        thr.E = 0;
+    }
+    return relTol >= kMinRelTol || e > -50;  // (ta >= 2^-50)
+}
 
 // One interval of the rule from its five nodes (ends A, B, middle M, inner V,
 // W): the nodes' g on one exponent E (Exp), the fine sum ih (per unit width) and
-// whether |ih - ic| < max(relTol ic, (absTol / |x_D|) 2^level).
+// whether |ih - ic| < max(relTol ic, (absTol / |x_D|) 2^level).  (Exp's threshold is
+// rounded up: a difference of zero passes however large g is, as in FP64.)
 struct Interval {
     uint64_t a, b, m, v, w, ih;
     int E;
@@ -425,7 +457,7 @@ MPGB_HD Interval intervalSums(const Node& A, const Node& B, const Node& V, const
     uint64_t tol = mulhi(ic, Q.rel), ta;
     if constexpr (EXPR) {
         const int sh = o.E - thr.E - level;
-        ta = sh < 0 ? ~0ull : shr(thr.m, sh);
+        ta = sh < 0 ? ~0ull : shr(thr.m - 1, sh) + 1;
     } else {
         ta = (thr.m >> (63 - level)) ? ~0ull : thr.m << level;
     }

@@ -377,8 +377,9 @@ struct NodePoly {
 // traversal integrates g and, for adjoints, the moments of g' t^j, and J and
 // E follow from the moments.  False (nothing done) where its range does not
 // hold: a rule it is not built for, a nugget, coefficients with
-// sum |b_j| > 31 or not finite, Hermite functions at |x_D| > 52, or SoftPlus
-// with d_D f(0) < -4 (g' would lose relative accuracy).  The bounds hold for
+// sum |b_j| > 31 or not finite, Hermite functions at |x_D| > 52, SoftPlus
+// with d_D f(0) < -4 (g' would lose relative accuracy), or tolerances near the
+// sums' last bit (fx::threshold).  The bounds hold for
 // all but the far tails of ordinary maps (dim 8, order 4, N(0, 1) points:
 // every point up to |x_D| = 5).  Measured there at 1M points: the quadrature's
 // share of an evaluation 1.27 -> 0.33 ms, the fused adjoint 5.68 -> 4.17 ms
@@ -432,17 +433,9 @@ __device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd
     }
     bad |= sum > (31u << 23);
     if constexpr (!EXPR) bad |= d0 < -(4ll << 58);
-    if (bad) return false;
-    const double ta = Q.absTol / fabs(xd);
     fx::Threshold thr;
-    if constexpr (EXPR) {
-        const uint64_t t = (uint64_t)__double_as_longlong(ta);
-        thr.m = ((t & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
-        thr.E = (int)(t >> 52) - 1023;
-    } else {
-        thr.m = ta < 32.0 ? (uint64_t)(ta * 0x1p57) : 1ull << 62;
-        thr.E = 0;
-    }
+    bad |= !fx::threshold<EXPR>(Q.absTol / fabs(xd), Q.relTol, thr);
+    if (bad) return false;
     fx::Sums<NM> S;
     const int ms = ENV && NEEDJ ? fx::momentShift(xd) : 0;
     fx::integrate<EXPR, PMAX, ENV, NM>(p, Q.fx, Q.maxSub, Q.minSub, (int)Q.maxIntervals, thr, ms, S);
@@ -1857,14 +1850,7 @@ struct FixedPoint {
             ta = Q.absTol * fma(r, e, r);
             if (!(ax > 1e-200)) ta = __longlong_as_double(0x7ff0000000000000ULL);
         }
-        if constexpr (EXPR) {
-            const uint64_t t = (uint64_t)__double_as_longlong(ta);
-            thr.m = ((t & 0x000fffffffffffffull) | 0x0010000000000000ull) << 10;
-            thr.E = (int)(t >> 52) - 1023;
-        } else {
-            thr.m = ta < 32.0 ? (uint64_t)(ta * 0x1p57) : 1ull << 62;
-            thr.E = 0;
-        }
+        bad |= !fx::threshold<EXPR>(ta, Q.relTol, thr);
         return !bad;
     }
     // The value of an integral, and of a node (the slope of T at t = 1).
