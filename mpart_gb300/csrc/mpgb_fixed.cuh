@@ -73,12 +73,20 @@ MPGB_HD uint64_t mulhiAny(uint64_t a, uint64_t b) {
     return madWide(hi32(a), hi32(b), hi32(m1)) + hi32(m2);
 }
 
+// The same with the low words' product: rounded to nearest also where a or b
+// is small (mulhi and mulhiAny add the mean of a product that is not there).
+MPGB_HD uint64_t mulhiRound(uint64_t a, uint64_t b) {
+    const uint64_t m1 = madWide(lo32(a), hi32(b), hi32(mulWide(lo32(a), lo32(b))));
+    const uint64_t m2 = madWide(hi32(a), lo32(b), (uint64_t)lo32(m1) + 0x80000000ull);
+    return madWide(hi32(a), hi32(b), (uint64_t)hi32(m1) + hi32(m2));
+}
+
 // floor(a b / 2^32).
 MPGB_HD uint64_t mul32(uint64_t a, uint32_t b) { return madWide(hi32(a), b, hi32(mulWide(lo32(a), b))); }
 
-// a b / 2^32, rounded.
-MPGB_HD uint64_t mul32Round(uint64_t a, uint32_t b) {
-    return madWide(hi32(a), b, hi32(madWide(lo32(a), b, 0x80000000ull)));
+// a b / 2^32, rounded; ties up, or down with down = 1.
+MPGB_HD uint64_t mul32Round(uint64_t a, uint32_t b, uint32_t down = 0) {
+    return madWide(hi32(a), b, hi32(madWide(lo32(a), b, (uint64_t)(0x80000000u - down))));
 }
 
 // a b / 2^32 of two 32-bit numbers, rounded.
@@ -88,6 +96,10 @@ MPGB_HD uint64_t shr(uint64_t x, int n) { return n < 64 ? x >> n : 0; }
 // x / 2^n rounded to nearest (n < 0: x 2^-n).
 MPGB_HD uint64_t scaleRound(uint64_t x, int n) {
     return n < 0 ? x << -n : (n < 64 ? (x + ((1ull << n) >> 1)) >> n : 0);
+}
+// The same with ties to even.
+MPGB_HD uint64_t scaleEven(uint64_t x, int n) {
+    return n <= 0 ? x << -n : (n < 64 ? (x + ((1ull << (n - 1)) - 1) + ((x >> n) & 1)) >> n : 0);
 }
 // x / 2^n rounded to nearest, n >= 0.
 MPGB_HD uint64_t shrRound(uint64_t x, int n) { return n < 64 ? (x + ((1ull << n) >> 1)) >> n : 0; }
@@ -280,26 +292,35 @@ struct Poly {
     bool wideZ;
 };
 
-// The envelope 2^(-Z t^2) (63 fraction bits) for t2 = t^2, t2 = 1 by its flag.
+// The envelope 2^(-Z t^2) for t2 = t^2, t2 = 1 by its flag: m 2^-n, m with 63
+// fraction bits.
+struct Envelope {
+    uint64_t m;
+    int n;
+};
 template <int NB>
-MPGB_HD uint64_t envelope(const Poly<NB, true>& p, uint64_t t2, bool one) {
+MPGB_HD Envelope envelope(const Poly<NB, true>& p, uint64_t t2, bool one) {
+    Envelope e{0, 127};
     uint64_t W = one ? p.Z : mulhiAny(t2, p.Z);
     if (p.wideZ) {
-        if (W >> 60) return 0;
+        if (W >> 60) return e;
         W <<= 4;
     }
-    int n;
-    const uint64_t m = exp2neg(W, n);
-    return shr(m, n);
+    e.m = exp2neg(W, e.n);
+    return e;
 }
 
-// Z and its format for |x_D| < 53 (false beyond).
+// Z and its format for |x_D| < 52.6 (false beyond), from 64-bit products: in
+// FP64 the constant's own rounding would be common to all points.
 template <int NB>
 MPGB_HD bool setEnvelope(Poly<NB, true>& p, double x) {
-    const double z = (x * x) * 0.72134752044448170368;  // x^2 / (2 ln 2)
-    p.wideZ = !(z < 126.0);
-    const bool ok = z < 2000.0;
-    p.Z = ok ? (uint64_t)(z * (p.wideZ ? 0x1p53 : 0x1p57) + 0.5) : 0;
+    constexpr uint64_t kHalfLog2e = 0xb8aa3b295c17f0bcull;  // 1 / (2 ln 2), 64 fraction bits
+    const int e = expBound(x);
+    const uint64_t X = mantissa64(x);
+    const uint64_t z = mulhiAny(mulhiAny(X, X), kHalfLog2e);  // x^2 / (2 ln 2) = z 2^(2 e - 64)
+    const bool ok = e < 6 || (e == 6 && z < (2000ull << 52));
+    p.wideZ = e > 4 || (e == 4 && z >= (126ull << 56));
+    p.Z = ok ? scaleRound(z, (p.wideZ ? 11 : 7) - 2 * e) : 0;
     return ok;
 }
 
@@ -315,16 +336,18 @@ MPGB_HD uint64_t horner(const Poly<NB, ENV>& p, uint64_t t) {
 }
 
 // A node: g (SoftPlus: 57 fraction bits; Exp: mantissa with 62 and exponent
-// E), f = g' (62 fraction bits; Exp: g itself), fe = g' times the envelope.
+// E), f = g' (62 fraction bits; Exp: g itself), fe = g' times the envelope's
+// mantissa and n its exponent (fe 2^-n).
 struct Node {
     uint64_t g, f, fe;
-    int E;
+    int E, n;
 };
 
 template <bool EXPR, bool DERIV>
 MPGB_HD void rect(uint64_t D, Node& o, uint64_t& gp63) {
     o.E = 0;
     o.f = o.fe = 0;
+    o.n = 0;
     gp63 = 0;
     if constexpr (EXPR) {
         o.g = expMant(D, o.E);
@@ -343,9 +366,13 @@ MPGB_HD Node nodeAt(const Poly<NB, ENV>& p, uint64_t t) {
     Node o;
     uint64_t gp;
     if constexpr (ENV) {
-        const uint64_t e = envelope(p, mulhiAny(t, t), false);
+        const Envelope v = envelope(p, mulhiAny(t, t), false);
+        const uint64_t e = shrRound(v.m, v.n);
         rect<EXPR, DERIV>(p.a + mulhiAny(horner(p, t), e << 1) - e, o, gp);
-        if constexpr (DERIV) o.fe = mulhi(gp, e);
+        if constexpr (DERIV) {
+            o.fe = mulhiRound(gp, v.m);
+            o.n = v.n;
+        }
     } else {
         rect<EXPR, DERIV>(horner(p, t), o, gp);
     }
@@ -363,9 +390,13 @@ MPGB_HD Node nodeEnd(const Poly<NB, ENV>& p, bool one) {
     Node o;
     uint64_t gp;
     if constexpr (ENV) {
-        const uint64_t e = one ? envelope(p, 0, true) : 0x7fffffffffffffffull;
+        const Envelope v = one ? envelope(p, 0, true) : Envelope{0x7fffffffffffffffull, 0};
+        const uint64_t e = shrRound(v.m, v.n);
         rect<EXPR, DERIV>(p.a + mulhiAny(q, e << 1) - e, o, gp);
-        if constexpr (DERIV) o.fe = mulhi(gp, e);
+        if constexpr (DERIV) {
+            o.fe = mulhiRound(gp, v.m);
+            o.n = v.n;
+        }
     } else {
         rect<EXPR, DERIV>(q, o, gp);
     }
@@ -500,7 +531,7 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
                        Threshold thr, int ms, Sums<NM>& R) {
     constexpr bool D = NM > 0;
     uint64_t stG[32], stF[D && !EXPR ? 32 : 1], stFe[D && ENV ? 32 : 1];
-    int stE[EXPR ? 32 : 1];
+    int stE[EXPR ? 32 : 1], stN[D && ENV ? 32 : 1];
     R.g = R.m0 = 0;
     R.E = -200;
     R.over = false;
@@ -536,11 +567,20 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
             R.g += shrRound(ih, dn);
             if constexpr (D) {
                 uint64_t fa, fb, fm, fv, fw;
+                int tail = 0;  // the moments' units below: 2^(-62 - tail)
                 if constexpr (ENV) {
-                    fa = A.fe; fb = B.fe; fm = M.fe; fv = V.fe; fw = W.fe;
+                    // The shift to t = 0 multiplies an interval's moments, and
+                    // their rounding, by up to 2^(ms j): intervals under a small
+                    // envelope (largest at the left end) carry more bits, as many
+                    // as the shifted moments leave room for.  (Without them an
+                    // order-5 J_k was 2e-15 of its integral off at |x_D| = 10.)
+                    tail = A.n - ms * NM - 1;
+                    tail = tail > 0 ? tail : 0;
+                    const int da = EXPR ? E - tail : -tail;
+                    fa = shrRound(A.fe, da + A.n - A.E); fb = shrRound(B.fe, da + B.n - B.E);
+                    fm = shrRound(M.fe, da + M.n - M.E); fv = shrRound(V.fe, da + V.n - V.E);
+                    fw = shrRound(W.fe, da + W.n - W.E);
                     if constexpr (EXPR) {
-                        fa = shr(fa, E - A.E); fb = shr(fb, E - B.E); fm = shr(fm, E - M.E);
-                        fv = shr(fv, E - V.E); fw = shr(fw, E - W.E);
                         R.m0 = R.g;
                     } else {
                         R.m0 += shrRound(mulhi(A.f + B.f, Q.w0) + mulhi(M.f, Q.wM) + mulhi(V.f + W.f, Q.w1), level);
@@ -551,26 +591,35 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
                     fa = A.f; fb = B.f; fm = M.f; fv = V.f; fw = W.f;
                 }
                 uint64_t mu[NM];
-                fb = mulhi(fb, Q.w0);
-                fm = mulhi(fm, Q.wM);
-                mu[0] = mulhi(fa, Q.w0) + fb + fm + mulhi(fv + fw, Q.w1);
+                // (The envelope makes terms of a few units, which the shift to
+                // t = 0 multiplies by up to 2^(5 j): products and shifts are
+                // rounded to nearest, ties either way.  Halves up and the
+                // short product's mean were 6e-17 of the fifth moment of every
+                // point, 1e-15 of an order-5 gradient.)
+                auto mul = [](uint64_t x, uint64_t y) {
+                    if constexpr (ENV) return mulhiRound(x, y);
+                    else return mulhi(x, y);
+                };
+                fb = mul(fb, Q.w0);
+                fm = mul(fm, Q.wM);
+                mu[0] = mul(fa, Q.w0) + fb + fm + mul(fv + fw, Q.w1);
 #pragma unroll
-                for (int j = 1; j < NM; ++j) mu[j] = fb + ((fm + ((1ull << j) >> 1)) >> j) + mulhi(fv, Q.mLo[j]) + mulhi(fw, Q.mHi[j]);
+                for (int j = 1; j < NM; ++j) mu[j] = fb + ((fm + ((1ull << j) >> 1)) >> j) + mul(fv, Q.mLo[j]) + mul(fw, Q.mHi[j]);
 #pragma unroll
                 for (int j = 0; j < NM; ++j) {
-                    if constexpr (ENV) mu[j] = scaleRound(mu[j], level * j + dn - ms * (EXPR ? j : j + 1));
+                    if constexpr (ENV) mu[j] = scaleEven(mu[j], level * j + dn - ms * (EXPR ? j : j + 1));
                     else mu[j] = shrRound(mu[j], level * j + dn);
                 }
 #pragma unroll
                 for (int i = 0; i + 1 < NM; ++i) {
 #pragma unroll
                     for (int j = NM - 1; j > i; --j) {
-                        if constexpr (ENV) mu[j] += mul32Round(mu[j - 1], lo) << ms;
+                        if constexpr (ENV) mu[j] += mul32Round(mu[j - 1], lo, (uint32_t)mu[j] & 1) << ms;
                         else mu[j] += mul32Round(mu[j - 1], lo);
                     }
                 }
 #pragma unroll
-                for (int j = 0; j < NM; ++j) R.m[j] += mu[j];
+                for (int j = 0; j < NM; ++j) R.m[j] += ENV ? scaleEven(mu[j], tail) : mu[j];
             }
             if constexpr (EXPR) {
                 if (R.g >> 62) {
@@ -596,7 +645,10 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
             if constexpr (D) {
                 if constexpr (EXPR) B.f = B.g;
                 else B.f = stF[L];
-                if constexpr (ENV) B.fe = stFe[L];
+                if constexpr (ENV) {
+                    B.fe = stFe[L];
+                    B.n = stN[L];
+                }
             }
         } else {
             ++level;
@@ -604,7 +656,10 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
             stG[level] = B.g;
             if constexpr (EXPR) stE[level] = B.E;
             if constexpr (D && !EXPR) stF[level] = B.f;
-            if constexpr (D && ENV) stFe[level] = B.fe;
+            if constexpr (D && ENV) {
+                stFe[level] = B.fe;
+                stN[level] = B.n;
+            }
             B = M;
         }
         if (count >= maxIntervals) {

@@ -42,3 +42,23 @@ def test_tight_absolute_tolerances(lib, expr, x, abs_tol):
         else:
             assert 0 < out[0] <= 2 ** 13
             assert out[1] <= 2.0 ** -53 + abs_tol / x
+
+
+@pytest.mark.parametrize("expr", [0, 1])
+def test_hermite_function_moments_have_no_common_bias(lib, expr):
+    """The moments' errors average out over points, up to the envelope's order
+    4 and beyond: those of Hermite functions meet in alternating sums, where a
+    common 6e-17 of the fifth came back as 1e-15 of an order-5 gradient.  A
+    moment's error is some 4e-16 at worst (j = 5, over these points): the mean
+    of 40,000 is within 4 x 4e-16 / 200 = 8e-18, and the functions' own
+    2^-57 = 7e-18 on top."""
+    r = np.random.default_rng(17 + expr)
+    n = 40_000
+    x = np.where(np.arange(n) % 2 == 0, r.standard_normal(n), r.standard_normal(n) ** 2 + 0.5 * r.standard_normal(n))
+    x = np.where(np.abs(x) < 1e-3, 1e-3, x)
+    b = r.normal(0.0, 0.1, (n, 6)) * np.sign(x)[:, None] ** np.arange(6) * np.abs(x)[:, None] ** np.arange(6)
+    b *= np.minimum(1.0, 25.0 / np.abs(b).sum(1))[:, None]
+    a = 0.5 + 0.05 * r.standard_normal(n)
+    mean = np.zeros(6)
+    lib.fa_moment_bias(expr, _p(b), _p(a), _p(x), ctypes.c_long(n), ctypes.c_double(1e-7), _p(mean))
+    assert np.all(np.abs(mean) <= 1.5e-17), mean
