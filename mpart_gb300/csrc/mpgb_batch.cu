@@ -144,13 +144,14 @@ __global__ void segScatterKernel(const SortSeg* segs, const int* chunkSeg, const
 struct GatherSeg {
     const double* src;
     const int32_t* slotTerm;
+    const uint8_t* slotOrder;
     int off, nSlots;
 };
 
 __global__ void __launch_bounds__(512) gatherSegKernel(const GatherSeg* g, double* cm, int2* cmFx, int* scale) {
     const GatherSeg s = g[blockIdx.x];
-    gatherComponent(s.src, s.slotTerm, s.nSlots, cm + s.off, cmFx ? cmFx + s.off : nullptr, scale + blockIdx.x,
-                    kNoLimbs);
+    gatherComponent(s.src, s.slotTerm, s.slotOrder, s.nSlots, cm + s.off, cmFx ? cmFx + s.off : nullptr,
+                    scale + blockIdx.x * kFxScales);
 }
 
 // Fixed-order reduction of each component's partial rows (the single-map
@@ -462,12 +463,13 @@ private:
         for (auto& bc : comps_) {
             const auto& part = maps_[bc.map]->Parts()[bc.part];
             part.owner->CheckCoefficients("MapBatch");
-            g.push_back({part.owner->Coeffs() + part.coeffOffset, bc.prog->dSlotTerm, bc.slotOffset, bc.prog->nSlots});
+            g.push_back({part.owner->Coeffs() + part.coeffOffset, bc.prog->dSlotTerm, bc.prog->dSlotOrder, bc.slotOffset,
+                         bc.prog->nSlots});
         }
         upload(gatherBuf_, g, s);
         cm_.ensure(std::max(1, totalSlots_) * sizeof(double));
         cmFx_.ensure((totalSlots_ + 1) * sizeof(int2));
-        cmScale_.ensure(nC * sizeof(int));
+        cmScale_.ensure(nC * kFxScales * sizeof(int));
         gatherSegKernel<<<nC, 512, 0, s>>>(gatherBuf_.as<GatherSeg>(), cm_.as<double>(),
                                            limbMap(basis_, 1) ? cmFx_.as<int2>() : nullptr, cmScale_.as<int>());
         MPGB_CUDA(cudaGetLastError());

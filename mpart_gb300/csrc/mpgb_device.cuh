@@ -182,56 +182,120 @@ __device__ __forceinline__ double prefixProduct(int depth, const int* r, const d
     return phi;
 }
 
+// Largest last-input order the fixed-point kernels are built for.
+constexpr int kFxMaxOrder = 6;
+
+// A coefficient for the fixed-point phase A: c 2^-s = (h 2^28 + l) 2^-58 with
+// |l| <= 2^27 and 2^s above four times the largest |c| of its last-input order
+// (|h| <= 2^28: the sums of 16 nodes in phaseALimbs stay in 64 bits).  The
+// orders are separate sums a_k and d_D f has none of a_0: with one exponent for
+// the component a constant term of 1e7 moved log-determinants by 6e-10.
+// A component has kFxScales exponents, the last of them 0 or kNoLimbs.
+constexpr int kFxScales = kFxMaxOrder + 2;
+constexpr int kNoLimbs = 1 << 20;
+// Which order a slot's coefficient belongs to (ComponentProgram::slotOrder),
+// with kRootSlot for those of the root (product 1).
+constexpr int kRootSlot = 128;
+// An order whose largest coefficient is not the root's and stands this many
+// bits above both the root's and 1 (order 0, the size of T: above 2^10) keeps
+// FP64: at a point where its product vanishes the rest would be left with the
+// bits below it.
+constexpr int kFxSpan = 6, kFxSpanValue = 10;
+
 // One block gathers a component's coefficients into its slots, as doubles (cm)
-// and, unless limbs is null, as limbs scaled by 2^-s (see kNoLimbs).  The
-// first kGatherKeep values of a thread stay in registers between the two.
-__device__ __forceinline__ void gatherComponent(const double* src, const int32_t* slotTerm, int nSlots, double* cm,
-                                                int2* limbs, int* scale, int noLimbs) {
-    constexpr int kGatherKeep = 4;
-    __shared__ double red[32];
-    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5, nw = blockDim.x >> 5, step = blockDim.x;
-    double s = 0.0, v[kGatherKeep];
+// and, unless limbs is null, as limbs scaled by 2^-s of their order (scale, see
+// kNoLimbs).  The first kGatherKeep values of a thread stay in registers
+// between the two.
+__device__ __forceinline__ void gatherComponent(const double* src, const int32_t* slotTerm, const uint8_t* slotOrder,
+                                                int nSlots, double* cm, int2* limbs, int* scale) {
+    constexpr int kGatherKeep = 4, kOrders = kFxMaxOrder + 1;
+    __shared__ int top[2][kOrders];  // bounds of the root's |c| and of the largest other
+    const int lane = threadIdx.x & 31, step = blockDim.x;
+    double v[kGatherKeep];
+    int ord[kGatherKeep];
     bool bad = false;
 #pragma unroll
     for (int q = 0; q < kGatherKeep; ++q) {
         const int j = threadIdx.x + q * step;
         const int t = j < nSlots ? slotTerm[j] : -1;
+        ord[q] = (limbs && j < nSlots) ? slotOrder[j] : 0;
         v[q] = t >= 0 ? src[t] : 0.0;
     }
+    if (!limbs) {
+#pragma unroll
+        for (int q = 0; q < kGatherKeep; ++q)
+            if ((int)threadIdx.x + q * step < nSlots) cm[threadIdx.x + q * step] = v[q];
+        for (int j = threadIdx.x + kGatherKeep * step; j < nSlots; j += step) {
+            const int t = slotTerm[j];
+            cm[j] = t >= 0 ? src[t] : 0.0;
+        }
+        return;
+    }
+    if (threadIdx.x < 2 * kOrders) top[0][threadIdx.x] = -1023;
+    __syncthreads();
+    int m[2][kOrders];
+#pragma unroll
+    for (int k = 0; k < kOrders; ++k) m[0][k] = m[1][k] = -1023;
+    auto see = [&](double x, int o) {
+        const int e = fx::expBound(x);
+        bad |= e > 900;
+#pragma unroll
+        for (int k = 0; k < kOrders; ++k) {
+            if (o == (k | kRootSlot)) m[0][k] = max(m[0][k], e);
+            if (o == k) m[1][k] = max(m[1][k], e);
+        }
+    };
 #pragma unroll
     for (int q = 0; q < kGatherKeep; ++q) {
         const int j = threadIdx.x + q * step;
-        if (j < nSlots) cm[j] = v[q];
-        s = fmax(s, fabs(v[q]));
-        bad |= !(fabs(v[q]) < 0x1p900);
+        if (j < nSlots) {
+            cm[j] = v[q];
+            see(v[q], ord[q]);
+        }
     }
     for (int j = threadIdx.x + kGatherKeep * step; j < nSlots; j += step) {
         const int t = slotTerm[j];
         const double x = t >= 0 ? src[t] : 0.0;
         cm[j] = x;
-        s = fmax(s, fabs(x));
-        bad |= !(fabs(x) < 0x1p900);
+        see(x, slotOrder[j]);
     }
-    if (!limbs) return;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) s = fmax(s, __shfl_xor_sync(0xffffffffu, s, o));
-    if (lane == 0) red[wp] = s;
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+        for (int k = 0; k < kOrders; ++k) {
+            const int e = __reduce_max_sync(0xffffffffu, m[r][k]);
+            if (lane == 0) atomicMax(&top[r][k], e);
+        }
     bad = __syncthreads_or(bad);
-    s = 0.0;
-    for (int q = 0; q < nw; ++q) s = fmax(s, red[q]);
-    const bool ok = !bad && (s == 0.0 || s > 0x1p-900);
-    const int e = s == 0.0 ? 0 : fx::expBound(s) + 2;
-    if (threadIdx.x == 0) *scale = ok ? e : noLimbs;
+    bool ok = !bad;
+    int s[kOrders];
+#pragma unroll
+    for (int k = 0; k < kOrders; ++k) {
+        const int root = top[0][k], rest = top[1][k], all = max(root, rest);
+        s[k] = all < -900 ? 0 : all + 2;
+        ok = ok && (all >= -900 || all <= -1022) && (rest <= (k == 0 ? kFxSpanValue : kFxSpan) || rest <= root + kFxSpan);
+    }
+    if (threadIdx.x < kFxScales) {
+        int x = ok ? 0 : kNoLimbs;
+#pragma unroll
+        for (int k = 0; k < kOrders; ++k)
+            if ((int)threadIdx.x == k) x = s[k];
+        scale[threadIdx.x] = x;
+    }
     if (!ok) return;
-    auto put = [&](int j, double x) {
+    auto put = [&](int j, double x, int o) {
+        int e = 0;
+#pragma unroll
+        for (int k = 0; k < kOrders; ++k)
+            if ((o & (kRootSlot - 1)) == k) e = s[k];
         const long long f = fx::toFixed(x, 58 - e);
         const long long h = (f + (1ll << 27)) >> 28;
         limbs[j] = make_int2((int)h, (int)(f - (h << 28)));
     };
 #pragma unroll
     for (int q = 0; q < kGatherKeep; ++q)
-        if ((int)threadIdx.x + q * step < nSlots) put(threadIdx.x + q * step, v[q]);
-    for (int j = threadIdx.x + kGatherKeep * step; j < nSlots; j += step) put(j, cm[j]);
+        if ((int)threadIdx.x + q * step < nSlots) put(threadIdx.x + q * step, v[q], ord[q]);
+    for (int j = threadIdx.x + kGatherKeep * step; j < nSlots; j += step) put(j, cm[j], slotOrder[j]);
 }
 
 // Sort bucket of a point by |x_D| (256 buckets): width 1/32 below 4, width 1/4

@@ -277,6 +277,7 @@ struct DevBuf {
 struct GatherDescHost {
     const double* src;
     const int32_t* slotTerm;
+    const uint8_t* slotOrder;
     int slotOffset;
     int nSlots;
 };
@@ -376,8 +377,8 @@ namespace mpgb {
 __global__ void __launch_bounds__(512) gatherMultiKernel(const GatherDescHost* descs, double* cm, int2* cmFx,
                                                          int* scale) {
     const GatherDescHost g = descs[blockIdx.x];
-    gatherComponent(g.src, g.slotTerm, g.nSlots, cm + g.slotOffset, cmFx ? cmFx + g.slotOffset : nullptr,
-                    scale + blockIdx.x, kNoLimbs);
+    gatherComponent(g.src, g.slotTerm, g.slotOrder, g.nSlots, cm + g.slotOffset, cmFx ? cmFx + g.slotOffset : nullptr,
+                    scale + blockIdx.x * kFxScales);
 }
 
 __global__ void sumRowsKernel(const double* rows, int nRows, long long N, double* out, long long outStride) {
@@ -687,7 +688,7 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
                              cudaMemcpyHostToDevice));
         W.cm.ensure(std::max(1, W.totalSlots) * sizeof(double), stream);
         W.cmFx.ensure((W.totalSlots + 1) * sizeof(int2), stream);
-        W.cmScale.ensure(W.hostComps.size() * sizeof(int), stream);
+        W.cmScale.ensure(W.hostComps.size() * kFxScales * sizeof(int), stream);
         W.status.ensure(sizeof(int) * 4, stream);
         MPGB_CUDA(cudaMemset(W.status.p, 0, sizeof(int) * 4));
         W.built = true;
@@ -697,7 +698,7 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
     int off = 0;
     for (auto& pt : parts_) {
         pt.owner->CheckCoefficients("MonotoneComponent");
-        g.push_back({pt.owner->Coeffs() + pt.coeffOffset, pt.prog->dSlotTerm, off, pt.prog->nSlots});
+        g.push_back({pt.owner->Coeffs() + pt.coeffOffset, pt.prog->dSlotTerm, pt.prog->dSlotOrder, off, pt.prog->nSlots});
         off += pt.prog->nSlots;
     }
     bool same = g.size() == W.hostGather.size();

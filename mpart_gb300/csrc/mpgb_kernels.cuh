@@ -728,7 +728,7 @@ __device__ __forceinline__ bool fillLeadLimbs(const CompDesc& c, const SmemLayou
 // tree order).  Every thread of the block calls it; outliers only stage.
 template <int PMAX>
 __device__ __forceinline__ void phaseALimbs(const CompDesc& c, const SmemLayout& L, int tid, const int2* cl, int room,
-                                            bool outlier, int e, int scale, double* a, double* pc) {
+                                            bool outlier, int e, const int* scale, double* a, double* pc) {
     const int tpb = blockDim.x;
     const int rowB = tpb * 8;
     long long hh[PMAX + 1], m[PMAX + 1];
@@ -820,9 +820,9 @@ __device__ __forceinline__ void phaseALimbs(const CompDesc& c, const SmemLayout&
     }
     if (outlier) return;
     fold();
-    const double sc = ldexp(1.0, e + scale - 60);
 #pragma unroll
     for (int k = 0; k <= PMAX; ++k) {
+        const double sc = ldexp(1.0, e + __ldg(&scale[k]) - 60);
         double v = (double)(long long)lo[k];
         // (a total beyond 64 bits)
         if (up[k] != (int)((long long)lo[k] >> 63)) v = fma((double)up[k], 0x1p64, (double)lo[k]);
@@ -999,12 +999,11 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
             // a_k when no coefficient gradient is asked for).
             constexpr bool kLimbs = limbBasis<BASIS, PMAX>();
             bool limbs = false, outlier = false;
-            int phiScale = 0, cScale = 0;
+            int phiScale = 0;
             if constexpr (kLimbs) {
                 if (prm.cmFx && prm.stageDoubles >= kStageMin &&
                     (!(flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) || (flags & kFlagImplicit))) {
-                    cScale = __ldg(&prm.cmScale[ci]);
-                    limbs = cScale != kNoLimbs;
+                    limbs = __ldg(&prm.cmScale[ci * kFxScales + kFxScales - 1]) != kNoLimbs;
                 }
             }
             if (limbs) {
@@ -1029,8 +1028,8 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                              : nullptr;
             if (kLimbs && limbs) {
                 if constexpr (kLimbs) {
-                    phaseALimbs<PMAX>(c, L, tid, prm.cmFx + c.slotOffset, prm.stageDoubles, outlier, phiScale, cScale, a,
-                                      rc);
+                    phaseALimbs<PMAX>(c, L, tid, prm.cmFx + c.slotOffset, prm.stageDoubles, outlier, phiScale,
+                                      prm.cmScale + ci * kFxScales, a, rc);
                     if (outlier) phaseA<PMAX>(c, L, tid, cm, a, nullptr);
                     else if (flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) fillLead<BASIS>(c, L, tid, prm.bc);
                 }

@@ -83,13 +83,15 @@ namespace noalloc {
 struct GatherDesc {
     const double* src;
     const int32_t* slotTerm;
+    const uint8_t* slotOrder;
     int slotOffset;
     int nSlots;
 };
 
 __global__ void __launch_bounds__(512) gatherNA(const GatherDesc* descs, double* cm, int2* cmFx, int* scale) {
     const GatherDesc g = descs[blockIdx.x];
-    gatherComponent(g.src, g.slotTerm, g.nSlots, cm + g.slotOffset, cmFx + g.slotOffset, scale + blockIdx.x, kNoLimbs);
+    gatherComponent(g.src, g.slotTerm, g.slotOrder, g.nSlots, cm + g.slotOffset, cmFx + g.slotOffset,
+                    scale + blockIdx.x * kFxScales);
 }
 
 // Bump allocator over the static array (offsets only; nothing is allocated).
@@ -167,7 +169,7 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         d.nodeA = p.dNodeA; d.nodeSlot = p.dNodeSlot; d.nodeC = p.dNodeC; d.nodeCRows = p.dNodeCRows;
         d.slotTerm = p.dSlotTerm; d.leadDeg = p.dLeadDeg; d.rowOff = p.dRowOff;
         parts[c].owner->CheckCoefficients("FusedForwardAdjoint (no allocation)");
-        gather[c] = {parts[c].owner->Coeffs() + parts[c].coeffOffset, p.dSlotTerm, slotOff, p.nSlots};
+        gather[c] = {parts[c].owner->Coeffs() + parts[c].coeffOffset, p.dSlotTerm, p.dSlotOrder, slotOff, p.nSlots};
         slotOff += p.nSlots;
         pm = std::max(pm, p.P);
         dmax = std::max(dmax, p.D);
@@ -197,7 +199,7 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
     const size_t oRows = cv.take(std::max<size_t>(1, rowBase.size()) * sizeof(long long));
     const size_t oCm = cv.take(std::max(1, slotOff) * sizeof(double));
     const size_t oCmFx = cv.take((slotOff + 1) * sizeof(int2));
-    const size_t oScale = cv.take(nComps * sizeof(int));
+    const size_t oScale = cv.take(nComps * kFxScales * sizeof(int));
     const size_t oPart = cv.take(std::max<long long>(1, partBase) * sizeof(double));
     if (cv.used > kNoAllocScratchBytes) {
         std::ostringstream os;

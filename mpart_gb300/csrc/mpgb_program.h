@@ -87,8 +87,10 @@ struct ComponentProgram {
     std::vector<uint32_t> nodeA, nodeSlot, nodeC;
     std::vector<uint16_t> nodeCRows;
     std::vector<int32_t> slotTerm, leadDeg, rowOff, nodeCIdx, nodeCRow;
+    std::vector<uint8_t> slotOrder;  // a slot's last-input order, with kRootSlot for the root's
     uint32_t *dNodeA = nullptr, *dNodeSlot = nullptr, *dNodeC = nullptr;
     uint16_t* dNodeCRows = nullptr;
+    uint8_t* dSlotOrder = nullptr;
     int32_t *dSlotTerm = nullptr, *dLeadDeg = nullptr, *dRowOff = nullptr, *dNodeCIdx = nullptr, *dNodeCRow = nullptr;
     // Work per point (FP64 operations of phases A and C), for load balancing.
     double weight = 1.0;
@@ -199,6 +201,7 @@ struct ComponentProgram {
             for (int k = 0; k < nk; ++k) {
                 auto it = t.kTerm.find(k);
                 slotTerm.push_back(it == t.kTerm.end() ? -1 : it->second);
+                slotOrder.push_back((uint8_t)(k | (n == 0 ? kRootSlot : 0)));
             }
             slotOf[n] = slot;
             nkOf[n] = nk;
@@ -246,6 +249,7 @@ struct ComponentProgram {
         dNodeC = toDevice(nodeC);
         dNodeCRows = toDevice(nodeCRows);
         dSlotTerm = toDevice(slotTerm);
+        dSlotOrder = toDevice(slotOrder);
         dLeadDeg = toDevice(leadDeg);
         dRowOff = toDevice(rowOff);
         dNodeCIdx = toDevice(nodeCIdx);
@@ -258,6 +262,7 @@ struct ComponentProgram {
         cudaFree(dNodeC);
         cudaFree(dNodeCRows);
         cudaFree(dSlotTerm);
+        cudaFree(dSlotOrder);
         cudaFree(dLeadDeg);
         cudaFree(dRowOff);
         cudaFree(dNodeCIdx);

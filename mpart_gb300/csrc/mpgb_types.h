@@ -76,9 +76,6 @@ enum FusedFlags : int {
     kFlagImplicitFirst = 512,  // with kFlagImplicit: the sums start at zero (first launch)
 };
 
-// Largest last-input order the fixed-point kernels are built for.
-constexpr int kFxMaxOrder = 6;
-
 // Where the fixed-point phase A is used: Hermite polynomials.  The linear
 // first function of the HermiteFunctions basis has no normalisation, so on
 // data with long tails most tiles hold points beyond the scale (6-D order-5
@@ -86,11 +83,6 @@ constexpr int kFxMaxOrder = 6;
 __host__ __device__ constexpr bool limbMap(int basis, int pmax) {
     return basis == kBasisProbHermite && pmax <= kFxMaxOrder;
 }
-
-// A coefficient for the fixed-point phase A: c 2^-s = (h 2^28 + l) 2^-58 with
-// |l| <= 2^27 and 2^s above four times the component's largest |c| (|h| <=
-// 2^28: the sums of 16 nodes in phaseALimbs stay in 64 bits).
-constexpr int kNoLimbs = 1 << 20;
 
 // One component's reductions at the end of a KL step: its partial rows
 // [rowOff, rowOff + nRows) of rowBase into grad[outOff .. outOff + nTerms) and
@@ -145,9 +137,9 @@ struct FusedParams {
     long long rcStride;  // batch launches: doubles of rcache per block, of at most rcBlocks blocks
     int rcBlocks;
     // Monotone components, fixed-point phase A and reduction: the gathered
-    // coefficients as limbs (LimbCoef) and, per component, the exponent s they
-    // were scaled by (kNoLimbs: not finite); null: FP64.  rcache then holds
-    // the products' limbs.
+    // coefficients as limbs and, per component, kFxScales exponents (the last
+    // kNoLimbs: not finite, or too far apart); null: FP64.  rcache then holds the
+    // products' limbs.
     const int2* cmFx;
     const int* cmScale;
     // Optional: per point and component, the quadrature's interval count / 8

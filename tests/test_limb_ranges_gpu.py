@@ -1,0 +1,81 @@
+"""Coefficients of very different sizes: the fixed-point phase A holds each sum
+a_k to its own terms, as FP64 does.
+
+Tolerances.  Log-determinants of a map whose constant term changes are compared
+with the same map without it: a_k, k >= 1, does not meet the constant, so they
+agree to the rounding of a_k, 1e-15 relative to terms of at most 10.  Gradients
+are compared with the sum of the per-point ones (FP64 products) relative to the
+sum of their magnitudes, 3e-14: a fixed-point sum over a tile keeps 2^-53.5 of
+its largest product and weight, and those add up to 2^-8 of it or more here."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _dev(a):
+    import torch
+    return torch.as_tensor(np.ascontiguousarray(a), dtype=torch.float64, device="cuda")
+
+
+def _opts(M, pos="SoftPlus", basis="ProbabilistHermite"):
+    return M.MapOptions(quadType=M.QuadTypes.AdaptiveClenshawCurtis, posFuncType=getattr(M.PosFuncTypes, pos),
+                        basisType=getattr(M.BasisTypes, basis))
+
+
+def _check_gradient(M, comp, x, sens, ld_scale=0.0):
+    import torch
+    n = x.shape[1]
+    y, ld, cg = (torch.zeros(s, dtype=torch.float64, device="cuda") for s in ((1, n), (n,), (comp.numCoeffs,)))
+    comp.FusedForwardAdjointImpl(_dev(x), sens=_dev(sens), logdet_sens_scale=ld_scale, out_eval=y, out_logdet=ld,
+                                 coeff_grad=cg)
+    dense = comp.CoeffGrad(_dev(x), _dev(sens)).cpu().numpy().astype(np.longdouble)
+    if ld_scale:
+        dense = dense + ld_scale * comp.LogDeterminantCoeffGrad(_dev(x)).cpu().numpy().astype(np.longdouble)
+    err = np.abs(cg.cpu().numpy() - dense.sum(1))
+    size = np.abs(dense).sum(1)
+    assert np.all(err <= 3e-14 * size), float(np.max(err / np.maximum(size, 1e-300)))
+    return y, ld
+
+
+@pytest.mark.parametrize("pos", ["SoftPlus", "Exp"])
+@pytest.mark.parametrize("c0", [1.0, 1e3, 1e6, 1e9, 1e12, 1e16])
+def test_constant_term(gpu, oracle, c0, pos):
+    import torch
+    M = gpu
+    r = np.random.default_rng(11)
+    mset = M.FixedMultiIndexSet(3, 3)
+    comp, plain = M.CreateComponent(mset, _opts(M, pos)), M.CreateComponent(mset, _opts(M, pos))
+    c = r.normal(0.0, 0.1, comp.numCoeffs)
+    c[0] = 0.0
+    plain.SetCoeffs(c)
+    c[0] = c0
+    comp.SetCoeffs(c)
+    x, sens = r.standard_normal((3, 5000)), r.standard_normal((1, 5000))
+    d = (comp.LogDeterminant(_dev(x)) - plain.LogDeterminant(_dev(x))).abs().max()
+    assert float(d) <= 1e-14
+    # (T itself: the constant plus T without it, each rounded)
+    t, t0 = comp.Evaluate(_dev(x)), plain.Evaluate(_dev(x))
+    assert torch.all((t - c0 - t0).abs() <= 2.0 ** -51 * c0 + 1e-13)
+    _check_gradient(M, comp, x, sens, 0.5)
+
+
+@pytest.mark.parametrize("c", [[0.0, 1e8, 0.3, 0.0, 1.0], [1.0, 1e-9, 1e8, 0.5, 0.2], [1e-7, 1e-7, 2e-7, 1e-8, 1e-7]])
+def test_coefficients_of_one_order(gpu, c):
+    """Terms of one order whose largest coefficient meets a vanishing product:
+    the others keep their digits (a_0 = sum c phi in float64, few roundings)."""
+    import torch
+    M = gpu
+    comp = M.CreateComponent(M.FixedMultiIndexSet.from_multis([[0, 0, 0], [1, 0, 0], [0, 1, 0], [1, 1, 0], [0, 0, 1]]),
+                             _opts(M))
+    comp.SetCoeffs(np.array(c))
+    r = np.random.default_rng(2)
+    x = r.standard_normal((3, 999))
+    x[0, ::2], x[1, ::3] = 1e-9, 0.0
+    ref = M.CreateComponent(M.FixedMultiIndexSet.from_multis([[0, 0, 1]]), _opts(M))
+    ref.SetCoeffs(np.array(c[4:]))
+    got = comp.Evaluate(_dev(x)) - ref.Evaluate(_dev(x))
+    nrm = (2.0 * np.pi) ** -0.25
+    terms = np.stack([c[0] + 0 * x[0], c[1] * nrm * x[0], c[2] * nrm * x[1], c[3] * nrm ** 2 * x[0] * x[1]])
+    size = _dev(np.abs(terms).sum(0) + 2.0 * np.abs(c[4]) + 2.0 * np.abs(x[2]))
+    assert torch.all((got.reshape(-1) - _dev(terms.sum(0))).abs() <= 1e-14 * size)
