@@ -666,8 +666,19 @@ __device__ __forceinline__ void phaseAStaged(const CompDesc& c, const SmemLayout
 // A point's products are scaled by 2^-e with 2^e above any of them, so they
 // carry 57 fraction bits below that bound; points with e > kFxMaxScale or a
 // basis value of 16 or more ("outliers": far tails) keep FP64 products.
+//
+// A small product keeps fewer digits than a double of its size.  In a_k that
+// does not show beside terms of ordinary size; a tile with an input that is
+// below 1/2 at all of its points (and not zero) has none and takes FP64
+// (narrowTile).  A sum over a tile's points keeps 2^-53.5 of the largest product
+// and weight; one whose terms' magnitudes do not add up to kMinShare of those is
+// formed again in FP64 (reduceLimbs; 2e-14 of the sum of magnitudes at worst).
+// Both were relative to the largest alone: gradients of terms in three inputs
+// of size 1e-3 were 1e-8 off.  N(0, 1) inputs: no tile is narrow, one sum in
+// 10^5 (7-D order 6: 4 in 10^4) is formed again.
 // --------------------------------------------------------------------------
 constexpr int kFxMaxScale = 5;
+constexpr int kMinShare = 8;  // 2^-8
 
 template <int BASIS, int PMAX>
 __host__ __device__ constexpr bool limbBasis() {
@@ -712,6 +723,39 @@ __device__ __forceinline__ bool fillLeadLimbs(const CompDesc& c, const SmemLayou
         *reinterpret_cast<int2*>(b) = make_int2((int)(v >> 31), (int)v & 0x7fffffff);
     }
     return false;
+}
+
+// Whether some input of the component that is not zero throughout stays below
+// 1/2 at every active point of the tile.  Every thread of the block calls it.
+__device__ __forceinline__ bool narrowTile(const CompDesc& c, const SmemLayout& L, int tid, bool active) {
+    __shared__ unsigned sWide[4], sSome[4];
+    const int tpb = blockDim.x;
+    bool narrow = false;
+    for (int d0 = 0; d0 < c.D - 1; d0 += 32) {
+        const int nd = min(32, c.D - 1 - d0);
+        unsigned wide = 0, some = 0;
+        for (int d = 0; d < nd; ++d) {
+            const double x = L.X[(d0 + d) * tpb + tid];
+            const int e = (active && __ldg(&c.leadDeg[d0 + d]) > 0) ? fx::expBound(x) : -1022;
+            if (e >= 0) wide |= 1u << d;
+            if (e > -1022) some |= 1u << d;
+        }
+        wide = __reduce_or_sync(0xffffffffu, wide);
+        some = __reduce_or_sync(0xffffffffu, some);
+        if (d0) __syncthreads();
+        if ((tid & 31) == 0) {
+            sWide[tid >> 5] = wide;
+            sSome[tid >> 5] = some;
+        }
+        __syncthreads();
+        wide = some = 0;
+        for (int q = 0; q < (tpb >> 5); ++q) {
+            wide |= sWide[q];
+            some |= sSome[q];
+        }
+        narrow |= (some & ~wide) != 0;
+    }
+    return narrow;
 }
 
 // Phase A of a tile from the points' limb tables.  The tree is staged in
@@ -822,12 +866,33 @@ __device__ __forceinline__ void phaseALimbs(const CompDesc& c, const SmemLayout&
     fold();
 #pragma unroll
     for (int k = 0; k <= PMAX; ++k) {
-        const double sc = ldexp(1.0, e + __ldg(&scale[k]) - 60);
+        // 2^(e + scale - 60): scale is 0 or within 902
+        const double sc = __longlong_as_double((long long)(e + __ldg(&scale[k]) - 60 + 1023) << 52);
         double v = (double)(long long)lo[k];
         // (a total beyond 64 bits)
         if (up[k] != (int)((long long)lo[k] >> 63)) v = fma((double)up[k], 0x1p64, (double)lo[k]);
         a[k] = v * sc;
     }
+}
+
+constexpr int kFxAgain = (int)0x80000000;  // (no product's high limb)
+__device__ __forceinline__ int productSize(int a, int b) { return abs((int)(fx::madWideS(a, b, 0) >> 32)); }
+
+// Whether an order of `check` has a sum of |phi w| below kMinShare over all
+// points of the tile (8 lanes a node, as in reduceLimbs; rarely called).
+static __device__ __noinline__ bool littleSums(const int4* row, const int4* Wl, int perNode, unsigned check) {
+    bool little = false;
+    for (int k = 0; __any_sync(0xffffffffu, check >> k); ++k) {
+        int size = 0;
+        for (int u = 0; 8 * u < perNode; ++u) {
+            const int4 v = row[8 * u], x = Wl[k * perNode + 8 * u];
+            size += (productSize(v.x, x.x) + productSize(v.z, x.z)) >> 3;
+        }
+#pragma unroll
+        for (int o = 1; o < 8; o <<= 1) size += __shfl_xor_sync(0xffffffffu, size, o);
+        little |= (check >> k & 1) && size < (1 << (26 - kMinShare - 3));
+    }
+    return little;
 }
 
 // Sum over the tile's points of phi_n W_k for the nodes of one component, from
@@ -837,9 +902,12 @@ __device__ __forceinline__ void phaseALimbs(const CompDesc& c, const SmemLayout&
 // two points each at a time: 16-byte loads, whole lines of rc, the next
 // nodes' lines in flight during the sums.  Measured with phase A: the dim-8
 // order-4 fused adjoint at 1M points 4.17 -> 3.3 ms.
+// A node with a sum whose terms' magnitudes stay below kMinShare (32 of the
+// points decide, all of them if those do not reach it) is left out and marked in
+// its row of rc, column `mark`; *redo is set.
 template <int PMAX>
-__device__ __forceinline__ void reduceLimbs(const CompDesc& c, const double* rc, const double* W, const int* sE,
-                                            double* part) {
+__device__ __forceinline__ void reduceLimbs(const CompDesc& c, double* rc, const double* W, const int* sE,
+                                            double* part, int mark, int* redo) {
     const int tid = threadIdx.x, tpb = blockDim.x;
     const int lane = tid & 31, q = lane & 7;
     const int perNode = tpb >> 1;  // int4 per row (8 lanes x 4 or 8)
@@ -864,10 +932,12 @@ __device__ __forceinline__ void reduceLimbs(const CompDesc& c, const double* rc,
         if (n0 + step < c.nCNodes) fetch(n0 + step + (lane >> 3), nx);
         const int nkm = __reduce_max_sync(0xffffffffu, nk);
         long long mine = 0;
+        unsigned check = 0;  // orders whose 32 points do not reach kMinShare
 #pragma unroll
         for (int k = 0; k <= PMAX; ++k) {
             if (k < nkm) {
                 long long hh = 0, m1 = 0, m2 = 0;
+                int size = 0;  // sum of |phi w|, 2^32 units
 #pragma unroll
                 for (int u = 0; u < 8; ++u) {
                     if (u == 4) {
@@ -882,6 +952,7 @@ __device__ __forceinline__ void reduceLimbs(const CompDesc& c, const double* rc,
                     hh = fx::madWideS(v.z, x.z, hh);
                     m1 = fx::madWideS(v.z, x.w, m1);
                     m2 = fx::madWideS(v.w, x.z, m2);
+                    if (u < 2) size += productSize(v.x, x.x) + productSize(v.z, x.z);
                 }
                 // Eight lanes' sums need three more bits: the low ones, and
                 // eight of the fraction, apart.  Rounded once, ties to even:
@@ -889,20 +960,65 @@ __device__ __forceinline__ void reduceLimbs(const CompDesc& c, const double* rc,
                 // 1M points.
                 m1 += m2 << 3;
                 long long s = hh + (m1 >> 30);
-                int low = ((int)s & 7) << 8 | ((int)(m1 >> 22) & 255);
+                // (The size rides above the low bits, in 2^15 of its units.)
+                int low = ((int)s & 7) << 8 | ((int)(m1 >> 22) & 255) | (size >> 15) << 14;
                 s >>= 3;
 #pragma unroll
                 for (int o = 1; o < 8; o <<= 1) {
                     s += __shfl_xor_sync(0xffffffffu, s, o);
                     low += __shfl_xor_sync(0xffffffffu, low, o);
                 }
+                // (the largest product and weight: 2^58; no weights: no error)
+                const bool little = (low >> 14) < (1 << (26 - kMinShare - 15)) && k < nk && sE[k] > -900;
+                low &= (1 << 14) - 1;
+                if (little) check |= 1u << k;
                 s += (low + 1023 + (int)((s + (low >> 11)) & 1)) >> 11;
                 if (q == k) mine = s;
             }
         }
-        if (q < nk) {
+        bool again = false;
+        if (__any_sync(0xffffffffu, check)) {
+            const int n = n0 + (lane >> 3);
+            double* row = rc + (long long)(n < c.nCNodes ? (int)__ldg(&c.nodeCRow[n]) : 0) * tpb;
+            again = littleSums(reinterpret_cast<const int4*>(row) + q, Wl, perNode, check);
+            if (again && q == 0) {
+                reinterpret_cast<int2*>(row)[mark] = make_int2(kFxAgain, 0);
+                *redo = 1;
+            }
+        }
+        if (!again && q < nk) {
             const int t = __ldg(&c.slotTerm[slot + q]);
             if (t >= 0) part[t] += (double)mine * ldexp(1.0, sE[q] - 56);
+        }
+    }
+}
+
+// The nodes reduceLimbs marked, in FP64 over the points that are not in `out`
+// (rarely called).
+template <int PMAX>
+__device__ __noinline__ void redoNodes(const CompDesc& c, const double* B, int bstride, const double* W,
+                                       const double* rc, int mark, const unsigned* out, double* part) {
+    const int tpb = blockDim.x;
+    for (int n = threadIdx.x; n < c.nCNodes; n += tpb) {
+        if (reinterpret_cast<const int2*>(rc + (long long)__ldg(&c.nodeCRow[n]) * tpb)[mark].x != kFxAgain) continue;
+        const uint32_t nw = __ldg(&c.nodeC[n]);
+        const int depth = nw & 31, nk = (nw >> 5) & 31, slot = nw >> 10;
+        const uint16_t* rows = c.nodeCRows + (size_t)n * kMaxDepth;
+        double acc[PMAX + 1];
+#pragma unroll
+        for (int k = 0; k <= PMAX; ++k) acc[k] = 0.0;
+        for (int j = 0; j < tpb; ++j) {
+            if ((out[j >> 5] >> (j & 31)) & 1u) continue;
+            double phi = 1.0;
+            for (int d = 0; d < depth; ++d) phi *= B[(int)__ldg(&rows[d]) * bstride + j];
+            accumSlots<PMAX>(nk, phi, W + j, tpb, acc);
+        }
+#pragma unroll
+        for (int k = 0; k <= PMAX; ++k) {
+            if (k < nk) {
+                const int t = __ldg(&c.slotTerm[slot + k]);
+                if (t >= 0) part[t] += acc[k];
+            }
         }
     }
 }
@@ -1007,9 +1123,12 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                 }
             }
             if (limbs) {
-                outlier = fillLeadLimbs<BASIS>(c, L, tid, prm.bc, phiScale);
+                limbs = !narrowTile(c, L, tid, active);
+                if (limbs) outlier = fillLeadLimbs<BASIS>(c, L, tid, prm.bc, phiScale);
+                else fillLead<BASIS>(c, L, tid, prm.bc);
                 // A warp with an outlier walks the tree twice: with more than
                 // one per warp on average the whole tile takes FP64.
+                // (a count in either case: the tables' barrier)
                 if (__syncthreads_count(outlier) > (tpb >> 5)) {
                     limbs = false;
                     if (!outlier) fillLead<BASIS>(c, L, tid, prm.bc);
@@ -1251,7 +1370,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
             if (kLimbs && limbs && rc) {
                 if constexpr (kLimbs) {
                     constexpr int kRound = 8;
-                    __shared__ int sMax[PMAX + 1];
+                    __shared__ int sMax[PMAX + 1], sRedo;
                     __shared__ unsigned sOut[4];
                     __shared__ double sOutW[kRound][PMAX + 1];
                     __shared__ int sOutIdx[kRound];
@@ -1264,6 +1383,7 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                     }
                     if (skip && !outlier && !(flags & kFlagInput)) fillLead<BASIS>(c, L, tid, prm.bc);
                     if (tid <= PMAX) sMax[tid] = -4096;
+                    if (tid == 0) sRedo = 0;
                     __syncthreads();
 #pragma unroll
                     for (int k = 0; k <= PMAX; ++k) {
@@ -1281,13 +1401,23 @@ __device__ __forceinline__ void fusedBody(const FusedParams& prm, const WorkItem
                     }
                     __syncthreads();
                     double* part = prm.partials + item.partialBase;
-                    reduceLimbs<PMAX>(c, rc, L.W, sMax, part);
-                    int nOut = 0, rank = 0;
+                    int nOut = 0, rank = 0, mark = 0;
                     for (int q = 0; q < (tpb >> 5); ++q) {
                         const unsigned x = sOut[q];
+                        if (mark == 32 * q) mark += x == ~0u ? 32 : __ffs(~x) - 1;  // (the first point that is not out)
                         nOut += __popc(x);
                         if (q < (tid >> 5)) rank += __popc(x);
                         else if (q == (tid >> 5)) rank += __popc(x & ((1u << (tid & 31)) - 1u));
+                    }
+                    reduceLimbs<PMAX>(c, rc, L.W, sMax, part, mark, &sRedo);
+                    __syncthreads();
+                    if (sRedo) {
+                        // The marked nodes in FP64, over the points in range.
+                        if (!skip && !(flags & kFlagInput)) fillLead<BASIS>(c, L, tid, prm.bc);
+#pragma unroll
+                        for (int k = 0; k <= PMAX; ++k) L.W[k * tpb + tid] = w[k];
+                        __syncthreads();
+                        redoNodes<PMAX>(c, L.B, L.bstride, L.W, rc, mark, sOut, part);
                     }
                     for (int r0 = 0; r0 < nOut; r0 += kRound) {
                         __syncthreads();

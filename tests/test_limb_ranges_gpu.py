@@ -1,12 +1,15 @@
-"""Coefficients of very different sizes: the fixed-point phase A holds each sum
-a_k to its own terms, as FP64 does.
+"""Coefficients, inputs and adjoint weights of very different sizes: the
+fixed-point phase A and reduced adjoint hold each sum to its own terms, as FP64
+does.  Sums over points are compared with the per-point gradients (FP64
+products) relative to the sum of their magnitudes: no floor.
 
-Tolerances.  Log-determinants of a map whose constant term changes are compared
-with the same map without it: a_k, k >= 1, does not meet the constant, so they
-agree to the rounding of a_k, 1e-15 relative to terms of at most 10.  Gradients
-are compared with the sum of the per-point ones (FP64 products) relative to the
-sum of their magnitudes, 3e-14: a fixed-point sum over a tile keeps 2^-53.5 of
-its largest product and weight, and those add up to 2^-8 of it or more here."""
+Tolerances.  A sum of products whose magnitudes add up to 2^-8 of the largest
+product and weight of their tile keeps 2^-53.5 of the latter, 2e-14 of its own
+size; below that it is formed in FP64.  The per-point gradients and their sum
+add a few 1e-16: 3e-14.  Log-determinants of a map whose constant term changes
+are compared with the same map without it: a_k, k >= 1, does not meet the
+constant, so they agree to the rounding of a_k, 1e-15 relative to terms of at
+most 10."""
 import numpy as np
 import pytest
 
@@ -36,6 +39,41 @@ def _check_gradient(M, comp, x, sens, ld_scale=0.0):
     size = np.abs(dense).sum(1)
     assert np.all(err <= 3e-14 * size), float(np.max(err / np.maximum(size, 1e-300)))
     return y, ld
+
+
+@pytest.mark.parametrize("n", [1, 100, 1000, 20_000])
+@pytest.mark.parametrize("scale", [0.3, 1e-1, 1e-2, 1e-3, 1e-4, 1e-6, 1e-9])
+def test_small_inputs(gpu, oracle, scale, n):
+    M = gpu
+    r = np.random.default_rng(n)
+    comp = M.CreateComponent(M.FixedMultiIndexSet(4, 4), _opts(M))
+    c = r.normal(0.0, 0.1, comp.numCoeffs)
+    comp.SetCoeffs(c)
+    x = r.standard_normal((4, n))
+    x[:3] *= scale
+    _check_gradient(M, comp, x, r.standard_normal((1, n)), 0.7)
+
+
+@pytest.mark.parametrize("n", [100, 1000, 20_000])
+@pytest.mark.parametrize("kind", ["mixed", "one_hot", "plus_minus_one", "masked"])
+def test_inputs_and_weights_that_do_not_meet(gpu, kind, n):
+    """Products that are small at every point although each input is not, and
+    weights whose largest lie where the products vanish."""
+    M = gpu
+    r = np.random.default_rng(7)
+    comp = M.CreateComponent(M.FixedMultiIndexSet(4, 4), _opts(M))
+    comp.SetCoeffs(r.normal(0.0, 0.1, comp.numCoeffs))
+    x, sens = r.standard_normal((4, n)), r.standard_normal((1, n))
+    if kind == "mixed":  # each input large at a third of the points, tiny elsewhere
+        x[:3] *= np.where(np.arange(n) % 3 == np.arange(3)[:, None], 1.0, 1e-5)
+    elif kind == "one_hot":
+        x[:3] = np.where(np.arange(n) % 3 == np.arange(3)[:, None], 1.0, 1e-7 * x[:3])
+    elif kind == "plus_minus_one":  # He_2 vanishes up to noise
+        x[:3] = np.sign(x[:3]) * (1.0 + 1e-6 * r.standard_normal((3, n)))
+    else:  # the points with weights up to 1e12 have no second input
+        sens *= 10.0 ** np.where(np.arange(n) % 4 == 0, r.uniform(0, 12, n), 0.0)
+        x[1, ::4] = 0.0
+    _check_gradient(M, comp, x, sens)
 
 
 @pytest.mark.parametrize("pos", ["SoftPlus", "Exp"])
