@@ -315,28 +315,70 @@ struct KLPlan {
 };
 
 // Work items and reduction tables of a launch: they depend on the map and the
-// number of points alone, so a call with a size seen before uploads nothing.
-enum class PlanStyle { AllComps, PerComp, Reduced };
+// number of points alone, so a call with a size used lately uploads nothing.
+// Implicit: the reduced launches of the components one by one (InverseCoeffGrad),
+// each with partial rows and node cache of its own from 0.
+enum class PlanStyle { AllComps, PerComp, Reduced, Implicit };
 struct LaunchPlan {
     long long N = -1;
     PlanStyle style = PlanStyle::AllComps;
-    int onlyComp = -1;
     int tpb = 128;
-    bool uploaded = false;  // false after a build inside a stream capture (the copies have not run)
-    bool captured = false;  // a captured graph may read it: kept as long as the map
-    long long used = 0;     // call counter of the last use
     std::vector<WorkItem> items;
     std::vector<long long> rows;       // partial rows, by component
     std::vector<KLReduceDesc> reduce;  // per component
+    std::vector<int> itemOff;          // Implicit: first item of each component
     int maxTerms = 0;
     size_t partialDoubles = 1;
     long long rcTotal = 0;
-    DevBuf dItems, dRows, dReduce;
+    // The three tables on the device, one after another.
+    DevBuf table;
+    size_t rowAt = 0, reduceAt = 0;
+    std::vector<unsigned char> host;  // the copies' source (a captured copy reads it at every replay)
+    bool ready = false;     // the upload has been issued outside a capture
+    bool settled = false;   // ... and the host has waited for it
+    bool inFlight = false;  // asynchronous calls may still be reading the tables
+    bool captured = false;  // a captured graph reads them: kept as they are as long as the map
+    long long used = 0;     // call counter of the last use
+    // After the upload, and after the last asynchronous use on each stream.
+    struct After {
+        cudaStream_t stream;
+        cudaEvent_t event;
+    };
+    std::vector<After> uploads, uses;
+    LaunchPlan() = default;
+    LaunchPlan(const LaunchPlan&) = delete;
+    ~LaunchPlan() {
+        for (auto* v : {&uploads, &uses})
+            for (auto& a : *v) cudaEventDestroy(a.event);
+    }
+    static void mark(std::vector<After>& v, cudaStream_t s) {
+        for (auto& a : v)
+            if (a.stream == s) {
+                MPGB_CUDA(cudaEventRecord(a.event, s));
+                return;
+            }
+        After a{s, nullptr};
+        MPGB_CUDA(cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming));
+        v.push_back(a);
+        MPGB_CUDA(cudaEventRecord(a.event, s));
+    }
+    static void wait(const std::vector<After>& v, cudaStream_t s) {
+        for (auto& a : v)
+            if (a.stream != s) MPGB_CUDA(cudaStreamWaitEvent(s, a.event, 0));
+    }
+    const WorkItem* dItems() const { return (const WorkItem*)table.p; }
+    const long long* dRows() const { return (const long long*)((const char*)table.p + rowAt); }
+    const KLReduceDesc* dReduce() const { return (const KLReduceDesc*)((const char*)table.p + reduceAt); }
 };
-constexpr size_t kMaxPlans = 48;
+// Sets kept per style and map besides those of captured graphs (sizes in turn:
+// the parts of an epoch and its last, a training and a test set), and the
+// table bytes beyond which a style keeps one.
+constexpr int kPlansPerStyle = 8;
+constexpr size_t kPlanBytes = size_t(16) << 20;
 
 struct MapWorkspace {
     std::vector<std::unique_ptr<LaunchPlan>> plans;
+    std::vector<LaunchPlan*> plansInCall;  // since the last Finish
     long long planClock = 0;
     int* hostStatus = nullptr;  // pinned: a pageable copy is staged by the driver
     ~MapWorkspace() {
@@ -643,6 +685,9 @@ void buildLaunchConstants(const MapOptions& o, QuadParams& q, BasisConsts& b) {
 
 void MonotoneMapBase::Prepare(cudaStream_t stream) {
     MapWorkspace& W = *ws_;
+    // (left by a call that threw)
+    for (LaunchPlan* p : W.plansInCall) p->inFlight = true;
+    W.plansInCall.clear();
     if (!W.built) {
         int dev = 0;
         MPGB_CUDA(cudaGetDevice(&dev));
@@ -718,8 +763,21 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
 }
 
 void MonotoneMapBase::Finish(cudaStream_t stream, const char* fn) {
-    if (async_) return;
+    MapWorkspace& W = *ws_;
+    if (async_) {
+        for (LaunchPlan* p : W.plansInCall) {
+            LaunchPlan::mark(p->uses, stream);
+            p->inFlight = true;
+        }
+        W.plansInCall.clear();
+        return;
+    }
     int st = CheckStatus(stream);
+    for (LaunchPlan* p : W.plansInCall) {
+        p->settled = true;  // (the stream has been waited for, and with it the upload)
+        p->inFlight = false;
+    }
+    W.plansInCall.clear();
     if (st & kStatusInf) {
         std::ostringstream os;
         os << fn << ": MonotoneIntegrand: nan was encountered in value of g(df(...)).";
@@ -899,81 +957,140 @@ static double* rectCache(MapWorkspace& W, long long rcTotal, cudaStream_t stream
     return W.rcache.as<double>();
 }
 
-// The plan for (N, style, onlyComp), built on first use.  At most kMaxPlans are
-// kept; the least recently used makes room (after a device synchronisation:
-// launches in flight may still read it).
+// The tables of a plan on the host.
+static void buildPlan(MapWorkspace& W, const std::vector<MonotoneMapBase::Part>& parts, long long N, PlanStyle style,
+                      LaunchPlan& q) {
+    const bool reduced = style == PlanStyle::Reduced || style == PlanStyle::Implicit;
+    const int nComps = (int)parts.size();
+    q.N = N;
+    q.style = style;
+    q.tpb = tileSize(N, W.numSMs, reduced);
+    q.items.clear();
+    q.rows.clear();
+    q.reduce.clear();
+    q.itemOff.clear();
+    q.maxTerms = 0;
+    q.partialDoubles = 1;
+    q.rcTotal = 0;
+    std::vector<std::vector<int>> itemsOf;
+    auto addRows = [&](int c) {
+        const ComponentProgram& g = *parts[c].prog;
+        KLReduceDesc d{};
+        d.rowOff = (int)q.rows.size();
+        for (int id : itemsOf[c])
+            for (int sg = 0; sg < g.cSegs; ++sg) q.rows.push_back(q.items[id].partialBase + (long long)sg * g.numTerms);
+        d.nRows = (int)q.rows.size() - d.rowOff;
+        d.nTerms = g.numTerms;
+        d.outOff = (int)parts[c].mapCoeffOffset;
+        d.comp = c;
+        q.reduce.push_back(d);
+        q.maxTerms = std::max(q.maxTerms, d.nTerms);
+    };
+    if (style == PlanStyle::AllComps) {
+        q.items = itemsAllComps(N, nComps, q.tpb);
+    } else if (style == PlanStyle::Implicit) {
+        for (int c = 0; c < nComps; ++c) {
+            long long rc = 0;
+            auto own = itemsPerComp(parts, N, W.numSMs, true, q.tpb, nullptr, nullptr, c, &rc);
+            q.itemOff.push_back((int)q.items.size());
+            itemsOf.assign(nComps, {});
+            for (auto& it : own) {
+                itemsOf[c].push_back((int)q.items.size());
+                q.items.push_back(it);
+            }
+            q.rcTotal = std::max(q.rcTotal, rc);
+            addRows(c);
+        }
+        q.itemOff.push_back((int)q.items.size());
+    } else {
+        q.items = itemsPerComp(parts, N, W.numSMs, reduced, q.tpb, nullptr, &itemsOf, -1, &q.rcTotal);
+        for (int c = 0; reduced && c < nComps; ++c) addRows(c);
+    }
+    if (reduced)
+        for (auto& it : q.items)
+            q.partialDoubles = std::max<size_t>(
+                q.partialDoubles,
+                (size_t)it.partialBase + (size_t)parts[it.c0].prog->numTerms * parts[it.c0].prog->cSegs);
+    auto at = [&](size_t bytes) { return (bytes + 15) & ~size_t(15); };
+    q.rowAt = at(q.items.size() * sizeof(WorkItem));
+    q.reduceAt = q.rowAt + at(q.rows.size() * sizeof(long long));
+    q.host.resize(std::max<size_t>(16, q.reduceAt + q.reduce.size() * sizeof(KLReduceDesc)));
+    auto put = [&](size_t off, const void* v, size_t bytes) {
+        if (bytes) std::memcpy(q.host.data() + off, v, bytes);
+    };
+    put(0, q.items.data(), q.items.size() * sizeof(WorkItem));
+    put(q.rowAt, q.rows.data(), q.rows.size() * sizeof(long long));
+    put(q.reduceAt, q.reduce.data(), q.reduce.size() * sizeof(KLReduceDesc));
+}
+
+// The plan for (N, style).  A size that is not kept takes the place of the least
+// recently used one, in stream order: its buffer is written after the launches
+// that read it, on whichever stream they run (an event), and neither the host
+// nor other streams wait, so that a sequence of ever new sizes costs one small
+// copy a call.  (Synchronising and giving buffers back instead made the 49th
+// size wait for the whole device, and a first call at a size for its stream.)
+// Inside a capture the tables are copied by the graph too (the same bytes),
+// unless the host has seen their upload end.
 static LaunchPlan& launchPlan(MapWorkspace& W, const std::vector<MonotoneMapBase::Part>& parts, long long N,
-                              PlanStyle style, int onlyComp, cudaStream_t stream) {
-    LaunchPlan* P = nullptr;
-    for (auto& p : W.plans)
-        if (p->N == N && p->style == style && p->onlyComp == onlyComp) P = p.get();
+                              PlanStyle style, cudaStream_t stream) {
     cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
     MPGB_CUDA(cudaStreamIsCapturing(stream, &cs));
     const bool capturing = cs != cudaStreamCaptureStatusNone;
-    if (P) P->captured = P->captured || capturing;
-    if (P && P->uploaded) {
-        P->used = ++W.planClock;
-        return *P;
+    LaunchPlan* P = nullptr;
+    for (auto& p : W.plans)
+        if (p->N == N && p->style == style && (p->ready || (capturing && p->captured))) P = p.get();
+    bool upload = !P;
+    if (P && capturing) {
+        P->captured = true;
+        upload = !P->settled;
     }
     if (!P) {
-        if (W.plans.size() >= kMaxPlans && !capturing) {
-            auto old = std::min_element(W.plans.begin(), W.plans.end(), [](auto const& x, auto const& y) {
-                return x->captured != y->captured ? y->captured : x->used < y->used;
-            });
-            if (!(*old)->captured) {
-                MPGB_CUDA(cudaDeviceSynchronize());
-                W.plans.erase(old);
-            }
-        }
         auto fresh = std::make_unique<LaunchPlan>();
-        LaunchPlan& q = *fresh;
-        q.N = N;
-        q.style = style;
-        q.onlyComp = onlyComp;
-        q.captured = capturing;
-        q.tpb = tileSize(N, W.numSMs, style == PlanStyle::Reduced);
-        if (style == PlanStyle::AllComps) {
-            q.items = itemsAllComps(N, (int)parts.size(), q.tpb);
-        } else {
-            std::vector<std::vector<int>> itemsOf;
-            const bool reduced = style == PlanStyle::Reduced;
-            q.items = itemsPerComp(parts, N, W.numSMs, reduced, q.tpb, nullptr, &itemsOf, onlyComp, &q.rcTotal);
-            for (int c = 0; reduced && c < (int)parts.size(); ++c) {
-                const ComponentProgram& g = *parts[c].prog;
-                KLReduceDesc d{};
-                d.rowOff = (int)q.rows.size();
-                for (int id : itemsOf[c])
-                    for (int sg = 0; sg < g.cSegs; ++sg)
-                        q.rows.push_back(q.items[id].partialBase + (long long)sg * g.numTerms);
-                d.nRows = (int)q.rows.size() - d.rowOff;
-                d.nTerms = g.numTerms;
-                d.outOff = (int)parts[c].mapCoeffOffset;
-                d.comp = c;
-                q.reduce.push_back(d);
-                q.maxTerms = std::max(q.maxTerms, d.nTerms);
-            }
-            if (reduced)
-                for (auto& it : q.items)
-                    q.partialDoubles = std::max<size_t>(
-                        q.partialDoubles, (size_t)it.partialBase +
-                                              (size_t)parts[it.c0].prog->numTerms * parts[it.c0].prog->cSegs);
+        buildPlan(W, parts, N, style, *fresh);
+        const size_t need = fresh->host.size();
+        int kept = 0;
+        size_t bytes = 0;
+        LaunchPlan* old = nullptr;
+        for (auto& p : W.plans) {
+            if (p->captured) continue;
+            bytes += p->table.bytes;
+            if (p->style != style) continue;
+            ++kept;
+            // (a capture can neither wait for a launch outside it nor allocate)
+            if (capturing && (p->inFlight || p->table.bytes < need)) continue;
+            if (!old || p->used < old->used) old = p.get();
         }
-        W.plans.push_back(std::move(fresh));
-        P = W.plans.back().get();
+        if (old && (capturing || kept >= kPlansPerStyle || bytes + need > kPlanBytes)) {
+            if (!capturing) {
+                LaunchPlan::wait(old->uploads, stream);
+                LaunchPlan::wait(old->uses, stream);
+            }
+            buildPlan(W, parts, N, style, *old);
+            P = old;
+        } else {
+            W.plans.push_back(std::move(fresh));
+            P = W.plans.back().get();
+        }
+        P->captured = capturing;
+        P->ready = P->settled = false;
     }
     P->used = ++W.planClock;
-    auto put = [&](DevBuf& d, const void* h, size_t bytes) {
-        d.ensure(std::max<size_t>(bytes, 8), stream);
-        if (bytes) MPGB_CUDA(cudaMemcpyAsync(d.p, h, bytes, cudaMemcpyHostToDevice, stream));
-    };
-    put(P->dItems, P->items.data(), P->items.size() * sizeof(WorkItem));
-    put(P->dRows, P->rows.data(), P->rows.size() * sizeof(long long));
-    put(P->dReduce, P->reduce.data(), P->reduce.size() * sizeof(KLReduceDesc));
-    if (!capturing) {
-        // (the next call may use the plan on another stream)
-        MPGB_CUDA(cudaStreamSynchronize(stream));
-        P->uploaded = true;
+    if (upload) {
+        const size_t need = P->host.size();
+        if (P->table.bytes < need) {
+            size_t room = 16384;
+            while (room < need) room *= 2;
+            P->table.ensure(room, stream);
+        }
+        MPGB_CUDA(cudaMemcpyAsync(P->table.p, P->host.data(), need, cudaMemcpyHostToDevice, stream));
+        if (!capturing) {
+            LaunchPlan::mark(P->uploads, stream);
+            P->ready = true;
+        }
+    } else if (!capturing && !P->settled) {
+        LaunchPlan::wait(P->uploads, stream);
     }
+    if (!capturing) W.plansInCall.push_back(P);
     return *P;
 }
 
@@ -1033,10 +1150,10 @@ static int stageDoubles(const MapWorkspace& W, const FusedParams& p, bool input)
 }
 
 static void launch(MapWorkspace& W, const MapOptions& o, FusedParams& p, const LaunchPlan& plan, int needJ, int needE,
-                   cudaStream_t stream) {
-    const int nItems = (int)plan.items.size();
+                   cudaStream_t stream, int comp = -1) {
+    const int nItems = comp < 0 ? (int)plan.items.size() : plan.itemOff[comp + 1] - plan.itemOff[comp];
     p.tpb = plan.tpb;
-    p.items = plan.dItems.as<WorkItem>();
+    p.items = plan.dItems() + (comp < 0 ? 0 : plan.itemOff[comp]);
     if (nItems == 0) return;
     const size_t smem = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, (p.flags & kFlagInput) != 0);
     if (smem > 227 * 1024) throw std::invalid_argument("Component too large for the shared-memory tile.");
@@ -1071,7 +1188,7 @@ static void inputGradient(MapWorkspace& W, const MapOptions& o, const std::vecto
     const bool split = !async && nComps > 1 && (N + tpb - 1) / tpb < 4LL * W.numSMs && slabBytes <= kMaxSlabBytes;
     if (!split) {
         p.outInput = out.data; p.inputRs = out.rowStride; p.inputCs = out.colStride;
-        launch(W, o, p, launchPlan(W, parts, N, PlanStyle::AllComps, -1, stream), needJ, needE, stream);
+        launch(W, o, p, launchPlan(W, parts, N, PlanStyle::AllComps, stream), needJ, needE, stream);
         return;
     }
     W.inputSlabs.ensure(slabBytes, stream);
@@ -1079,7 +1196,7 @@ static void inputGradient(MapWorkspace& W, const MapOptions& o, const std::vecto
     p.inputRs = N;
     p.inputCs = 1;
     p.inputCompStride = (long long)nDims * N;
-    launch(W, o, p, launchPlan(W, parts, N, PlanStyle::PerComp, -1, stream), needJ, needE, stream);
+    launch(W, o, p, launchPlan(W, parts, N, PlanStyle::PerComp, stream), needJ, needE, stream);
     sumInputGradKernel<<<dim3((unsigned)((N + 127) / 128), (unsigned)nDims), 128, 0, stream>>>(
         W.inputSlabs.as<double>(), W.comps.as<CompDesc>(), nComps, nDims, N, out.data, out.rowStride, out.colStride);
     MPGB_CUDA(cudaGetLastError());
@@ -1112,7 +1229,7 @@ void MonotoneMapBase::EvaluateImpl(StridedMatrix const& pts, StridedMatrix const
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, -1, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     // The reference's EvaluateImpl calls EvaluateSingle without the nugget
@@ -1136,7 +1253,7 @@ void MonotoneMapBase::LogDeterminantImpl(StridedMatrix const& pts, StridedMatrix
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::AllComps, -1, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::AllComps, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagLogDet;
@@ -1158,7 +1275,7 @@ void MonotoneMapBase::CoeffGradImpl(StridedMatrix const& pts, StridedMatrix cons
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, -1, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagCoefDenseT;
@@ -1180,7 +1297,7 @@ void MonotoneMapBase::LogDeterminantCoeffGradImpl(StridedMatrix const& pts, Stri
     if (N == 0) return;
     Prepare(stream);
     MapWorkspace& W = *ws_;
-    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, -1, stream);
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::PerComp, stream);
     FusedParams p{};
     baseParams(W, opts_, p, N);
     p.flags = kFlagCoefDenseL;
@@ -1419,7 +1536,7 @@ void MonotoneMapBase::FusedForwardAdjoint(StridedMatrix const& pts, StridedMatri
     const bool wantLogDet = !outLogDet.empty();
     if (wantCoef || !outEval.empty() || wantLogDet) {
         LaunchPlan& plan =
-            launchPlan(W, parts_, N, wantCoef ? PlanStyle::Reduced : PlanStyle::PerComp, -1, stream);
+            launchPlan(W, parts_, N, wantCoef ? PlanStyle::Reduced : PlanStyle::PerComp, stream);
         FusedParams p{};
         baseParams(W, opts_, p, N);
         p.pts = pts.data; p.ptsRs = pts.rowStride; p.ptsCs = pts.colStride;
@@ -1462,8 +1579,7 @@ void MonotoneMapBase::FusedForwardAdjoint(StridedMatrix const& pts, StridedMatri
         }
         if (wantCoef) {
             // Fixed-order reduction of every component's partial rows.
-            MPGB_CUDA(launchKLReduce(W.partials.as<double>(), plan.dRows.as<long long>(),
-                                     plan.dReduce.as<KLReduceDesc>(), nComps, plan.maxTerms, coeffGrad, nullptr,
+            MPGB_CUDA(launchKLReduce(W.partials.as<double>(), plan.dRows(), plan.dReduce(), nComps, plan.maxTerms, coeffGrad, nullptr,
                                      nullptr, 1.0, nullptr, stream));
         }
     }
@@ -1705,11 +1821,11 @@ void MonotoneMapBase::InverseCoeffGrad(StridedMatrix const& pts, StridedMatrix c
     for (size_t c = 0; c < parts_.size(); ++c) order[c] = (int)c;
     std::stable_sort(order.begin(), order.end(), [&](int a, int b) { return parts_[a].outRow > parts_[b].outRow; });
     const bool wantCoef = coeffGrad != nullptr;
+    // (one plan for all components; the same tiles with and without the
+    // coefficient gradient: the same input gradient to the bit)
+    LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::Implicit, stream);
     for (size_t q = 0; q < order.size(); ++q) {
         const int c = order[q];
-        // (the same tiles with and without the coefficient gradient: the same
-        // input gradient to the bit)
-        LaunchPlan& plan = launchPlan(W, parts_, N, PlanStyle::Reduced, c, stream);
         FusedParams p{};
         baseParams(W, opts_, p, N);
         if (wantCoef) p.rcache = rectCache(W, plan.rcTotal, stream);
@@ -1724,9 +1840,9 @@ void MonotoneMapBase::InverseCoeffGrad(StridedMatrix const& pts, StridedMatrix c
             p.partials = W.partials.as<double>();
         }
         orderPoints(W, parts_, pts, p, c, stream);
-        launch(W, opts_, p, plan, 1, 0, stream);
+        launch(W, opts_, p, plan, 1, 0, stream, c);
         if (wantCoef) {
-            MPGB_CUDA(launchReduceRows(W.partials.as<double>(), plan.dRows.as<long long>(), (int)plan.rows.size(),
+            MPGB_CUDA(launchReduceRows(W.partials.as<double>(), plan.dRows() + plan.reduce[c].rowOff, plan.reduce[c].nRows,
                                        parts_[c].prog->numTerms, -1.0, coeffGrad + parts_[c].mapCoeffOffset, 0,
                                        stream));
         }
