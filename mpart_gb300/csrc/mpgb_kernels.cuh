@@ -378,8 +378,8 @@ struct NodePoly {
 // E follow from the moments.  False (nothing done) where its range does not
 // hold: a rule it is not built for, a nugget, coefficients with
 // sum |b_j| > 31 or not finite, Hermite functions at |x_D| > 52, SoftPlus
-// with d_D f(0) < -4 or, for adjoints, int g' < 2^-6 (g' would lose relative
-// accuracy), or tolerances near the sums' last bit (fx::threshold).  The bounds hold for
+// with d_D f(0) < -4 or, for adjoints, moments of g' below 2^-10 (g' would lose
+// relative accuracy), or tolerances near the sums' last bit (fx::threshold).  The bounds hold for
 // all but the far tails of ordinary maps (dim 8, order 4, N(0, 1) points:
 // every point up to |x_D| = 5).  Measured there at 1M points: the quadrature's
 // share of an evaluation 1.27 -> 0.33 ms, the fused adjoint 5.68 -> 4.17 ms
@@ -445,11 +445,18 @@ __device__ __forceinline__ bool integrateFixed(const double* a, int P, double xd
         R.Ih = __longlong_as_double(0x7ff8000000000000ULL);
         return true;
     }
-    // (A SoftPlus that falls from there on: int g' below 2^-6 leaves its moments
-    // fewer digits than FP64's.  d_D f from -4 to -28 on the way to x_D = 3: an
-    // order-6 J_k 1e-13 off.)
-    if constexpr (NEEDJ && !EXPR)
-        if ((ENV ? S.m0 : S.m[0]) < (1ull << 56)) return false;
+    // (A SoftPlus that falls from there on leaves the moments fewer digits than
+    // FP64's: d_D f from -4 to -28 on the way to x_D = 3, an order-6 J_k 1e-13
+    // off.  The highest moment counts where |x_D| > 1.)
+    if constexpr (NEEDJ && !EXPR) {
+        uint64_t top = ENV ? S.m0 : S.m[0];
+        if (fx::expBound(xd) > 0) {
+#pragma unroll
+            for (int j = 1; j < PMAX; ++j)
+                if (j == P - 1) top = S.m[j];
+        }
+        if (top < (1ull << 52)) return false;
+    }
     // 2^E of the Exp sums (|E| <= 64)
     const double sc = EXPR ? __longlong_as_double((long long)(S.E - 62 + 1023) << 52) : 0x1p-62;
     const double G = (double)S.g * (EXPR ? sc : 0x1p-57);
