@@ -269,7 +269,7 @@ public:
                 depthMax_ = std::max(depthMax_, pg->maxDepth);
                 pclass_ = std::max(pclass_, batchOrderClass(pg->P));
                 maxCNodes_ = std::max(maxCNodes_, pg->nCNodes);
-                stageNeed_ = std::max(stageNeed_, std::max(kStageMin, std::min(kStageCap, pg->nSlots + 2 * (pg->nNodes + 2))));
+                stageNeed_.add(pg->nSlots, pg->nNodes);
             }
         }
         totalSlots_ = slot;
@@ -614,19 +614,8 @@ private:
         // Phase A's inputs staged in shared memory: as for single maps (the
         // batch kernel's register budget: 4 blocks for order classes up to 4, 2
         // above).
-        {
-            const size_t base = smem + 2048;
-            const size_t lb = pclass_ <= 4 ? 4 : 2;
-            auto blocks = [&](size_t b) { return std::min<size_t>(lb, (size_t)smemPerSM_ / b); };
-            auto fits = [&](int n) {
-                const size_t with = base + (size_t)n * sizeof(double);
-                return with <= 227 * 1024 && blocks(with) == blocks(base);
-            };
-            int n = stageNeed_;
-            while (n >= kStageMin && !fits(n)) n /= 2;
-            if (n < kStageMin) n = base + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
-            p.stageDoubles = n;
-        }
+        p.stageDoubles = stageRoom(stageNeed_, p.cmFx != nullptr, smem + (p.cmFx ? 2048 : 1024), (size_t)smemPerSM_,
+                                   pclass_ <= 4 ? 4 : 2);
         // The kept products of a tile, one cache per resident block (at most
         // 512 threads an SM); above 2 GiB the reduction forms them again in FP64.
         p.rcStride = (long long)maxCNodes_ * tpb_;
@@ -721,8 +710,9 @@ private:
     int basis_ = 0, pos_ = 0;
     QuadParams quad_{};
     BasisConsts bc_{};
-    int dmax_ = 1, nBmax_ = 0, depthMax_ = 0, pclass_ = 2, totalSlots_ = 0, numSMs_ = 1, stageNeed_ = 0, maxCNodes_ = 0,
+    int dmax_ = 1, nBmax_ = 0, depthMax_ = 0, pclass_ = 2, totalSlots_ = 0, numSMs_ = 1, maxCNodes_ = 0,
         smemPerSM_ = 0;
+    StageNeed stageNeed_;
     int tpb_ = 128;
     std::map<std::pair<int, int>, int> tiles_;
     Buf gradScratch_;  // autotuning: coefficient adjoints of timed calls

@@ -16,6 +16,7 @@
 
 #include "mpgb_fastmath.cuh"
 #include "mpgb_fixed.cuh"
+#include "mpgb_stage.h"
 
 namespace mpgb {
 
@@ -36,11 +37,6 @@ constexpr int kMaxSubCap = 32;
 // built for; reduced launches cut each component into this many work items
 // per SM.
 constexpr int kFusedBlocksPerSM = 4;
-// Largest phase-A staging (coefficient doubles plus table words) a fused
-// launch keeps in shared memory.
-constexpr int kStageCap = 2048;
-// Smallest staging the fixed-point phase A works with (its chunks of nodes).
-constexpr int kStageMin = 256;
 // Inverse: doubles of a saved root-solver state (RootSolve::save).
 constexpr int kSolveStateDoubles = 14;
 // Inverse warp pass: lanes per deferred point (32 / kWarpGroup points per warp).

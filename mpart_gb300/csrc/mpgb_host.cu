@@ -393,7 +393,7 @@ struct MapWorkspace {
     QuadParams quad{};
     BasisConsts bc{};
     int pmax = 1, dmax = 1, nBmax = 0, depthMax = 0;
-    int stageNeed = 0;  // doubles of the largest phase-A staging among the monotone components (<= kStageCap)
+    StageNeed stageNeed;  // of the monotone components
     int smemPerSM = 0;
     int basis = 0;  // kernel family: the options' basis, or kBasisSigmoid
     bool built = false;
@@ -716,7 +716,7 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
             W.dmax = std::max(W.dmax, p.D);
             W.nBmax = std::max(W.nBmax, p.nB);
             W.depthMax = std::max(W.depthMax, p.maxDepth);
-            if (p.kind == 0) W.stageNeed = std::max(W.stageNeed, std::max(kStageMin, std::min(kStageCap, p.nSlots + 2 * (p.nNodes + 2))));
+            if (p.kind == 0) W.stageNeed.add(p.nSlots, p.nNodes);
         }
         MPGB_CUDA(cudaDeviceGetAttribute(&W.smemPerSM, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev));
         W.totalSlots = slotOff;
@@ -1132,21 +1132,15 @@ static void orderPoints(MapWorkspace& W, const std::vector<MonotoneMapBase::Part
     p.permStride = N;
 }
 
-// Phase A's inputs are staged in shared memory (FusedParams::stageDoubles):
-// the largest of the full need, halves of it and kStageMin that does not lower
-// the number of blocks an SM holds (phaseALimbs takes a component in chunks),
-// or kStageMin all the same.
+// Phase A's staging in shared memory (FusedParams::stageDoubles); whether a
+// launch takes limbs is fusedBody's own rule.
 static int stageDoubles(const MapWorkspace& W, const FusedParams& p, bool input) {
-    if (W.stageNeed == 0 || W.smemPerSM <= 0) return 0;
-    const size_t base = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, input) + 2048;
-    auto blocks = [&](size_t b) { return std::min<size_t>(kFusedBlocksPerSM, (size_t)W.smemPerSM / b); };
-    auto fits = [&](int n) {
-        const size_t with = base + (size_t)n * sizeof(double);
-        return with <= 227 * 1024 && blocks(with) == blocks(base);
-    };
-    for (int n = W.stageNeed; n >= kStageMin; n /= 2)
-        if (fits(n)) return n;
-    return base + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
+    const bool limbs = p.cmFx && (!(p.flags & (kFlagCoefDenseT | kFlagCoefDenseL | kFlagInput)) ||
+                                  (p.flags & kFlagImplicit));
+    // (static shared memory: fusedBody's limb reduction, 2 KB with room to spare)
+    const size_t base = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, W.pmax, input) +
+                        (limbMap(W.basis, W.pmax) ? 2048 : 1024);
+    return stageRoom(W.stageNeed, limbs, base, (size_t)std::max(0, W.smemPerSM), kFusedBlocksPerSM);
 }
 
 static void launch(MapWorkspace& W, const MapOptions& o, FusedParams& p, const LaunchPlan& plan, int needJ, int needE,

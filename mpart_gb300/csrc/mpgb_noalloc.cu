@@ -262,7 +262,7 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         buildLaunchConstants(o, p.quad, p.bc);
         const size_t smem = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, pmax, false);
         if (smem > 227 * 1024) throw std::invalid_argument("component too large for the shared-memory tile");
-        p.stageDoubles = smem + 2048 + kStageMin * sizeof(double) <= 227 * 1024 ? kStageMin : 0;
+        p.stageDoubles = p.cmFx && smem + 2048 + kStageMin * sizeof(double) <= kSmemPerBlock ? kStageMin : 0;
         const int basis = o.basisType == BasisTypes::HermiteFunctions ? kBasisHermiteFunctions : kBasisProbHermite;
         const int pos = o.posFuncType == PosFuncTypes::Exp ? kPosExp : kPosSoftPlus;
         if (p.flags) MPGB_CUDA(launchFused(basis, pos, pmax, p, (int)items.size(), needJ, 0, stream));
