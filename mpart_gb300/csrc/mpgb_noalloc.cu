@@ -90,7 +90,7 @@ struct GatherDesc {
 
 __global__ void __launch_bounds__(512) gatherNA(const GatherDesc* descs, double* cm, int2* cmFx, int* scale) {
     const GatherDesc g = descs[blockIdx.x];
-    gatherComponent(g.src, g.slotTerm, g.slotOrder, g.nSlots, cm + g.slotOffset, cmFx + g.slotOffset,
+    gatherComponent(g.src, g.slotTerm, g.slotOrder, g.nSlots, cm + g.slotOffset, cmFx ? cmFx + g.slotOffset : nullptr,
                     scale + blockIdx.x * kFxScales);
 }
 
@@ -198,9 +198,14 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
     const size_t oItems = cv.take(std::max<size_t>(1, items.size()) * sizeof(WorkItem));
     const size_t oRows = cv.take(std::max<size_t>(1, rowBase.size()) * sizeof(long long));
     const size_t oCm = cv.take(std::max(1, slotOff) * sizeof(double));
-    const size_t oCmFx = cv.take((slotOff + 1) * sizeof(int2));
-    const size_t oScale = cv.take(nComps * kFxScales * sizeof(int));
     const size_t oPart = cv.take(std::max<long long>(1, partBase) * sizeof(double));
+    // (coefficients as limbs where there is room left: without them phase A is FP64)
+    const int basis = o.basisType == BasisTypes::HermiteFunctions ? kBasisHermiteFunctions : kBasisProbHermite;
+    Carve fx = cv;
+    const size_t oCmFx = fx.take((slotOff + 1) * sizeof(int2));
+    const size_t oScale = fx.take(nComps * kFxScales * sizeof(int));
+    const bool limbs = limbMap(basis, pmax) && fx.used <= kNoAllocScratchBytes;
+    if (limbs) cv = fx;
     if (cv.used > kNoAllocScratchBytes) {
         std::ostringstream os;
         os << "the no-allocation entry point needs " << cv.used << " bytes of scratch for this call but holds "
@@ -216,8 +221,8 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         MPGB_CUDA(cudaMemcpyAsync(base + oRows, rowBase.data(), rowBase.size() * sizeof(long long), cudaMemcpyHostToDevice, stream));
     }
     double* cm = (double*)(base + oCm);
-    gatherNA<<<nComps, 512, 0, stream>>>((const GatherDesc*)(base + oGather), cm, (int2*)(base + oCmFx),
-                                         (int*)(base + oScale));
+    gatherNA<<<nComps, 512, 0, stream>>>((const GatherDesc*)(base + oGather), cm,
+                                         limbs ? (int2*)(base + oCmFx) : nullptr, (int*)(base + oScale));
     MPGB_CUDA(cudaGetLastError());
     countLaunches(stream, 1);
 
@@ -227,7 +232,7 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         p.comps = (const CompDesc*)(base + oComps);
         p.items = (const WorkItem*)(base + oItems);
         p.cm = cm;
-        p.cmFx = limbMap(o.basisType == BasisTypes::HermiteFunctions ? kBasisHermiteFunctions : kBasisProbHermite, pmax) ? (const int2*)(base + oCmFx) : nullptr;
+        p.cmFx = limbs ? (const int2*)(base + oCmFx) : nullptr;
         p.cmScale = (const int*)(base + oScale);
         p.N = N;
         p.tpb = kTpbNA;
@@ -263,7 +268,6 @@ void run(MonotoneMapBase& map, const mpgb_matrix& pts, const mpgb_matrix& sens, 
         const size_t smem = fusedSmemBytes(p.tpb, p.dmax, p.nBmax, p.depthMax, pmax, false);
         if (smem > 227 * 1024) throw std::invalid_argument("component too large for the shared-memory tile");
         p.stageDoubles = p.cmFx && smem + 2048 + kStageMin * sizeof(double) <= kSmemPerBlock ? kStageMin : 0;
-        const int basis = o.basisType == BasisTypes::HermiteFunctions ? kBasisHermiteFunctions : kBasisProbHermite;
         const int pos = o.posFuncType == PosFuncTypes::Exp ? kPosExp : kPosSoftPlus;
         if (p.flags) MPGB_CUDA(launchFused(basis, pos, pmax, p, (int)items.size(), needJ, 0, stream));
         if (valuesApart) {
