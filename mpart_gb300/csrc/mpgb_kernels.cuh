@@ -1694,8 +1694,13 @@ struct SigmoidInverseEval {
 };
 
 // Comparisons of doubles on their bits: a DSETP holds the FP64 pipe as long as
-// a DFMA, and a solver step compares as often as it multiplies.  (A NaN that
-// arithmetic makes has its sign bit clear: it is above every number.)
+// a DFMA, and a solver step compares as often as it multiplies.  A NaN without
+// its sign bit is above every number; one with it (a NaN coefficient made on an
+// x86 host carries it, and FP64 arithmetic passes it on) loses it first.
+__device__ __forceinline__ double plainNaN(double x) {
+    const long long b = __double_as_longlong(x);
+    return (unsigned long long)b > 0xfff0000000000000ULL ? __longlong_as_double(0x7ff8000000000000LL) : x;
+}
 __device__ __forceinline__ bool absLess(double x, double tol) {  // |x| < tol, tol >= 0
     return (__double_as_longlong(x) & 0x7fffffffffffffffLL) < __double_as_longlong(tol);
 }
@@ -1825,6 +1830,8 @@ struct RootSolve {
     __device__ void step_(double y, double yd, const F& f, double xtol, double ftol, unsigned maxBracket,
                           int method) {
         const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+        y = plainNaN(y);
+        yd = plainNaN(yd);
         if (phase == kITP) {
             // One iteration of InverseSingleBracket's loop (RootFinding.h:152-170).
             const double xc = x, d = __dsub_rn(y, yd);
