@@ -664,7 +664,7 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
         }
         if (count >= maxIntervals) {
             R.over = true;
-            return;
+            break;
         }
     }
     R.nInt = count;

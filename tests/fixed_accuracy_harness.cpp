@@ -139,3 +139,17 @@ extern "C" void fa_moment_bias(int expr, const double* b, const double* a, const
     }
     for (int j = 0; j < kNB; ++j) mean[j] = (double)(s[j] / n);
 }
+
+// Intervals reported when the budget runs out (the field is set to -7 before).
+extern "C" int fa_over(int budget) {
+    const fx::Rule R = rule(0.0);
+    fx::Poly<kNB, false> p;
+    bool bad = false;
+    for (int j = 0; j < kNB; ++j) p.c[j] = (uint64_t)fx::toFixed58(0.5 - 0.3 * j, bad) + (1ull << 63);
+    p.a = p.Z = 0;
+    p.wideZ = false;
+    fx::Sums<0> S;
+    S.nInt = -7;
+    fx::integrate<false, kNB, false, 0>(p, R, 30, 0, budget, fx::Threshold{1, 0}, 0, S);
+    return S.over ? S.nInt : -1;
+}

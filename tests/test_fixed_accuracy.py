@@ -62,3 +62,9 @@ def test_hermite_function_moments_have_no_common_bias(lib, expr):
     mean = np.zeros(6)
     lib.fa_moment_bias(expr, _p(b), _p(a), _p(x), ctypes.c_long(n), ctypes.c_double(1e-7), _p(mean))
     assert np.all(np.abs(mean) <= 1.5e-17), mean
+
+
+@pytest.mark.parametrize("budget", [1, 2, 17])
+def test_intervals_of_an_exhausted_budget(lib, budget):
+    """The count is the next call's sort key, also where the budget ended it."""
+    assert lib.fa_over(budget) == budget
