@@ -31,15 +31,26 @@ struct Buf {
     void* p = nullptr;
     size_t n = 0;
     void ensure(size_t bytes) {
-        if (bytes <= n) return;
+        if (!tryEnsure(bytes)) throw CudaError("CUDA error cudaErrorMemoryAllocation (out of memory) at cudaMalloc");
+    }
+    // False where the device has no room (the buffer is empty then).
+    bool tryEnsure(size_t bytes) {
+        if (bytes <= n) return true;
         if (p) {
             MPGB_CUDA(cudaDeviceSynchronize());
             cudaFree(p);
             p = nullptr;
             n = 0;
         }
-        MPGB_CUDA(cudaMalloc(&p, bytes));
+        const cudaError_t e = cudaMalloc(&p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            p = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        MPGB_CUDA(e);
         n = bytes;
+        return true;
     }
     template <class T>
     T* as() const { return static_cast<T*>(p); }
@@ -617,11 +628,12 @@ private:
         p.stageDoubles = stageRoom(stageNeed_, p.cmFx != nullptr, smem + (p.cmFx ? 2048 : 1024), (size_t)smemPerSM_,
                                    pclass_ <= 4 ? 4 : 2);
         // The kept products of a tile, one cache per resident block (at most
-        // 512 threads an SM); above 2 GiB the reduction forms them again in FP64.
+        // 512 threads an SM); above 2 GiB, or without room for them, the reduction
+        // forms them again in FP64.
         p.rcStride = (long long)maxCNodes_ * tpb_;
         const long long blocks = std::min<long long>((long long)items.size(), (512LL / tpb_) * numSMs_);
-        if (p.rcStride * blocks * (long long)sizeof(double) <= (2LL << 30)) {
-            rcache_.ensure((size_t)(p.rcStride * blocks) * sizeof(double));
+        if (p.rcStride * blocks * (long long)sizeof(double) <= (2LL << 30) &&
+            rcache_.tryEnsure((size_t)(p.rcStride * blocks) * sizeof(double))) {
             p.rcache = rcache_.as<double>();
             p.rcBlocks = (int)blocks;
         }

@@ -8,9 +8,11 @@
 // word is three IMAD.WIDE, a twentieth of a DFMA's time.  The fraction has 57
 // to 63 bits, so every step rounds at 2^-57 or below where a double near 1
 // rounds at 2^-53: the integrand, its weighted sums and the error estimate
-// that drives the subdivision are closer to the exact ones than in FP64.
-// Arguments outside the range (|d_D f| possibly above 31, non-finite values,
-// other rules) keep the FP64 path.
+// that drives the subdivision are closer to the exact ones than in FP64 where
+// they are of ordinary size.  Values far below it have fewer digits than a
+// double: such quadratures, and arguments outside the range (|d_D f| possibly
+// above 31, non-finite values, other rules), keep the FP64 path (integrateFixed
+// in mpgb_kernels.cuh lists them).
 //
 // The functions are plain C++ on uint64_t, the same on the host (tests) and
 // the device.

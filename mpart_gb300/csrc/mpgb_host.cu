@@ -257,15 +257,28 @@ struct DevBuf {
     void* p = nullptr;
     size_t bytes = 0;
     void ensure(size_t b, cudaStream_t s) {
-        if (b <= bytes) return;
+        if (!tryEnsure(b, s)) throw CudaError("CUDA error cudaErrorMemoryAllocation (out of memory) at cudaMalloc");
+    }
+    // False where the device has no room (the buffer is empty then): for
+    // scratch that a launch can do without.
+    bool tryEnsure(size_t b, cudaStream_t s) {
+        if (b <= bytes) return true;
         if (p) {
             MPGB_CUDA(cudaStreamSynchronize(s));
             MPGB_CUDA(cudaFree(p));
             p = nullptr;
+            bytes = 0;
         }
-        size_t nb = std::max<size_t>(b, 256);
-        MPGB_CUDA(cudaMalloc(&p, nb));
+        const size_t nb = std::max<size_t>(b, 256);
+        const cudaError_t e = cudaMalloc(&p, nb);
+        if (e == cudaErrorMemoryAllocation) {
+            p = nullptr;
+            cudaGetLastError();
+            return false;
+        }
+        MPGB_CUDA(e);
         bytes = nb;
+        return true;
     }
     ~DevBuf() {
         if (p) cudaFree(p);
@@ -950,10 +963,10 @@ static std::vector<WorkItem> itemsPerComp(const std::vector<MonotoneMapBase::Par
 // The node cache of a reduced launch (rcTotal doubles, from itemsPerComp):
 // phase A keeps per tile the rectified products of a sigmoid expansion, or
 // the deeper prefix products of a monotone component, for the reduction.
-// Above 2 GiB the reduction forms them again.
+// Above 2 GiB, or where the device has no room, the reduction forms them again.
 static double* rectCache(MapWorkspace& W, long long rcTotal, cudaStream_t stream) {
     if (rcTotal <= 0 || rcTotal > (2LL << 30) / (long long)sizeof(double)) return nullptr;
-    W.rcache.ensure((size_t)rcTotal * sizeof(double), stream);
+    if (!W.rcache.tryEnsure((size_t)rcTotal * sizeof(double), stream)) return nullptr;
     return W.rcache.as<double>();
 }
 
@@ -1179,13 +1192,13 @@ static void inputGradient(MapWorkspace& W, const MapOptions& o, const std::vecto
     const int nComps = (int)parts.size(), nDims = (int)out.rows;
     const int tpb = tileSize(N, W.numSMs, false);
     const size_t slabBytes = (size_t)nComps * nDims * N * sizeof(double);
-    const bool split = !async && nComps > 1 && (N + tpb - 1) / tpb < 4LL * W.numSMs && slabBytes <= kMaxSlabBytes;
+    const bool split = !async && nComps > 1 && (N + tpb - 1) / tpb < 4LL * W.numSMs && slabBytes <= kMaxSlabBytes &&
+                       W.inputSlabs.tryEnsure(slabBytes, stream);
     if (!split) {
         p.outInput = out.data; p.inputRs = out.rowStride; p.inputCs = out.colStride;
         launch(W, o, p, launchPlan(W, parts, N, PlanStyle::AllComps, stream), needJ, needE, stream);
         return;
     }
-    W.inputSlabs.ensure(slabBytes, stream);
     p.outInput = W.inputSlabs.as<double>();
     p.inputRs = N;
     p.inputCs = 1;
@@ -1408,8 +1421,9 @@ void MonotoneMapBase::InverseImpl(StridedMatrix const& x1, StridedMatrix const& 
         // every point (kept in inverseA for the solver) and a root estimate;
         // the points are sorted by |estimate| (the cost of a solver step grows
         // with the range [0, x] its quadrature covers); a persistent queue
-        // launch solves them, expensive ones first, one integrand node per
-        // lane and loop iteration (inverseQueueKernel).
+        // launch solves them, expensive ones first: in fixed point one interval
+        // per lane (or four lanes) and loop iteration (inverseFixedKernel), else
+        // in FP64 one integrand node (inverseQueueKernel).
         W.inverseA.ensure((size_t)(W.pmax + 1) * N * sizeof(double), stream);
         W.inverseList.ensure((size_t)N * sizeof(int), stream);
         const int warpBlocks = kWarpPassBlocksPerSM * W.numSMs;

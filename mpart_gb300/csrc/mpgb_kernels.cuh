@@ -1,5 +1,8 @@
 // Fused kernels for MParT monotone components on sm_103a: FP64 and, for what
-// GB300's FP64 rate bounded, fixed point of higher precision (mpgb_fixed.cuh).
+// GB300's FP64 rate bounded, 64-bit fixed point (mpgb_fixed.cuh).  Fixed point
+// holds 57 to 62 bits below a bound of the values, more than a double near the
+// bound and fewer far below it: each use says where that suffices and sends the
+// rest to FP64.
 //
 // One thread per point.  A block holds a tile of points and walks a range of
 // components; per point and component:
