@@ -75,14 +75,6 @@ MPGB_HD uint64_t mulhiAny(uint64_t a, uint64_t b) {
     return madWide(hi32(a), hi32(b), hi32(m1)) + hi32(m2);
 }
 
-// The same with the low words' product: rounded to nearest also where a or b
-// is small (mulhi and mulhiAny add the mean of a product that is not there).
-MPGB_HD uint64_t mulhiRound(uint64_t a, uint64_t b) {
-    const uint64_t m1 = madWide(lo32(a), hi32(b), hi32(mulWide(lo32(a), lo32(b))));
-    const uint64_t m2 = madWide(hi32(a), lo32(b), (uint64_t)lo32(m1) + 0x80000000ull);
-    return madWide(hi32(a), hi32(b), (uint64_t)hi32(m1) + hi32(m2));
-}
-
 // floor(a b / 2^32).
 MPGB_HD uint64_t mul32(uint64_t a, uint32_t b) { return madWide(hi32(a), b, hi32(mulWide(lo32(a), b))); }
 
@@ -372,7 +364,7 @@ MPGB_HD Node nodeAt(const Poly<NB, ENV>& p, uint64_t t) {
         const uint64_t e = shrRound(v.m, v.n);
         rect<EXPR, DERIV>(p.a + mulhiAny(horner(p, t), e << 1) - e, o, gp);
         if constexpr (DERIV) {
-            o.fe = mulhiRound(gp, v.m);
+            o.fe = mulhi(gp, v.m);
             o.n = v.n;
         }
     } else {
@@ -396,7 +388,7 @@ MPGB_HD Node nodeEnd(const Poly<NB, ENV>& p, bool one) {
         const uint64_t e = shrRound(v.m, v.n);
         rect<EXPR, DERIV>(p.a + mulhiAny(q, e << 1) - e, o, gp);
         if constexpr (DERIV) {
-            o.fe = mulhiRound(gp, v.m);
+            o.fe = mulhi(gp, v.m);
             o.n = v.n;
         }
     } else {
@@ -593,20 +585,15 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
                     fa = A.f; fb = B.f; fm = M.f; fv = V.f; fw = W.f;
                 }
                 uint64_t mu[NM];
-                // (The envelope makes terms of a few units, which the shift to
-                // t = 0 multiplies by up to 2^(5 j): products and shifts are
-                // rounded to nearest, ties either way.  Halves up and the
-                // short product's mean were 6e-17 of the fifth moment of every
-                // point, 1e-15 of an order-5 gradient.)
-                auto mul = [](uint64_t x, uint64_t y) {
-                    if constexpr (ENV) return mulhiRound(x, y);
-                    else return mulhi(x, y);
-                };
-                fb = mul(fb, Q.w0);
-                fm = mul(fm, Q.wM);
-                mu[0] = mul(fa, Q.w0) + fb + fm + mul(fv + fw, Q.w1);
+                // (The shift to t = 0 multiplies units by up to 2^(5 ms): its
+                // ties are rounded either way.  Halves up, without the tail's
+                // bits, were 6e-17 of the fifth moment of every point, 1e-15
+                // of an order-5 gradient.)
+                fb = mulhi(fb, Q.w0);
+                fm = mulhi(fm, Q.wM);
+                mu[0] = mulhi(fa, Q.w0) + fb + fm + mulhi(fv + fw, Q.w1);
 #pragma unroll
-                for (int j = 1; j < NM; ++j) mu[j] = fb + ((fm + ((1ull << j) >> 1)) >> j) + mul(fv, Q.mLo[j]) + mul(fw, Q.mHi[j]);
+                for (int j = 1; j < NM; ++j) mu[j] = fb + ((fm + ((1ull << j) >> 1)) >> j) + mulhi(fv, Q.mLo[j]) + mulhi(fw, Q.mHi[j]);
 #pragma unroll
                 for (int j = 0; j < NM; ++j) {
                     if constexpr (ENV) mu[j] = scaleEven(mu[j], level * j + dn - ms * (EXPR ? j : j + 1));
@@ -620,8 +607,12 @@ MPGB_HD void integrate(const Poly<NB, ENV>& p, const Rule& Q, int maxSub, int mi
                         else mu[j] += mul32Round(mu[j - 1], lo);
                     }
                 }
+                if (ENV && tail) {
 #pragma unroll
-                for (int j = 0; j < NM; ++j) R.m[j] += ENV ? scaleEven(mu[j], tail) : mu[j];
+                    for (int j = 0; j < NM; ++j) mu[j] = scaleEven(mu[j], tail);
+                }
+#pragma unroll
+                for (int j = 0; j < NM; ++j) R.m[j] += mu[j];
             }
             if constexpr (EXPR) {
                 if (R.g >> 62) {
