@@ -1037,6 +1037,9 @@ def run_gpu(args):
         "gpu_launches": launches,
         "roofline": {"bound": "fp64", "achieved": achieved, "peak": peak_tf, "unit": "TFLOP/s",
                      "frac": achieved / peak_tf, "traffic": traffic,
+                     "note": "model operations against the FP64 peak; most of them run as integer instructions "
+                             "(64-bit fixed point), so frac compares with a perfect FP64 kernel and is not the FP64 "
+                             "pipe's load",
                      "peak_source": "DFMA probe in this run (MEASURED_PEAKS.json has no FP64 figure)",
                      "flops_per_point": fpp, "evals_per_point": E,
                      "reference_algorithm": {
