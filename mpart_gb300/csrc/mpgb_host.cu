@@ -357,6 +357,7 @@ struct LaunchPlan {
         cudaStream_t stream;
         cudaEvent_t event;
     };
+    static constexpr size_t kMaxStreams = 16;
     std::vector<After> uploads, uses;
     LaunchPlan() = default;
     LaunchPlan(const LaunchPlan&) = delete;
@@ -370,10 +371,19 @@ struct LaunchPlan {
                 MPGB_CUDA(cudaEventRecord(a.event, s));
                 return;
             }
-        After a{s, nullptr};
-        MPGB_CUDA(cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming));
-        v.push_back(a);
-        MPGB_CUDA(cudaEventRecord(a.event, s));
+        if (v.size() >= kMaxStreams) {
+            // (s takes over the first one's entry: after it, s's event covers both)
+            After a = v.front();
+            v.erase(v.begin());
+            MPGB_CUDA(cudaStreamWaitEvent(s, a.event, 0));
+            a.stream = s;
+            v.push_back(a);
+        } else {
+            After a{s, nullptr};
+            MPGB_CUDA(cudaEventCreateWithFlags(&a.event, cudaEventDisableTiming));
+            v.push_back(a);
+        }
+        MPGB_CUDA(cudaEventRecord(v.back().event, s));
     }
     static void wait(const std::vector<After>& v, cudaStream_t s) {
         for (auto& a : v)

@@ -916,7 +916,8 @@ static __device__ __noinline__ bool littleSums(const int4* row, const int4* Wl, 
 // node (nodes sorted by nk: the orders of a warp's four nodes run together),
 // two points each at a time: 16-byte loads, whole lines of rc, the next
 // nodes' lines in flight during the sums.  Measured with phase A: the dim-8
-// order-4 fused adjoint at 1M points 4.17 -> 3.3 ms.
+// order-4 fused adjoint at 1M points 4.17 -> 3.3 ms (3.4 with the check that
+// follows).
 // A node with a sum whose terms' magnitudes stay below kMinShare (32 of the
 // points decide, all of them if those do not reach it) is left out and marked in
 // its row of rc, column `mark`; *redo is set.

@@ -138,3 +138,26 @@ def test_implicit_gradient_of_many_components(gpu, dim, n):
     lam = torch.linalg.solve(J.transpose(1, 2), w.T[:, :, None])[:, :, 0].T.contiguous()
     g = -tm.CoeffGrad(x, lam).sum(1)
     assert torch.all((a[0] - g).abs() <= 1e-10 * torch.clamp(g.abs(), min=1e-3 * float(g.abs().max())))
+
+
+def test_more_streams_than_are_followed(gpu):
+    """One map on more streams in turn than a set keeps events for."""
+    import torch
+    tm = _map(gpu)
+    x = _points(2, 500)
+    xs = [x[:, :n].contiguous() for n in range(100, 140)]
+    ref = [_map(gpu).Evaluate(a) for a in xs]
+    streams = [torch.cuda.Stream() for _ in range(24)]
+    out = [torch.zeros(2, a.shape[1], dtype=torch.float64, device="cuda") for a in xs]
+    torch.cuda.synchronize()
+    tm.SetAsync(True)
+    last = torch.cuda.current_stream()
+    for k in range(200):
+        s = streams[k % 24]
+        s.wait_stream(last)
+        with torch.cuda.stream(s):
+            tm.EvaluateImpl(xs[k % 40], out[k % 40])
+        last = s
+    torch.cuda.synchronize()
+    for a, b in zip(out, ref):
+        assert torch.equal(a, b)
