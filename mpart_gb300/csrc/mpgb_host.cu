@@ -404,10 +404,13 @@ struct MapWorkspace {
     std::vector<LaunchPlan*> plansInCall;  // since the last Finish
     long long planClock = 0;
     int* hostStatus = nullptr;  // pinned: a pageable copy is staged by the driver
+    long long statusReads = 0;
     ~MapWorkspace() {
         if (hostStatus) cudaFreeHost(hostStatus);
     }
-    DevBuf comps, cm, cmFx, cmScale, gather, partials, lossPart, logdetRows, status;
+    int2* cmFx = nullptr;  // in cm's buffer; null: no limbs
+    int* cmScale = nullptr;
+    DevBuf comps, cm, gather, partials, lossPart, logdetRows, status;
     DevBuf stage[8];
     std::vector<CompDesc> hostComps;
     std::vector<GatherDescHost> hostGather;
@@ -754,9 +757,14 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
         W.comps.ensure(W.hostComps.size() * sizeof(CompDesc), stream);
         MPGB_CUDA(cudaMemcpy(W.comps.p, W.hostComps.data(), W.hostComps.size() * sizeof(CompDesc),
                              cudaMemcpyHostToDevice));
-        W.cm.ensure(std::max(1, W.totalSlots) * sizeof(double), stream);
-        W.cmFx.ensure((W.totalSlots + 1) * sizeof(int2), stream);
-        W.cmScale.ensure(W.hostComps.size() * kFxScales * sizeof(int), stream);
+        // (one buffer: the coefficients, and for maps with limbs those and their scales)
+        const size_t slots = (size_t)W.totalSlots + 1;
+        const bool limbs = limbMap(W.basis, W.pmax);
+        W.cm.ensure(slots * sizeof(double) +
+                        (limbs ? slots * sizeof(int2) + W.hostComps.size() * kFxScales * sizeof(int) : 0),
+                    stream);
+        W.cmFx = limbs ? (int2*)(W.cm.as<double>() + slots) : nullptr;
+        W.cmScale = limbs ? (int*)(W.cmFx + slots) : nullptr;
         W.status.ensure(sizeof(int) * 4, stream);
         MPGB_CUDA(cudaMemset(W.status.p, 0, sizeof(int) * 4));
         W.built = true;
@@ -778,9 +786,8 @@ void MonotoneMapBase::Prepare(cudaStream_t stream) {
         MPGB_CUDA(cudaStreamSynchronize(stream));
         W.hostGather = g;
     }
-    const bool limbs = limbMap(W.basis, W.pmax);
-    gatherMultiKernel<<<(unsigned)g.size(), 512, 0, stream>>>(W.gather.as<GatherDescHost>(), W.cm.as<double>(),
-                                                              limbs ? W.cmFx.as<int2>() : nullptr, W.cmScale.as<int>());
+    gatherMultiKernel<<<(unsigned)g.size(), 512, 0, stream>>>(W.gather.as<GatherDescHost>(), W.cm.as<double>(), W.cmFx,
+                                                              W.cmScale);
     MPGB_CUDA(cudaGetLastError());
     countLaunches(stream, 1);
 }
@@ -828,10 +835,14 @@ double* MonotoneMapBase::StagingBuffer(int slot, size_t bytes, cudaStream_t stre
 int MonotoneMapBase::CheckStatus(cudaStream_t stream) {
     MapWorkspace& W = *ws_;
     if (!W.status.p) return 0;
-    if (!W.hostStatus) MPGB_CUDA(cudaMallocHost(&W.hostStatus, sizeof(int)));
-    MPGB_CUDA(cudaMemcpyAsync(W.hostStatus, W.status.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
+    // (a map's first read goes without the pinned word: page-locking it takes
+    // longer than the staged copy)
+    int first = 0;
+    if (W.statusReads++ == 1) MPGB_CUDA(cudaMallocHost(&W.hostStatus, sizeof(int)));
+    int* word = W.hostStatus ? W.hostStatus : &first;
+    MPGB_CUDA(cudaMemcpyAsync(word, W.status.p, sizeof(int), cudaMemcpyDeviceToHost, stream));
     MPGB_CUDA(cudaStreamSynchronize(stream));
-    const int st = *W.hostStatus;
+    const int st = *word;
     if (st) MPGB_CUDA(cudaMemsetAsync(W.status.p, 0, sizeof(int), stream));
     return st;
 }
@@ -887,8 +898,8 @@ void checkMatrix(const StridedMatrix& m, int64_t rows, int64_t cols, const char*
 static void baseParams(MapWorkspace& W, const MapOptions& o, FusedParams& p, long long N) {
     p.comps = W.comps.as<CompDesc>();
     p.cm = W.cm.as<double>();
-    p.cmFx = limbMap(W.basis, W.pmax) ? W.cmFx.as<int2>() : nullptr;
-    p.cmScale = W.cmScale.as<int>();
+    p.cmFx = W.cmFx;
+    p.cmScale = W.cmScale;
     p.N = N;
     p.tpb = kTpb;
     p.nugget = o.nugget;
