@@ -117,3 +117,53 @@ def test_coefficients_of_one_order(gpu, c):
     terms = np.stack([c[0] + 0 * x[0], c[1] * nrm * x[0], c[2] * nrm * x[1], c[3] * nrm ** 2 * x[0] * x[1]])
     size = _dev(np.abs(terms).sum(0) + 2.0 * np.abs(c[4]) + 2.0 * np.abs(x[2]))
     assert torch.all((got.reshape(-1) - _dev(terms.sum(0))).abs() <= 1e-14 * size)
+
+
+def _mixed(r, dim, n):
+    """Each input large at a part of the points where the others are tiny."""
+    return r.standard_normal((dim, n)) * np.where(np.arange(n) % dim == np.arange(dim)[:, None], 1.0, 1e-5)
+
+
+@pytest.mark.parametrize("tpb", [64, 128])
+def test_batch_of_maps_with_mixed_inputs(gpu, tpb):
+    M = gpu
+    import torch
+    r = np.random.default_rng(4)
+    maps, x, s = [], [], []
+    for d, o, n in ((2, 5, 1500), (4, 3, 700), (6, 2, 65)):
+        maps.append(M.CreateTriangular(d, d, o, _opts(M)))
+        maps[-1].SetCoeffs(r.normal(0.0, 0.1, maps[-1].numCoeffs))
+        x.append(_dev(_mixed(r, d, n)))
+        s.append(_dev(r.standard_normal((d, n))))
+    b = M.MapBatch(maps)
+    b.SetTuning(tpb, b.Tuning()[1])
+    z = lambda *q: torch.zeros(*q, dtype=torch.float64, device="cuda")  # noqa: E731
+    cg = [z(m.numCoeffs) for m in maps]
+    b.FusedForwardAdjoint(x, s, logdet_sens_scale=0.0, out_eval=[torch.zeros_like(a) for a in s],
+                          out_logdet=[z(a.shape[1]) for a in x], coeff_grad=cg)
+    for m, a, w, g in zip(maps, x, s, cg):
+        dense = m.CoeffGrad(a, w).cpu().numpy().astype(np.longdouble)
+        assert np.all(np.abs(g.cpu().numpy() - dense.sum(1)) <= 3e-14 * np.abs(dense).sum(1))
+
+
+@pytest.mark.parametrize("n", [100, 20_000])
+def test_implicit_gradient_with_mixed_inputs(gpu, n):
+    """-sum_p dT/dc lambda with lambda from the triangular solve in torch: the
+    solves agree to some 1e-15 of lambda's size."""
+    import torch
+    M = gpu
+    dim = 4
+    r = np.random.default_rng(9)
+    tm = M.CreateTriangular(dim, dim, 3, _opts(M))
+    tm.SetCoeffs(r.normal(0.0, 0.1, tm.numCoeffs))
+    x, w = _dev(_mixed(r, dim, n)), _dev(r.standard_normal((dim, n)))
+    g = tm.InverseCoeffGrad(torch.zeros(0, n, dtype=torch.float64, device="cuda"), x, w)[0]
+    J = torch.zeros(n, dim, dim, dtype=torch.float64, device="cuda")
+    one = torch.ones(1, n, dtype=torch.float64, device="cuda")
+    for i in range(dim):
+        c, xi = tm.GetComponent(i), x[:i + 1].contiguous()
+        J[:, i, :i + 1] = c.Gradient(xi, one).T
+        J[:, i, i] = torch.exp(c.LogDeterminant(xi))
+    lam = torch.linalg.solve(J.transpose(1, 2), w.T[:, :, None])[:, :, 0].T.contiguous()
+    dense = tm.CoeffGrad(x, lam)
+    assert torch.all((g + dense.sum(1)).abs() <= 1e-12 * dense.abs().sum(1))
